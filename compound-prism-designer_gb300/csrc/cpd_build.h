@@ -173,6 +173,18 @@ CPD_HDN inline void to_dev(const cpd_design &d, DevDesign &D)
     f.hL = (float)x::mul(0.5, D.L);
     f.ar = D.ar;
     f.B = D.B;
+    {
+        // what the certified pieces (cpd_piece.h) assume beyond the coating: the bound's centre
+        // on the exit circle, and an orthonormal detector frame with positive sizes
+        const float cx = (float)x::sub(D.cbx, D.ccx), cy = (float)x::sub(D.cby, D.ccy), rc = (float)D.crad;
+        const float off = cx * cx + cy * cy - rc * rc, nn = f.dnfx * f.dnfx + f.dnfy * f.dnfy - 1.f;
+        const float uu = f.dufx * f.dufx + f.dufy * f.dufy - 1.f, nu = f.dnfx * f.dufx + f.dnfy * f.dufy;
+        const bool circle = rc > 0.f && fabs(off) < 1e-3f * (rc * rc) && f.rho > 0.f && f.rho < 1.5f * rc;
+        const bool frame = fabs(nn) < 1e-5f && fabs(uu) < 1e-5f && fabs(nu) < 1e-5f;
+        const bool sizes = f.slope > 0.f && f.bin_size > 0.f && f.L > 0.f && finite(D.slope) && finite(D.L) &&
+                           finite(D.intercept) && finite(D.bin_size);
+        f.pieces = D.ar && circle && frame && sizes ? 1u : 0u;
+    }
     DFConst &c = D.dc;
     auto sp = [](double v) {
         ff::F2 r;

@@ -179,6 +179,8 @@ CPD_HDN inline bool reference_ray_df(const DevDesign &D, const float *z32, LamPa
         P.wzx = wzx.hi;
         P.wzy = wzy.hi;
         P.uz = dot(dx, dy, wzx, wzy).hi;
+        P.xref = (dx.hi * ey.hi - dy.hi * ex.hi) * C.irc.hi;
+        P.xz = (dx.hi * wzy.hi - dy.hi * wzx.hi) * C.irc.hi;
         P.ca = 2.f * dot(ex, ey, wzx, wzy).hi;
         P.cb = dot(wzx, wzy, wzx, wzy).hi;
         P.ud2 = 2.f * ud.hi;

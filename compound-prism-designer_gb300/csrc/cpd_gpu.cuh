@@ -30,12 +30,14 @@ struct alignas(16) DesignJob {
     uint32_t nchunk;     // ray chunks per 32-wavelength block
     uint32_t tile_rows;  // wavelength rows per entropy tile
     uint32_t ntiles;
-    uint32_t pad;
+    uint32_t pieces;     // evaluated by rows_kernel (certified pieces): no work items, no tiles
     float unit_hi, unit_lo;  // p per count unit, 2^-31 / R, float-float
     float lu_hi, lu_lo;      // log2 of that unit, float-float
     double pscale;           // 2^-31 / R in f64, for the optional p(d|lambda) output (set on the host:
                              // an f64 division on the device issues to the slow FP64 unit)
-    double pad2;
+    uint64_t grp_off;        // first group of rows of rows_kernel (no groups: work items)
+    uint32_t grp_rows;       // rows per group
+    uint32_t pad[3];
 };
 
 // A ray whose FP32 result fell inside a guard band: (design, wavelength row, ray). In
@@ -52,7 +54,8 @@ struct Control {
     unsigned long long item_counter;
     unsigned long long queue_count;
     unsigned int overflow;
-    unsigned int tiles_done;  // entropy tiles finished (single-design passes)
+    unsigned int tiles_done;  // entropy tiles (rows_kernel: blocks) finished (single-design passes)
+    unsigned long long group_counter;  // rows_kernel: groups claimed past each team's first
 };
 
 // What the host reads of a pass's Control words, written by the re-trace kernel (the
@@ -140,6 +143,8 @@ struct LaunchArgs {
     uint32_t mode;        // CPD_TRACE_*
     uint32_t adaptive;    // per-wavelength SEM stop: 1, or 2 with every row on the exact path
     uint32_t max_B;       // widest detector of the launch
+    uint64_t total_groups;  // groups of rows of the designs with J.pieces
+    uint32_t team;          // rows_kernel: warps per group
     Guards guards;
     double yguard_rel;
     double *p_out;        // optional W x B for the single design of the launch
@@ -262,6 +267,17 @@ void launch_loop(const LoopArgs &a, uint32_t grid, cudaStream_t stream);
 // CTAs of the loop kernel resident per SM.
 int loop_ctas_per_sm();
 
+// rows_kernel: the cells of a group of rows (a wider detector's row is a group of its own) and
+// its most rows. With 512 cells (6 KB) four warps of a block keep 20 warps per SM resident.
+constexpr uint32_t kRowsCells = 512;
+constexpr uint32_t kRowsGroup = 8;
+// How rows_kernel splits a pass of this many piece rows with tables of up to R rays: warps per
+// group of rows, and rows per group (a detector's cells may allow fewer).
+struct RowsPlan {
+    uint32_t team, group;
+};
+RowsPlan plan_rows(uint64_t rows, uint32_t R, uint32_t max_B, int num_sms);
+
 // Launches setup -> trace -> retrace -> entropy -> finalize on `stream` (adaptive
 // sampling: setup -> adaptive rounds -> exact rounds of the unsure rows -> entropy ->
 // finalize). Returns the
@@ -275,7 +291,7 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
 // Warps of the trace kernel resident at once with this block shape.
 // The kernel of a single-design pass's trace (its graph node's parameters carry the
 // design's constants and are updated per call).
-const void *trace_spans_kernel_fn();
+const void *single_trace_kernel_fn(const LaunchArgs &a);
 
 uint64_t trace_resident_warps(int num_sms, uint32_t warps_per_cta);
 

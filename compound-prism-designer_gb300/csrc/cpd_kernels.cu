@@ -24,20 +24,24 @@
 // adaptive_exact_kernel.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
+
 #include "cpd_build.h"
 #include "cpd_df.h"
 #include "cpd_gpu.cuh"
+#include "cpd_piece.h"
 
 namespace cpd {
 
 namespace {
 
-enum Field { F_ROW = 0, F_ITEM = 1, F_TILE = 2 };
+enum Field { F_ROW = 0, F_ITEM = 1, F_TILE = 2, F_GROUP = 3 };
 
 template <int FIELD>
 __device__ __forceinline__ uint64_t job_field(const DesignJob &j)
 {
-    return FIELD == F_ROW ? j.row_off : FIELD == F_ITEM ? j.item_off : j.tile_off;
+    return FIELD == F_ROW ? j.row_off : FIELD == F_ITEM ? j.item_off : FIELD == F_TILE ? j.tile_off : j.grp_off;
 }
 
 // Largest i with field(jobs[i]) <= v.
@@ -127,10 +131,14 @@ __device__ __forceinline__ uint2 setup_failed_row(const LaunchArgs &a, uint64_t 
 
 // A row's LamParams after lambda_setup_df: its guard-band rays queued as the mode asks, the
 // record written. Returns the row's fast-path range [core_lo, core_hi) (empty: hi <= lo).
-__device__ __forceinline__ uint2 setup_finish(const LaunchArgs &a, uint32_t d, uint32_t k, uint64_t row, LamParams &P)
+__device__ __forceinline__ uint2 setup_finish(const LaunchArgs &a, uint32_t d, uint32_t k, uint64_t row, LamParams &P,
+                                              bool pieces)
 {
     if (a.adaptive) {
         // the adaptive rounds trace every ray of the band themselves
+    } else if (pieces) {
+        // rows_kernel re-traces the guard bands itself; without a reference ray, all of the band
+        if (P.all_exact) P.core_lo = P.core_hi = P.band_hi;
     } else if (a.mode == CPD_TRACE_FP64 || (P.all_exact && a.mode == CPD_TRACE_HYBRID)) {
         push_ranges(a, d, k, P.band_lo, P.band_hi, 0u, 0u);
         P.core_lo = P.core_hi = 0;
@@ -157,7 +165,7 @@ __device__ __forceinline__ uint2 setup_row(const LaunchArgs &a, uint64_t row, ui
     if (D.status) return setup_failed_row(a, row);
     LamParams P;
     lambda_setup_df(D, u, z32, J.Rz, P, a.yguard_rel, a.lx + row, a.adaptive != 0);
-    return setup_finish(a, d, k, row, P);
+    return setup_finish(a, d, k, row, P, J.pieces != 0u);
 }
 
 // One warp per block of 32 rows. The block first copies its design record and, for
@@ -336,7 +344,7 @@ __global__ void __launch_bounds__(64) setup_pair_kernel(const LaunchArgs a)
             LamParams P;
             zero_lam_params(P);
             setup_tail(D, z32, J.Rz, P, a.lx + row, Sd, Sp, lost || Sp.lost);
-            core = setup_finish(a, 0u, (uint32_t)row, row, P);
+            core = setup_finish(a, 0u, (uint32_t)row, row, P, J.pieces != 0u);
         }
     }
     // this block's 32 rows are the trace's block blockIdx.x
@@ -547,13 +555,17 @@ __global__ void __maxnreg__(CPD_TRACE_MAXNREG) trace_kernel(const LaunchArgs a)
 
 // The queued rays, hybrid mode: the float-float re-trace.
 // The pass's final queue state for the host (no later kernel changes it).
-__device__ __forceinline__ void publish_status(const LaunchArgs &a)
+__device__ __forceinline__ void publish_status_all(const LaunchArgs &a)
 {
-    if (a.status && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (a.status && threadIdx.x == 0) {
         a.status->queue_count = a.ctl->queue_count;
         a.status->overflow = a.ctl->overflow;
         a.status->pad = 0u;
     }
+}
+__device__ __forceinline__ void publish_status(const LaunchArgs &a)
+{
+    if (blockIdx.x == 0) publish_status_all(a);
 }
 
 __global__ void __launch_bounds__(32) retrace_kernel(const LaunchArgs a)
@@ -1436,6 +1448,465 @@ __global__ void __launch_bounds__(kEntropyThreads, 4) entropy_block_kernel(const
     }
 }
 
+// ------------------------------------------------------------------ rows by certified pieces
+
+#ifndef CPD_ROWS_MAXNREG
+#define CPD_ROWS_MAXNREG 96
+#endif
+constexpr uint32_t kRowsWarps = 4;      // warps per block of rows_kernel, at least a team's
+constexpr uint32_t kRowsMaxTeam = 16;   // most warps of a team
+constexpr uint32_t kRowsBrief = 48;     // a range of up to this many rays goes through fast_ray whole
+constexpr uint32_t kRowsPieces = 15;    // pieces per half-warp (16 ends)
+constexpr uint32_t kRowsSplit = 24;     // a piece without a bound is cut again from this many rays
+constexpr uint32_t kRowsList = 64;      // entries of a warp's lists
+constexpr uint32_t kRowsFull = 28;      // waiting ranges that make a batch: one step adds at most 34
+constexpr uint32_t kRayBits = 22;       // (row of the group << kRayBits | ray) in one word
+constexpr uint32_t kRayMask = (1u << kRayBits) - 1u;
+static_assert(CPD_MAX_RAYS <= 1u << kRayBits && kRowsGroup <= 1u << (31 - kRayBits), "ray and row in one word");
+constexpr uint32_t kDirect = 0x80000000u;  // in a range's end: rays for the re-trace, past fast_ray
+
+// A warp's scratch.
+struct RowsWarp {
+    float4 rec_a[32];           // z of the left end (hi, lo), v0, v1
+    float4 rec_b[32];           // v2, e, first bin, tasks | extent task << 31
+    uint4 rec_c[32];            // rays [x, y), first task, row of the group
+    uint2 wait[kRowsList];      // ranges of rays for fast_ray: row and first ray, one past the last
+    uint32_t flag[kRowsList];   // rays for the float-float re-trace
+    uint2 sub[32];              // pieces to cut again, as ranges
+    uint32_t tfix[kRowsGroup];  // the rows' transmittances
+};
+
+// Shared memory of a block: the log2 table, per-bin sums (single-design passes), the warps'
+// scratch, and per team the cells of its group of rows: ext (u64) and cnt (u32).
+constexpr size_t rows_smem_bytes(uint32_t warps, uint32_t teams, uint32_t B)
+{
+    const uint32_t cells = B > kRowsCells ? B : kRowsCells;
+    return 4u * 4u * ff::kLogTable + 16u * (size_t)B + warps * sizeof(RowsWarp) + teams * 12u * (size_t)((cells + 3u) & ~3u);
+}
+
+__device__ __forceinline__ void team_sync(uint32_t team, uint32_t T)
+{
+    // a block has at most two teams of more than one warp; constant barrier numbers, or the
+    // block would reserve all sixteen
+    if (T == 1u) __syncwarp();
+    else if (team == 0u) asm volatile("bar.sync 1, %0;" ::"r"(T * 32u) : "memory");
+    else asm volatile("bar.sync 2, %0;" ::"r"(T * 32u) : "memory");
+}
+
+// The fixed-N hybrid estimate of the designs whose coated exit face admits certified pieces
+// (cpd_piece.h), from LamParams to the per-bin sums: trace, re-trace and entropy of a
+// wavelength row by one team of T warps, with no histogram in memory.
+//
+// A team takes groups of rows of one design (J.grp_rows of them; one row when T > 1), whose
+// cells live in shared memory: cnt counts the hits with the row's own transmittance (every hit
+// of a certified piece), ext adds up the others. Per group:
+//  1. Half a warp cuts a row's core range (T > 1: its share of it) into 15 pieces, lane i
+//     evaluating the ray at the left end of piece i. A piece in one bin, or lost whole, is
+//     counted at once; a mixed piece's bins come from its edges, two lanes per bin, each
+//     finding one edge by bisection of the piece's rays on its quadratic, or, where the edges
+//     lie too close, ray by ray. A piece without a bound is cut again into 15.
+//  2. Rays within the error of an edge, and short pieces without a bound, wait in the warp's
+//     list for fast_ray, 32 at a time over the rows of the group; what fast_ray flags, and the
+//     setup's guard bands, wait for the float-float re-trace in the same way.
+//  3. The cells' entropy terms, lane = bin, and the sums over the group's rows added to the
+//     design's.
+// Outcomes, flags and sums are those of trace_kernel, retrace_kernel and the entropy kernels,
+// integer for integer.
+template <bool PARAM_FC, bool WITH_P>
+__global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
+{
+    cudaTriggerProgrammaticLaunchCompletion();
+    extern __shared__ __align__(16) unsigned char rows_smem[];
+    const uint32_t T = a.team, tid = threadIdx.x, lane = tid & 31u, wib = tid >> 5;
+    const uint32_t nwarps = blockDim.x >> 5, teams = nwarps / T, team = wib / T, tw = wib - team * T;
+    const uint32_t maxc = ((a.max_B > kRowsCells ? a.max_B : kRowsCells) + 3u) & ~3u;
+    float *tab = reinterpret_cast<float *>(rows_smem);
+    unsigned long long *bs1 = reinterpret_cast<unsigned long long *>(tab + 4 * ff::kLogTable), *bs2 = bs1 + a.max_B;
+    RowsWarp *wsm = reinterpret_cast<RowsWarp *>(bs2 + a.max_B);
+    RowsWarp &w = wsm[wib];
+    unsigned long long *ext = reinterpret_cast<unsigned long long *>(wsm + nwarps) + (size_t)team * maxc;
+    uint32_t *cnt = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned long long *>(wsm + nwarps) + (size_t)teams * maxc) +
+                    (size_t)team * maxc;
+    const uint32_t tt = tw * 32u + lane, tn = T * 32u;  // thread of the team
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    for (uint32_t i = tid; i < 4u * ff::kLogTable; i += blockDim.x) tab[i] = a.logtab[i];
+    for (uint32_t b = tid; b < 2u * a.max_B; b += blockDim.x) bs1[b] = 0ull;
+    for (uint32_t c = tt; c < maxc; c += tn) {
+        cnt[c] = 0u;
+        ext[c] = 0ull;
+    }
+    __syncthreads();
+    cudaGridDependencySynchronize();  // the setup's LamParams and LamDF
+    const uint32_t gteam = blockIdx.x * teams + team, nteams = gridDim.x * teams;
+    const uint32_t sp = (blockIdx.x * nwarps + wib) % (uint32_t)kSpread;
+    for (uint64_t grp = gteam; grp < a.total_groups;) {
+        const uint32_t d = PARAM_FC ? 0u : find_job<F_GROUP>(a.jobs, a.njobs, grp);
+        const DesignJob &J = PARAM_FC ? a.one : a.jobs[d];
+        const uint32_t B = J.B;
+        const uint32_t k0 = (uint32_t)(grp - J.grp_off) * J.grp_rows, g = min(J.grp_rows, J.W - k0);
+        const uint64_t row0 = J.row_off + k0;
+        const float2 *__restrict__ zt = reinterpret_cast<const float2 *>(a.z32) + J.ray_off;
+        const LamParams *lp = a.lp + row0;
+        uint32_t nhit = 0u, nret = 0u, nfast = 0u;
+        PieceConst K;
+        {
+            const FastConst Cd = PARAM_FC ? FastConst{} : a.designs[d].fc;
+            K = piece_const(PARAM_FC ? a.fc : Cd);
+        }
+        // the same in every lane: entries of the lists, the next row, and what is left of the
+        // last rows' mixed pieces: tasks [t0, total), records [ir, nrec) from ray js on
+        uint32_t nwait = 0u, nflag = 0u, nsub = 0u, next = 0u;
+        uint32_t t0 = 0u, total = 0u, ir = 0u, nrec = 0u, js = 0u;
+        // of the lane's piece: its tasks
+        uint32_t incl = 0u, excl = 0u;
+        bool by_edge = false;
+        const uint32_t half = lane >> 4, hl = lane & 15u;
+        // One step per turn, each kind in one place (the code of every step once: inlined where
+        // their lists fill, the float-float steps alone would exceed the instruction cache).
+        for (;;) {
+            const bool rows_left = next < g || nsub != 0u;
+            const bool work_left = t0 < total || ir < nrec || rows_left;
+            if (nflag >= 32u || (nflag && !work_left && !nwait)) {
+                // ---- 32 flagged rays re-traced, one per lane
+                __syncwarp();
+                const uint32_t n = min(nflag, 32u);
+                if (lane < n) {
+                    const uint32_t r = w.flag[lane], rl = r >> kRayBits;
+                    const float2 z = __ldg(zt + (r & kRayMask));
+                    uint32_t bin = 0u;
+                    float t = 0.f;
+                    if (trace_df(a.designs[d], a.lx[row0 + rl], z.x, z.y, bin, t)) {
+                        atomicAdd(ext + rl * B + bin, (unsigned long long)t_fixed(t));
+                        nhit++;
+                    }
+                    nret++;
+                }
+                __syncwarp();
+                nflag -= n;
+                const uint32_t v = w.flag[32u + lane];
+                __syncwarp();
+                if (lane < nflag) w.flag[lane] = v;
+                continue;
+            }
+            if (nwait >= kRowsFull || (nwait && !work_left)) {
+                // ---- the first 32 rays of the waiting ranges through fast_ray
+                __syncwarp();
+                uint2 e0 = lane < nwait ? w.wait[lane] : make_uint2(0u, 0u);
+                const uint2 e1 = w.wait[32u + lane];
+                const uint32_t j0 = e0.x & kRayMask, len = (e0.y & ~kDirect) - j0;
+                uint32_t ic = lane < nwait ? len : 0u;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, ic, o);
+                    if (lane >= (uint32_t)o) ic = min(ic + v, 64u);  // only the first 32 matter
+                }
+                const uint32_t sum = __shfl_sync(0xffffffffu, ic, 31), m = min(sum, 32u);
+                uint32_t ec = __shfl_up_sync(0xffffffffu, ic, 1);
+                if (lane == 0u) ec = 0u;
+                // the range of ray `lane` of the batch: ranges marked at their first ray
+                const uint32_t starts = __reduce_or_sync(0xffffffffu, lane < nwait && ec < 32u ? 1u << ec : 0u);
+                const int i = __popc(starts & (lt_mask | 1u << lane)) - 1;
+                const uint32_t ent = __shfl_sync(0xffffffffu, e0.x, i) + lane - __shfl_sync(0xffffffffu, ec, i);
+                const bool direct = (__shfl_sync(0xffffffffu, e0.y, i) & kDirect) != 0u;
+                // ranges used up leave the list
+                const uint32_t gone = __popc(__ballot_sync(0xffffffffu, lane < nwait && ic <= m && ec < m));
+                if (lane < nwait && ec < m && ic > m) e0.x += m - ec;
+                __syncwarp();
+                if (lane >= gone && lane < nwait) w.wait[lane - gone] = e0;
+                if (32u + lane < nwait) w.wait[32u + lane - gone] = e1;
+                nwait -= gone;
+                int r = RAY_LOST;
+                if (lane < m) {
+                    r = RAY_FLAG;
+                    if (!direct) {
+                        const uint32_t rl = ent >> kRayBits;
+                        const FastConst Cd = PARAM_FC ? FastConst{} : a.designs[d].fc;
+                        const FastConst &C = PARAM_FC ? a.fc : Cd;
+                        const FastLimits Ld = PARAM_FC ? FastLimits{} : fast_limits(Cd, a.guards);
+                        const FastLimits &Lm = PARAM_FC ? a.fl : Ld;
+                        const LamParams P = lp[rl];
+                        const float2 z = __ldg(zt + (ent & kRayMask));
+                        uint32_t bin = 0u;
+                        float t = 0.f;
+                        r = fast_ray(C, Lm, P, a.guards, z.x, z.y, bin, t);
+                        if (r == RAY_HIT) {
+                            const uint32_t tf = t_fixed(t);
+                            if (tf == piece_tfix(P)) {
+                                atomicAdd(cnt + rl * B + bin, 1u);
+                            } else {
+                                atomicAdd(ext + rl * B + bin, (unsigned long long)tf);
+                                nhit++;
+                            }
+                        }
+                    }
+                }
+                const uint32_t f = __ballot_sync(0xffffffffu, r == RAY_FLAG);
+                if (r == RAY_FLAG) w.flag[nflag + __popc(f & lt_mask)] = ent;
+                nflag += __popc(f);
+                continue;
+            }
+            if (t0 < total) {
+                // ---- 16 tasks of the mixed pieces: two lanes per bin, one edge each
+                // the record of task t: those that start after t0 are marked at their first task
+                const uint32_t tau = lane >> 1, t = t0 + tau;
+                const uint32_t first_rec = __popc(__ballot_sync(0xffffffffu, by_edge && incl <= t0));
+                const uint32_t starts =
+                    __reduce_or_sync(0xffffffffu, by_edge && excl > t0 && excl < t0 + 16u ? 1u << (excl - t0) : 0u);
+                const bool act = t < total;
+                const uint32_t i = act ? first_rec + __popc(starts & ((2u << tau) - 1u)) : 0u;
+                const float4 ra = w.rec_a[i], rb = w.rec_b[i];
+                const uint4 rc = w.rec_c[i];
+                const uint32_t cw = __float_as_uint(rb.w), kt = t - rc.z;
+                const bool xt = (cw >> 31) && kt + 1u == (cw & 0x7fffffffu);
+                const int bq = __float_as_int(rb.z) + (int)kt;
+                const bool up = lane & 1u;
+                const Edge ed = piece_edge(K, bq, xt, up);
+                const float sg = ra.w > 0.f ? -1.f : 1.f;  // the rays' dz fall with their index
+                uint32_t jb = 0u, je = 0u;
+                if (act) {
+                    const EdgeRays er = edge_rays(rc.x, rc.y, sg, rb.y, [&](uint32_t j) {
+                        const float2 z = __ldg(zt + j);
+                        const float dd = (ra.x - z.x) + (ra.y - z.y);
+                        return ra.z + dd * (ra.w + dd * rb.x) - ed.v;
+                    });
+                    jb = er.jb;
+                    je = er.je;
+                }
+                // the bin's rays lie between its two edges' windows
+                const uint32_t ob = __shfl_xor_sync(0xffffffffu, jb, 1), oe = __shfl_xor_sync(0xffffffffu, je, 1);
+                const uint32_t first = sg > 0.f ? je : oe, last = sg > 0.f ? ob : jb;
+                const uint32_t bin = bq > 0 ? (uint32_t)bq : 0u;
+                if (act && !up && !xt && last > first && bin < B) atomicAdd(cnt + rc.w * B + bin, last - first);
+                const bool put = ed.emit && jb < je;
+                const uint32_t f = __ballot_sync(0xffffffffu, put);
+                if (put) w.wait[nwait + __popc(f & lt_mask)] = make_uint2(rc.w << kRayBits | jb, je);
+                nwait += __popc(f);
+                t0 += 16u;
+                continue;
+            }
+            if (ir < nrec) {
+                // ---- 32 rays of a mixed piece on its quadratic
+                const float4 ra = w.rec_a[ir], rb = w.rec_b[ir];
+                const uint4 rc = w.rec_c[ir];
+                const uint32_t j = rc.x + js + lane;
+                uint32_t bin = 0u;
+                int r = RAY_LOST;
+                if (j < rc.y) {
+                    const float2 z = __ldg(zt + j);
+                    r = piece_ray(K, B, 0.f, ra.z, ra.w, rb.x, rb.y, (ra.x - z.x) + (ra.y - z.y), bin);
+                }
+                // runs of consecutive rays in one bin: the first lane of each counts it
+                const uint32_t key = r == RAY_HIT ? bin : 0xffffffffu;
+                const uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
+                const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0u || key != prev);
+                if (r == RAY_HIT && (heads >> lane & 1u)) {
+                    const uint32_t after = heads & ~(lt_mask | 1u << lane);
+                    atomicAdd(cnt + rc.w * B + bin, (after ? (uint32_t)__ffs(after) - 1u : 32u) - lane);
+                }
+                const uint32_t f = __ballot_sync(0xffffffffu, r == RAY_FLAG);
+                if (r == RAY_FLAG) w.wait[nwait + __popc(f & lt_mask)] = make_uint2(rc.w << kRayBits | j, j + 1u);
+                nwait += __popc(f);
+                js += 32u;
+                if (rc.x + js >= rc.y) {
+                    ir++;
+                    js = 0u;
+                }
+                continue;
+            }
+            if (!rows_left) break;
+            // ---- the next two rows (T > 1: two shares of the row), pieces to cut again first
+            __syncwarp();
+            uint32_t rl = 0u, lo = 0u, hi = 0u;
+            const bool again = nsub != 0u;
+            if (again) {
+                if (nsub > half) {
+                    const uint2 v = w.sub[nsub - 1u - half];
+                    rl = v.x >> kRayBits;
+                    lo = v.x & kRayMask;
+                    hi = v.y;
+                }
+                nsub -= min(nsub, 2u);
+            } else {
+                // the half's row, its core range, and the guard bands around it
+                rl = T == 1u ? min(next + half, g - 1u) : 0u;
+                const bool has = T > 1u || next + half < g;
+                const uint4 rg = *reinterpret_cast<const uint4 *>(&lp[rl].core_lo);  // core, band
+                lo = rg.x;
+                hi = rg.y;
+                uint32_t blo = rg.z, b1 = lo, b2 = hi, bhi = rg.w;
+                if (!has) hi = lo = blo = b1 = b2 = bhi = 0u;
+                if (hl == 0u && tw == 0u && (T == 1u || half == 0u)) nfast += hi - lo;
+                if (T > 1u) {
+                    const uint32_t sh = 31u - __clz(2u * T), s = 2u * tw + half;  // share s of 2 T
+                    const auto share = [&](uint32_t &p, uint32_t &q) {
+                        const uint32_t n = q - p;
+                        q = p + (n * (s + 1u) >> sh);
+                        p = p + (n * s >> sh);
+                    };
+                    share(lo, hi);
+                    share(blo, b1);
+                    share(b2, bhi);
+                }
+                const bool ba = hl == 0u && b1 > blo, bb = hl == 1u && bhi > b2;
+                const uint32_t f = __ballot_sync(0xffffffffu, ba || bb);
+                if (f) {
+                    if (ba || bb)
+                        w.wait[nwait + __popc(f & lt_mask)] =
+                            make_uint2(rl << kRayBits | (ba ? blo : b2), (ba ? b1 : bhi) | kDirect);
+                    nwait += __popc(f);
+                }
+                next += 2u;
+            }
+            const uint32_t n = hi - lo;
+            // a short range goes to fast_ray whole: one "piece", of lane 0
+            const bool brief = n <= kRowsBrief;
+            const uint32_t L = brief ? n : (n + kRowsPieces - 1u) / kRowsPieces;
+            const uint32_t j0 = lo + hl * L, j1 = min(j0 + L, hi);
+            const bool mine = hl < kRowsPieces && j0 < hi;
+            Piece q;
+            PieceEdges pe;
+            float2 z = make_float2(0.f, 0.f);
+            {
+                const FastConst Cd = PARAM_FC ? FastConst{} : a.designs[d].fc;
+                const FastConst &C = PARAM_FC ? a.fc : Cd;
+                const FastLimits Ld = PARAM_FC ? FastLimits{} : fast_limits(Cd, a.guards);
+                const FastLimits &Lm = PARAM_FC ? a.fl : Ld;
+                const LamParams P = lp[rl];
+                if (!again && hl == 0u) w.tfix[rl] = piece_tfix(P);
+                if (n) z = __ldg(zt + min(j0, hi - 1u));
+                const PieceEnd e = piece_end(C, Lm, K, P, a.guards, z.x, z.y);
+                PieceEnd o = e;
+                o.dz = __shfl_down_sync(0xffffffffu, e.dz, 1);
+                o.v = __shfl_down_sync(0xffffffffu, e.v, 1);
+                o.gv = __shfl_down_sync(0xffffffffu, e.gv, 1);
+                o.ci = __shfl_down_sync(0xffffffffu, e.ci, 1);
+                o.cr = __shfl_down_sync(0xffffffffu, e.cr, 1);
+                o.cid = __shfl_down_sync(0xffffffffu, e.cid, 1);
+                o.gn = __shfl_down_sync(0xffffffffu, e.gn, 1);
+                o.px = __shfl_down_sync(0xffffffffu, e.px, 1);
+                o.py = __shfl_down_sync(0xffffffffu, e.py, 1);
+                o.cls = __shfl_down_sync(0xffffffffu, e.cls, 1);
+                q = piece_fit(C, K, P, e, o);
+                if (!C.pieces || brief) q.cls = PIECE_RAYS;
+                pe = piece_edges(K, q, o.dz - e.dz, j1 - j0);
+            }
+            if (mine && q.cls == PIECE_BIN) atomicAdd(cnt + rl * B + q.bin, j1 - j0);
+            // pieces without a bound: cut again, or their rays wait for fast_ray
+            const bool rays = mine && q.cls == PIECE_RAYS;
+            const bool cut = rays && !again && !brief && j1 - j0 >= kRowsSplit, wait = rays && !cut;
+            const uint32_t mc = __ballot_sync(0xffffffffu, cut), mw = __ballot_sync(0xffffffffu, wait);
+            const uint2 range = make_uint2(rl << kRayBits | j0, j1);
+            if (cut) w.sub[nsub + __popc(mc & lt_mask)] = range;
+            if (wait) w.wait[nwait + __popc(mw & lt_mask)] = range;
+            nsub += __popc(mc);
+            nwait += __popc(mw);
+            // mixed pieces: records of those binned by edges, then of those binned ray by ray
+            const bool mixed = mine && q.cls == PIECE_MIXED;
+            by_edge = mixed && pe.count != 0u;
+            const uint32_t me = __ballot_sync(0xffffffffu, by_edge), mr = __ballot_sync(0xffffffffu, mixed && !by_edge);
+            incl = by_edge ? pe.count : 0u;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= (uint32_t)o) incl += v;
+            }
+            excl = by_edge ? incl - pe.count : 0u;
+            t0 = js = 0u;
+            total = __shfl_sync(0xffffffffu, incl, 31);
+            ir = __popc(me);
+            nrec = ir + __popc(mr);
+            if (mixed) {
+                const uint32_t at = by_edge ? __popc(me & lt_mask) : ir + __popc(mr & lt_mask);
+                w.rec_a[at] = make_float4(z.x, z.y, q.v0, q.v1);
+                w.rec_b[at] = make_float4(q.v2, q.e, __int_as_float(pe.qa),
+                                          __uint_as_float(pe.count | (pe.ext ? 0x80000000u : 0u)));
+                w.rec_c[at] = make_uint4(j0, j1, excl, rl);
+            }
+            __syncwarp();
+        }
+        team_sync(team, T);
+        // 3. the cells' entropy terms
+        {
+            const ff::F2 unit{J.unit_hi, J.unit_lo}, lu{J.lu_hi, J.lu_lo};
+            const uint32_t *tfix = (wsm + team * T)->tfix;
+            const uint32_t phases = tn > B && T == 1u ? 32u / B : 1u;  // rows side by side when B < 32
+            const uint32_t ph = phases > 1u ? tt / B : 0u;
+            unsigned long long hl_sum = 0ull;
+            for (uint32_t b = phases > 1u ? tt - ph * B : tt; b < B; b += phases > 1u ? B : tn) {
+                unsigned long long c1 = 0ull, q2 = 0ull;
+                for (uint32_t r = ph; r < g; r += phases) {
+                    if (ph >= phases) break;
+                    const uint32_t c = r * B + b;
+                    const uint32_t v = cnt[c];
+                    const unsigned long long cv = ext[c] + (unsigned long long)v * tfix[r];
+                    if (v) {
+                        cnt[c] = 0u;
+                        nhit += v;
+                    }
+                    if (cv) {
+                        ext[c] = 0ull;
+                        unsigned long long hq, pq;
+                        entropy_cell(cv, unit, lu, tab, hq, pq);
+                        hl_sum += hq;
+                        q2 += pq;
+                        c1 += cv;
+                    }
+                    if (WITH_P) a.p_out[(uint64_t)(k0 + r) * B + b] = (double)cv * J.pscale;
+                }
+                if (c1) {
+                    if (PARAM_FC) {
+                        atomicAdd(bs1 + b, c1);
+                        atomicAdd(bs2 + b, q2);
+                    } else {
+                        atomicAdd(&a.S1[J.acc_off + b], c1);
+                        atomicAdd(&a.S2[J.acc_off + b], q2);
+                    }
+                }
+            }
+            hl_sum = warp_sum_u64(hl_sum);
+            nhit = __reduce_add_sync(0xffffffffu, nhit);
+            nret = __reduce_add_sync(0xffffffffu, nret);
+            nfast = __reduce_add_sync(0xffffffffu, nfast);
+            if (lane == 0u) {
+                if (hl_sum) atomicAdd(&a.acc[d].H, hl_sum);
+                if (nhit) atomicAdd(&a.acc[d].hits[sp], (unsigned long long)nhit);
+                if (nret) atomicAdd(&a.acc[d].retraced[sp], (unsigned long long)nret);
+                if (nfast) atomicAdd(&a.acc[d].fast[sp], (unsigned long long)nfast);
+            }
+        }
+        team_sync(team, T);  // the cells are clear for the next group
+        if (nteams >= a.total_groups) break;
+        if (T == 1u) {
+            unsigned long long c = 0;
+            if (lane == 0) c = atomicAdd(&a.ctl->group_counter, 1ull);
+            grp = nteams + __shfl_sync(0xffffffffu, c, 0);
+        } else {
+            grp += nteams;
+        }
+    }
+    if (PARAM_FC) {
+        // a single design: the block's per-bin sums, then the finalize by the last block
+        __shared__ unsigned last_block;
+        __shared__ FinalizeRed fin_red[kRowsMaxTeam];
+        __syncthreads();
+        const uint32_t B = a.one.B;
+        for (uint32_t b = tid; b < B; b += blockDim.x)
+            if (bs1[b]) {
+                atomicAdd(&a.S1[b], bs1[b]);
+                atomicAdd(&a.S2[b], bs2[b]);
+            }
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) last_block = atomicAdd(&a.ctl->tiles_done, 1u) == gridDim.x - 1u ? 1u : 0u;
+        __syncthreads();
+        if (last_block) {
+            __threadfence();
+            publish_status_all(a);
+            finalize_design(a, 0u, a.jobs[0], tid, blockDim.x, tab, fin_red);
+        }
+    }
+}
+
 // One warp per design after the entropy kernel.
 __global__ void __launch_bounds__(128) finalize_kernel(const LaunchArgs a)
 {
@@ -1443,6 +1914,7 @@ __global__ void __launch_bounds__(128) finalize_kernel(const LaunchArgs a)
     for (uint32_t i = threadIdx.x; i < 4u * ff::kLogTable; i += blockDim.x) tab[i] = a.logtab[i];
     __syncthreads();
     cudaGridDependencySynchronize();  // the entropy kernel's sums
+    if (!a.total_items && !a.adaptive) publish_status(a);  // no re-trace kernel in this pass
     // A pass whose re-trace queue overflowed is re-run by the host: write nothing.
     if (a.ctl->overflow || a.ctl->queue_count > a.qcap) return;
     const uint32_t lane = threadIdx.x & 31u;
@@ -2088,6 +2560,37 @@ void launch_k(void (*k)(const LaunchArgs), unsigned grid, unsigned block, size_t
     cudaLaunchKernelEx(&cfg, k, a);
 }
 
+// Resident blocks of rows_kernel per SM for blocks of `warps` warps and detectors of up to B
+// bins (asked once each: the answer depends on the block and its shared memory alone).
+static uint32_t rows_blocks_per_sm(uint32_t warps, uint32_t B)
+{
+    static std::atomic<uint8_t> known[3][CPD_MAX_BINS + 1];
+    std::atomic<uint8_t> &k = known[warps <= kRowsWarps ? 0 : warps <= 8u ? 1 : 2][B];
+    uint32_t n = k.load(std::memory_order_relaxed);
+    if (!n) {
+        // one-warp teams need the most shared memory of a kRowsWarps block
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rows_kernel<false, false>, 32 * warps,
+                                                      rows_smem_bytes(warps, warps <= kRowsWarps ? warps : 1u, B));
+        n = per_sm < 1 ? 1u : (uint32_t)per_sm;
+        k.store((uint8_t)n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+RowsPlan plan_rows(uint64_t rows, uint32_t R, uint32_t max_B, int num_sms)
+{
+    RowsPlan p;
+    const uint64_t resident = (uint64_t)num_sms * rows_blocks_per_sm(kRowsWarps, max_B) * kRowsWarps;
+    // several warps per row while all of them are resident at once and each half-warp keeps
+    // 32 rays or more
+    p.team = 1u;
+    while (p.team < kRowsMaxTeam && rows * p.team * 2u <= resident && R >= 128u * p.team) p.team *= 2u;
+    // two rows or more per warp once every warp has one
+    p.group = rows <= resident ? 1u : (uint32_t)std::min<uint64_t>(kRowsGroup, std::max<uint64_t>(2u, rows / resident));
+    return p;
+}
+
 int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaStream_t stream, cudaEvent_t *ev,
                 bool pdl)
 {
@@ -2129,6 +2632,15 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
         launches++;
     } else {
     if (ev) cudaEventRecord(ev[1], stream);
+    if (a.total_groups) {
+        const uint32_t warps = std::max(kRowsWarps, a.team), teams = warps / a.team;
+        const uint64_t need = (a.total_groups + teams - 1u) / teams;
+        const uint64_t resident = (uint64_t)num_sms * rows_blocks_per_sm(warps, a.max_B);
+        auto k = a.spans ? (a.p_out ? rows_kernel<true, true> : rows_kernel<true, false>)
+                         : (a.p_out ? rows_kernel<false, true> : rows_kernel<false, false>);
+        launch_k(k, (unsigned)std::min(need, resident), 32 * warps, rows_smem_bytes(warps, teams, a.max_B), stream, pdl, a);
+        launches++;
+    }
     if (a.mode != CPD_TRACE_FP64 && a.total_items) {
         int per_sm = 0;
         const int threads = (int)warps_per_cta * 32;
@@ -2146,9 +2658,11 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
     // the single-design trace re-traces its own flagged rays; what reaches the queue there
     // (the setup's guard bands, a warp's flags past kWarpFlags) is usually little, and a
     // grid of one block per SM is resident beside the trace, ready when it completes
-    launch_k(a.mode == CPD_TRACE_FP64 ? retrace_exact_kernel : retrace_kernel,
-             (unsigned)(num_sms * (a.spans ? 1 : 8)), 32, 0, stream, pdl, a);
-    launches++;
+    if (a.total_items) {
+        launch_k(a.mode == CPD_TRACE_FP64 ? retrace_exact_kernel : retrace_kernel,
+                 (unsigned)(num_sms * (a.spans ? 1 : 8)), 32, 0, stream, pdl, a);
+        launches++;
+    }
     }
     if (ev) cudaEventRecord(ev[3], stream);
     if (a.total_tiles) {
@@ -2175,7 +2689,7 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
         }
         launches++;
     }
-    if (a.njobs > 1 || !a.total_tiles) {
+    if (a.njobs > 1 || (!a.total_tiles && !(a.spans && a.total_groups))) {
         launch_k(finalize_kernel, (a.njobs + 3u) / 4u, 128, 0, stream, pdl, a);
         launches++;
     }
@@ -2192,10 +2706,20 @@ cudaError_t configure_kernels()
                                  (int)adapt1_smem_bytes(CPD_MAX_BINS));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(adaptive_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const int rows_bytes = (int)std::max(rows_smem_bytes(kRowsWarps, kRowsWarps, CPD_MAX_BINS),
+                                         rows_smem_bytes(kRowsMaxTeam, 1u, CPD_MAX_BINS));
+    const auto rows = {rows_kernel<false, false>, rows_kernel<false, true>, rows_kernel<true, false>, rows_kernel<true, true>};
+    for (auto k : rows)
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_bytes);
     return e;
 }
 
-const void *trace_spans_kernel_fn() { return reinterpret_cast<const void *>(trace_spans_kernel); }
+const void *single_trace_kernel_fn(const LaunchArgs &a)
+{
+    if (!a.total_groups) return reinterpret_cast<const void *>(trace_spans_kernel);
+    return a.p_out ? reinterpret_cast<const void *>(rows_kernel<true, true>)
+                   : reinterpret_cast<const void *>(rows_kernel<true, false>);
+}
 
 uint64_t trace_resident_warps(int num_sms, uint32_t warps_per_cta)
 {

@@ -22,6 +22,7 @@
 //    reported FLAG and re-traced in float-float (trace_df, cpd_df.h).
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cmath>
 #include <cstring>
@@ -84,6 +85,7 @@ struct alignas(16) FastConst {
     float hL;          // L / 2
     int32_t ar;
     uint32_t B;
+    uint32_t pieces;   // the certified pieces (cpd_piece.h) apply: coated, and the geometry they assume
 };
 
 // Float-float copies of the design tables (split on the host), for the per-wavelength
@@ -138,12 +140,14 @@ struct alignas(16) LamParams {
     float ci, ci2, crsq, cr;    // reference cosines (ci2 = 2 ci)
     float r, r2, kk;            // n_last, n_last^2, r ci - cr
     float cid, T, du, pos;      // reference detector cosine, distance (p - P).N / cid, d'.u, position
+    float uz;                   // d(ud) = uz dz: d.wz
     uint32_t core_lo, core_hi;  // sorted-ray range that clears every flat face (fast path)
     uint32_t band_lo, band_hi;  // [band_lo, core_lo) and [core_hi, band_hi): guard bands
     uint32_t all_exact;         // no usable reference ray: every core ray is re-traced exactly
-    float uz;                   // d(ud) = uz dz: d.wz
-    uint32_t pad[3];
+    float xref, xz;             // sine of the exit face's incidence angle, signed: xref + xz dz
+    uint32_t pad;
 };
+static_assert(offsetof(LamParams, core_lo) % 16 == 0, "the four ranges are one 16-byte load");
 
 
 // ----------------------------------------------------------------- exact f64 ops

@@ -319,8 +319,21 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     // identity of the tables in upload order (null entries: not from a cache)
     std::vector<const void *> tables_key;
     bool cacheable = true;
-    uint64_t rows = 0, hist = 0, lam = 0, ray = 0, rnk = 0, accc = 0, items = 0, tiles = 0;
+    uint64_t rows = 0, groups = 0, hist = 0, cells = 0, lam = 0, ray = 0, rnk = 0, accc = 0, items = 0, tiles = 0;
     uint32_t max_B = 0;
+    // a coated design under the fixed-N hybrid trace goes through rows_kernel (a device build
+    // decides in its record whether the pieces apply; if not, its rays go through fast_ray there)
+    const auto by_pieces = [&](const PassDesign &p) {
+        return mode == CPD_TRACE_HYBRID && !adaptive && (p.params ? p.params->ar_coated != 0 : p.dev->fc.pieces != 0);
+    };
+    uint64_t piece_rows = 0;
+    uint32_t piece_R = 0;
+    for (const PassDesign &p : ds) {
+        max_B = std::max(max_B, p.params ? p.params->bin_count : p.dev->B);
+        if (by_pieces(p)) piece_rows += p.W, piece_R = std::max(piece_R, p.R);
+    }
+    RowsPlan plan{1u, 1u};
+    if (piece_rows) plan = plan_rows(piece_rows, piece_R, max_B, ctx->num_sms);
     for (uint32_t i = 0; i < n; i++) {
         const PassDesign &p = ds[i];
         DesignJob &J = jobs[i];
@@ -330,7 +343,6 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
         J.Rz = (uint32_t)p.rays->z64.size();
         J.B = on_device ? p.params->bin_count : p.dev->B;
         J.row_off = rows;
-        J.hist_off = hist;
         const uint32_t lam_len = std::max(p.lam_len, p.W);
         auto lo = lam_offs.emplace(std::make_pair(p.lam_u, lam_len), lam);
         J.lam_off = lo.first->second;
@@ -348,25 +360,30 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
             tables_key.push_back(p.rays);
             cacheable = cacheable && p.rays_keep;
         }
-        max_B = std::max(max_B, J.B);
         J.acc_off = accc;
         J.item_off = items;
         J.tile_off = tiles;
         J.nchunk = std::max<uint32_t>(1u, (J.Rz + ctx->ray_tile - 1) / ctx->ray_tile);
+        J.pieces = by_pieces(p) ? 1u : 0u;
+        J.hist_off = hist;
+        J.grp_off = groups;
+        J.grp_rows = std::min(plan.group, std::max(1u, kRowsCells / J.B));
+        if (J.pieces) groups += (J.W + J.grp_rows - 1) / J.grp_rows;
         J.tile_rows = tile_rows_for(J.B, n);
         J.ntiles = (J.W + J.tile_rows - 1) / J.tile_rows;
         ff::split(kTScaleInv / (double)J.R, J.unit_hi, J.unit_lo);
         ff::split(-31.0 - std::log2((double)J.R), J.lu_hi, J.lu_lo);
         J.pscale = kTScaleInv / (double)J.R;
         rows += J.W;
-        hist += (uint64_t)J.W * J.B;
+        cells += (uint64_t)J.W * J.B;
+        if (!J.pieces) hist += (uint64_t)J.W * J.B;  // rows_kernel keeps its cells in shared memory
         if (owns_rays[i]) {
             ray += (J.Rz + 1u) & ~1u;  // even: every table starts 16-byte aligned
             if (adaptive) rnk += J.R;
         }
         accc += J.B;
-        items += (uint64_t)((J.W + 31) / 32) * J.nchunk;
-        tiles += J.ntiles;
+        if (!J.pieces) items += (uint64_t)((J.W + 31) / 32) * J.nchunk;
+        if (!J.pieces) tiles += J.ntiles;
     }
     // one input arena: wavelength points | z64 | z32 | ranks | designs | jobs (256-byte
     // sections; the ranks only under adaptive sampling). The tables come first, so their
@@ -439,7 +456,7 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     CPD_TRY(S.S2.ensure(sizeof(unsigned long long) * std::max<uint64_t>(accc, 1)));
     CPD_TRY(S.acc.ensure(sizeof(DesignAcc) * n));
     CPD_TRY(S.queue.ensure(sizeof(QEntry) * S.qcap));
-    if (p_out_host) CPD_TRY(S.pout.ensure(hist_bytes));
+    if (p_out_host) CPD_TRY(S.pout.ensure(sizeof(double) * cells));
     S.ctl_off = ctl_off;
     {
         const void *after[] = {S.lp.p, S.lx.p, S.hist.p, S.S1.p, S.S2.p, S.acc.p, S.queue.p, S.h_in.p, S.h_outs.p, S.in.p};
@@ -452,7 +469,7 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
         S.hist_dirty = false;
     }
     S.h2d += up_bytes;
-    S.d2h += out_bytes + (p_out_host ? sizeof(double) * hist : 0);
+    S.d2h += out_bytes + (p_out_host ? sizeof(double) * cells : 0);
     char *din = S.in.as<char>();
 
     LaunchArgs a;
@@ -462,6 +479,8 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     a.njobs = n;
     a.total_rows = rows;
     a.total_items = items;
+    a.total_groups = groups;
+    a.team = plan.team;
     a.total_tiles = tiles;
     a.lam_u = reinterpret_cast<const double *>(din + o_lam);
     a.z64 = reinterpret_cast<const double *>(din + o_z64);
@@ -554,7 +573,7 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
             c.args = a;
             if (a.spans) {
                 c.graph = g;
-                c.trace_node = find_kernel_node(g, trace_spans_kernel_fn());
+                c.trace_node = find_kernel_node(g, single_trace_kernel_fn(a));
                 if (!c.trace_node) {
                     cudaGraphExecDestroy(exec);
                     cudaGraphDestroy(g);
@@ -590,7 +609,7 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
         CPD_TRY(cudaGetLastError());
     }
     if (p_out_host)
-        CPD_TRY(cudaMemcpyAsync(p_out_host, S.pout.p, sizeof(double) * hist, cudaMemcpyDeviceToHost, s));
+        CPD_TRY(cudaMemcpyAsync(p_out_host, S.pout.p, sizeof(double) * cells, cudaMemcpyDeviceToHost, s));
     CPD_TRY(cudaEventRecord(S.done, s));
     S.n = n;
     S.hist_cells = hist;
@@ -718,7 +737,12 @@ int tune_pass(cpd_context *ctx, const std::vector<PassDesign> &ds, uint32_t mode
     // Besides the powers of two: tiles that make the work items a whole number of rounds
     // of the resident warps (2..6 items per warp), so that the last round is not a tail.
     std::vector<std::pair<uint32_t, uint32_t>> cands;
+    const bool pieces = mode == CPD_TRACE_HYBRID && std::all_of(ds.begin(), ds.end(), [](const PassDesign &p) {
+        return p.params ? p.params->ar_coated != 0 : p.dev->fc.pieces != 0;
+    });
+    if (pieces) cands.push_back({32u, 8u});  // no work items: the shape does not matter
     for (uint32_t w : kWarps) {
+        if (pieces) break;
         for (uint32_t rt : kTiles) cands.push_back({rt, w});
         uint64_t blocks = 0, rays = 0;
         for (const PassDesign &p : ds) {
