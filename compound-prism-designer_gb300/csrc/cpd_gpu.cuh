@@ -21,7 +21,7 @@ struct alignas(16) DesignJob {
     uint32_t B;          // detector bins
     uint64_t row_off;    // first global wavelength row (LamParams index)
     uint64_t hist_off;   // first histogram cell (rows x B, u64)
-    uint64_t lam_off;    // first wavelength u-point
+    uint64_t lam_off;    // first wavelength u-point (of a design whose points are not those of a seed)
     uint64_t ray_off;    // first entry of the sorted ray tables
     uint64_t rank_off;   // first entry of the rank table (adaptive sampling)
     uint64_t acc_off;    // first per-bin accumulator (B cells in each of S1, S2)
@@ -37,7 +37,26 @@ struct alignas(16) DesignJob {
                              // an f64 division on the device issues to the slow FP64 unit)
     uint64_t grp_off;        // first group of rows of rows_kernel (no groups: work items)
     uint32_t grp_rows;       // rows per group
-    uint32_t pad[3];
+    uint32_t seeded;         // the wavelength points are seed_point(seed, k)
+    double seed;
+};
+
+// A sorted ray table that the pass makes on the device (table_sort_kernel, table_z_kernel).
+// Up to kTableRays rays: larger tables, and seeds outside [0, 1), come from the host.
+constexpr uint32_t kTableRays = 16384;
+constexpr uint32_t kTableBucket = 32;  // most points of a bucket; the host makes a denser table
+struct alignas(16) TableJob {
+    double seed;                 // points seed_point(seed, j + 1), or
+    uint64_t seed_fixed;         // (the seed in 2^-64)
+    uint64_t u_off;              // the caller's own points, when `points` is set
+    uint64_t ray_off, rank_off;  // as DesignJob
+    // the order of the sequence's first R points without a seed, when the context keeps it: a
+    // seed only turns it, by rot
+    const uint32_t *order;
+    uint32_t rot;
+    uint32_t R;
+    uint32_t points;
+    uint32_t pad;
 };
 
 // A ray whose FP32 result fell inside a guard band: (design, wavelength row, ray). In
@@ -57,6 +76,10 @@ struct Control {
     unsigned int tiles_done;  // entropy tiles (rows_kernel: blocks) finished (single-design passes)
     unsigned long long group_counter;  // rows_kernel: groups claimed past each team's first
 };
+
+// Bits of Control::overflow: the re-trace queue was too small; a table could not be made on
+// the device.
+constexpr uint32_t kOverflowQueue = 1u, kOverflowTable = 2u;
 
 // What the host reads of a pass's Control words, written by the re-trace kernel (the
 // last kernel to change them) into mapped host memory.
@@ -105,6 +128,11 @@ struct LaunchArgs {
     uint64_t total_tiles;
     const double *lam_u;
     const double *z64;
+    const TableJob *tables;  // ray tables made by this pass
+    uint32_t ntables, table_max;  // and the rays of the largest
+    uint32_t nsort;          // the first nsort of them have no order yet
+    const double *ray_u;     // the callers' own ray points
+    uint32_t *perm;          // table_sort_kernel's order, for table_z_kernel
     const float *z32;     // (hi, lo) f32 pairs of the sorted z table
     const uint32_t *rank; // adaptive sampling: ray index -> sorted position (~0u: no start height)
     LamParams *lp;

@@ -17,27 +17,7 @@ namespace cpd {
 // f64 tables -> device record (cpd_build.h).
 void design_to_dev(const cpd_design &d, DevDesign &D) { build::to_dev(d, D); }
 
-// Shaw's inverse normal CDF (erf.rs:27-73), host-side: the ray tables are built here
-// so that the device never evaluates a logarithm on the exact path.
-double norminv(double x)
-{
-    static const double P[8] = {4.3304513840364031401e-8, 0.000036313870818023761224,
-                                0.0034424140686962222423, 0.085838533424158257377,
-                                0.73176759583280610539,   2.3884158540184385711,
-                                3.0333178251950406994,    1.2533141359896652729};
-    static const double Q[8] = {1.3141263119543315917e-6, 0.00030617264753008793976,
-                                0.014494272424798068406,  0.2168237095066675527,
-                                1.2356513216582148689,    2.9373357991677046357,
-                                2.9202373175993672857,    1.0};
-    const double u = x > 0.5 ? 1.0 - x : x;
-    const double v = -std::log(2.0 * u);
-    double p = P[0], q = Q[0];
-    for (int i = 1; i < 8; i++) {
-        p = std::fma(p, v, P[i]);
-        q = std::fma(q, v, Q[i]);
-    }
-    return std::copysign(v * p / q, x - 0.5);
-}
+double norminv(double u) { return x::norminv(u); }
 
 void ray_table(const double *ray_u, uint32_t R, std::vector<double> &z64, std::vector<float> &z32,
                std::vector<uint32_t> *rank)
@@ -59,13 +39,9 @@ void ray_table(const double *ray_u, uint32_t R, std::vector<double> &z64, std::v
     }
 }
 
-// The GPU point policy: u_i = fract(fma(i0 + i, 1/phi, seed)) (kernel.rs:128-130 in f64).
 void seed_points(double seed, uint32_t first, uint32_t n, double *out)
 {
-    for (uint32_t i = 0; i < n; i++) {
-        double v = std::fma((double)(first + i), kAlpha, seed);
-        out[i] = v - std::trunc(v);
-    }
+    for (uint32_t i = 0; i < n; i++) out[i] = x::seed_point(seed, first + i);
 }
 
 }  // namespace cpd

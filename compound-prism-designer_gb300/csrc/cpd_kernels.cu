@@ -61,7 +61,7 @@ __device__ __forceinline__ void push_ray(const LaunchArgs &a, uint32_t d, uint32
 {
     unsigned long long pos = atomicAdd(&a.ctl->queue_count, 1ull);
     if (pos < a.qcap) a.queue[pos] = QEntry{d, k, j, 0u};
-    else atomicOr(&a.ctl->overflow, 1u);
+    else atomicOr(&a.ctl->overflow, kOverflowQueue);
 }
 
 // The rays [j0, j1) and [j2, j3) of row k, queued with one atomic for the whole run (a row's
@@ -73,7 +73,7 @@ __device__ __forceinline__ void push_ranges(const LaunchArgs &a, uint32_t d, uin
     const uint32_t na = j1 > j0 ? j1 - j0 : 0u, nb = j3 > j2 ? j3 - j2 : 0u;
     if (na + nb == 0u) return;
     const unsigned long long pos = atomicAdd(&a.ctl->queue_count, (unsigned long long)(na + nb));
-    if (pos + na + nb > a.qcap) atomicOr(&a.ctl->overflow, 1u);
+    if (pos + na + nb > a.qcap) atomicOr(&a.ctl->overflow, kOverflowQueue);
     for (uint32_t i = 0; i < na + nb; i++) {
         if (pos + i >= a.qcap) break;
         a.queue[pos + i] = QEntry{d, k, i < na ? j0 + i : j2 + (i - na), 0u};
@@ -113,6 +113,128 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
 {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+}
+
+// The u-point of wavelength k of a design.
+__device__ __forceinline__ double lam_point(const LaunchArgs &a, const DesignJob &J, uint32_t k)
+{
+    return J.seeded ? x::seed_point(J.seed, k) : a.lam_u[J.lam_off + k];
+}
+
+// ------------------------------------------------------------------ ray tables on the device
+
+constexpr uint32_t kTableThreads = 1024;
+constexpr size_t table_smem_bytes(uint32_t buckets, uint32_t R) { return 4u * (size_t)buckets + 2u * (size_t)R; }
+
+// One block per table without a known order (the caller's own points, and the first table of a
+// size): the order of its points, perm[sorted position] = ray. The points go
+// into at least R buckets of equal width by their leading bits (a shared-memory count, a scan,
+// a scatter), and each bucket's few are put in order by one thread. The points of a seed are
+// spread evenly (the R1 sequence: at most three share a bucket); the caller's own may not be,
+// and a bucket of more than kTableBucket leaves the table to the host. Keys are integers (a
+// seed's points as 64-bit fractions: no FP64 instruction).
+__global__ void __launch_bounds__(kTableThreads) table_sort_kernel(const LaunchArgs a)
+{
+    cudaTriggerProgrammaticLaunchCompletion();
+    extern __shared__ __align__(16) uint32_t table_smem[];
+    __shared__ uint32_t warp_sum[kTableThreads / 32u];
+    const TableJob t = a.tables[blockIdx.x];
+    const uint32_t R = t.R, tid = threadIdx.x, lane = tid & 31u;
+    const uint32_t bits = R > 1024u ? 32u - __clz(R - 1u) : 10u, M = 1u << bits;
+    uint32_t *cnt = table_smem;
+    uint16_t *slot = reinterpret_cast<uint16_t *>(table_smem + M);
+    const uint64_t alpha = (uint64_t)(kAlpha * 18446744073709551616.0);
+    const double *pts = a.ray_u + t.u_off;
+    const auto bucket = [&](uint32_t j) -> uint32_t {
+        if (!t.points) return (uint32_t)((t.seed_fixed + alpha * (j + 1u)) >> (64u - bits));
+        const uint64_t b = (uint64_t)__double_as_longlong(pts[j]);  // in (0, 1): positive, exponent below 1023
+        const int e = (int)(b >> 52) - 1011;                         // value 2^64 = significand 2^e
+        const uint64_t m = (b & 0xfffffffffffffull) | 0x10000000000000ull;
+        return (uint32_t)((e >= 0 ? m << e : e > -64 ? m >> -e : 0ull) >> (64u - bits));
+    };
+    const auto key = [&](uint32_t j) -> uint64_t {
+        return t.points ? (uint64_t)__double_as_longlong(pts[j]) : t.seed_fixed + alpha * (j + 1u);
+    };
+    for (uint32_t i = tid; i < M; i += kTableThreads) cnt[i] = 0u;
+    __syncthreads();
+    for (uint32_t j = tid; j < R; j += kTableThreads) atomicAdd(cnt + bucket(j), 1u);
+    __syncthreads();
+    // exclusive scan of the counts: M / 1024 consecutive buckets per thread
+    const uint32_t per = M / kTableThreads, b0 = tid * per;
+    uint32_t sum = 0u, most = 0u;
+    for (uint32_t i = 0; i < per; i++) {
+        const uint32_t v = cnt[b0 + i];
+        sum += v;
+        most = max(most, v);
+    }
+    if (most > kTableBucket) atomicOr(&a.ctl->overflow, kOverflowTable);
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += v;
+    }
+    if (lane == 31u) warp_sum[tid >> 5] = incl;
+    __syncthreads();
+    uint32_t before = 0u;
+    {
+        const uint32_t v = lane < (tid >> 5) ? warp_sum[lane] : 0u;
+        before = __reduce_add_sync(0xffffffffu, v);
+    }
+    uint32_t at = before + incl - sum;
+    for (uint32_t i = 0; i < per; i++) {
+        const uint32_t v = cnt[b0 + i];
+        cnt[b0 + i] = at;
+        at += v;
+    }
+    __syncthreads();
+    for (uint32_t j = tid; j < R; j += kTableThreads) slot[atomicAdd(cnt + bucket(j), 1u)] = (uint16_t)j;
+    __syncthreads();
+    // cnt[b] is now the end of bucket b
+    for (uint32_t b = tid; b < M; b += kTableThreads) {
+        const uint32_t s = b ? cnt[b - 1u] : 0u, e = cnt[b];
+        if (e - s < 2u || e - s > kTableBucket) continue;
+        for (uint32_t i = s + 1u; i < e; i++) {
+            const uint16_t v = slot[i];
+            const uint64_t kv = key(v);
+            uint32_t q = i;
+            for (; q > s; q--) {
+                const uint16_t w = slot[q - 1u];
+                const uint64_t kw = key(w);
+                if (kw < kv || (kw == kv && w < v)) break;
+                slot[q] = w;
+            }
+            slot[q] = v;
+        }
+    }
+    __syncthreads();
+    uint32_t *perm = a.perm + t.ray_off;
+    for (uint32_t i = tid; i < R; i += kTableThreads) perm[i] = slot[i];
+}
+
+// One thread per sorted position: its z in f64 (the host's own operations but for CUDA's log),
+// split into floats, and the ray's rank. blockIdx.y is the table. A warp's f64 instruction
+// takes its scheduler ~64 cycles, so the positions are spread two warps to a block; with a
+// known order this kernel is all a new seed costs, beside the setup's face loop.
+__global__ void __launch_bounds__(64) table_z_kernel(const LaunchArgs a)
+{
+    cudaTriggerProgrammaticLaunchCompletion();
+    if (a.nsort) cudaGridDependencySynchronize();  // the order
+    const TableJob t = a.tables[blockIdx.y];
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= t.R) return;
+    const uint32_t at = i + t.rot;
+    const uint32_t j = t.order ? t.order[at < t.R ? at : at - t.R] : a.perm[t.ray_off + i];
+    double z = x::norminv(t.points ? a.ray_u[t.u_off + j] : x::seed_point(t.seed, j + 1u));
+    if (!isfinite(z)) {
+        // a point that rounds to 0: its start height is not finite, and the host's table leaves it out
+        atomicOr(&a.ctl->overflow, kOverflowTable);
+        z = 0.0;
+    }
+    float hi, lo;
+    split_f32(z, hi, lo);
+    reinterpret_cast<float2 *>(const_cast<float *>(a.z32))[t.ray_off + i] = make_float2(hi, lo);
+    if (a.rank) const_cast<uint32_t *>(a.rank)[t.rank_off + j] = i;
 }
 
 // The setup of one wavelength row (below): LamParams and LamDF, and the row's guard-band
@@ -191,6 +313,7 @@ __global__ void __launch_bounds__(32) setup_kernel(const LaunchArgs a)
     }
     __shared__ __align__(16) DevDesign sD;
     extern __shared__ __align__(16) float sz[];  // 2 even(stage_cap) floats
+    if (a.ntables) cudaGridDependencySynchronize();  // the ray tables
     const uint64_t row0 = blockIdx.x * (uint64_t)blockDim.x;
     const uint64_t row = row0 + threadIdx.x;
     const uint32_t d0 = find_job<F_ROW>(a.jobs, a.njobs, row0);
@@ -203,7 +326,7 @@ __global__ void __launch_bounds__(32) setup_kernel(const LaunchArgs a)
     if (row < a.total_rows) {
         d = find_job<F_ROW>(a.jobs, a.njobs, row);
         const DesignJob &J = a.jobs[d];
-        u = a.lam_u[J.lam_off + (row - J.row_off)];
+        u = lam_point(a, J, (uint32_t)(row - J.row_off));
     }
     {
         const char *src = reinterpret_cast<const char *>(a.designs + d0);
@@ -270,7 +393,9 @@ __global__ void __launch_bounds__(64) setup_pair_kernel(const LaunchArgs a)
     const DesignJob &J = a.one;
     const bool have = row < a.total_rows;
     const bool stage_z = J.Rz <= a.stage_cap;
-    const double u = have && warp == 0 ? a.lam_u[J.lam_off + row] : 0.0;
+    // the seed from the uploaded job: the parameter's is left out (it would make every seed a
+    // graph of its own)
+    const double u = have && warp == 0 ? lam_point(a, a.jobs[0], (uint32_t)row) : 0.0;
     {
         // two groups of copies: the design record, which the face loop needs, and the z
         // table, which only the ray ranges after the loop read (its copies land while the
@@ -279,7 +404,7 @@ __global__ void __launch_bounds__(64) setup_pair_kernel(const LaunchArgs a)
         char *dst = reinterpret_cast<char *>(&sD);
         for (uint32_t i = threadIdx.x; i < sizeof(DevDesign) / 16; i += blockDim.x) cp_async16(dst + 16 * i, src + 16 * i);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (stage_z) {
+        if (stage_z && !a.ntables) {
             const char *zs = reinterpret_cast<const char *>(a.z32 + 2 * J.ray_off);
             char *zd = reinterpret_cast<char *>(sz);
             const uint32_t n16 = (J.Rz + 1u) / 2u;  // 16-byte chunks (two rays each)
@@ -331,6 +456,16 @@ __global__ void __launch_bounds__(64) setup_pair_kernel(const LaunchArgs a)
         __syncthreads();  // the flags are written again at the next face
     }
     if (warp == 1) s_pos[lane] = Sp;
+    if (a.ntables) {
+        // tables made in this pass, beside the face loop
+        cudaGridDependencySynchronize();
+        if (stage_z) {
+            const char *zs = reinterpret_cast<const char *>(a.z32 + 2 * J.ray_off);
+            char *zd = reinterpret_cast<char *>(sz);
+            const uint32_t n16 = (J.Rz + 1u) / 2u;
+            for (uint32_t i = threadIdx.x; i < n16; i += blockDim.x) cp_async16(zd + 16 * i, zs + 16 * i);
+        }
+    }
     asm volatile("cp.async.wait_all;" ::: "memory");  // this thread's share of the z table
     __syncthreads();
     if (warp == 1) return;
@@ -599,7 +734,7 @@ __global__ void __launch_bounds__(32) retrace_exact_kernel(const LaunchArgs a)
         const DesignJob &J = a.jobs[e.design];
         uint32_t bin = 0;
         double t = 0.0;
-        if (x::trace(D, x::wavelength(D, a.lam_u[J.lam_off + e.k]), x::beam_y(D, a.z64[J.ray_off + e.j]), bin, t) ==
+        if (x::trace(D, x::wavelength(D, lam_point(a, J, e.k)), x::beam_y(D, a.z64[J.ray_off + e.j]), bin, t) ==
             0) {
             atomicAdd(a.hist + J.hist_off + (uint64_t)e.k * J.B + bin, (unsigned long long)t_fixed64(t));
             atomicAdd(&a.acc[e.design].hits[i % kSpread], 1ull);
@@ -693,7 +828,7 @@ __device__ bool adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lo
         if (tid == 0) {
             const unsigned long long pos = atomicAdd(&a.ctl->queue_count, 1ull);
             if (pos < a.qcap) a.queue[pos] = QEntry{d, k, 0u, 0u};
-            else atomicOr(&a.ctl->overflow, 1u);
+            else atomicOr(&a.ctl->overflow, kOverflowQueue);
         }
         return false;
     }
@@ -891,7 +1026,7 @@ __device__ bool adaptive_row1(const LaunchArgs &a, uint64_t row, unsigned long l
         if (lane == 0) {
             const unsigned long long pos = atomicAdd(&a.ctl->queue_count, 1ull);
             if (pos < a.qcap) a.queue[pos] = QEntry{d, k, 0u, 0u};
-            else atomicOr(&a.ctl->overflow, 1u);
+            else atomicOr(&a.ctl->overflow, kOverflowQueue);
         }
         return false;
     }
@@ -1539,7 +1674,9 @@ __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
     cudaGridDependencySynchronize();  // the setup's LamParams and LamDF
     const uint32_t gteam = blockIdx.x * teams + team, nteams = gridDim.x * teams;
     const uint32_t sp = (blockIdx.x * nwarps + wib) % (uint32_t)kSpread;
-    for (uint64_t grp = gteam; grp < a.total_groups;) {
+    // a pass whose table could not be made is re-run by the host: nothing is added
+    const bool bad = a.ctl->overflow != 0u;
+    for (uint64_t grp = gteam; grp < a.total_groups && !bad;) {
         const uint32_t d = PARAM_FC ? 0u : find_job<F_GROUP>(a.jobs, a.njobs, grp);
         const DesignJob &J = PARAM_FC ? a.one : a.jobs[d];
         const uint32_t B = J.B;
@@ -1902,7 +2039,7 @@ __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
         if (last_block) {
             __threadfence();
             publish_status_all(a);
-            finalize_design(a, 0u, a.jobs[0], tid, blockDim.x, tab, fin_red);
+            if (!bad) finalize_design(a, 0u, a.jobs[0], tid, blockDim.x, tab, fin_red);
         }
     }
 }
@@ -2544,11 +2681,11 @@ __global__ void __launch_bounds__(kLoopThreads, CPD_LOOP_MIN_BLOCKS) loop_kernel
 // A launch that, with `pdl`, may start before the previous kernel on the stream has
 // finished (programmatic dependent launch): the kernel waits for its predecessor's
 // results in cudaGridDependencySynchronize.
-void launch_k(void (*k)(const LaunchArgs), unsigned grid, unsigned block, size_t smem, cudaStream_t st, bool pdl,
+void launch_k(void (*k)(const LaunchArgs), dim3 grid, unsigned block, size_t smem, cudaStream_t st, bool pdl,
               const LaunchArgs &a)
 {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -2598,6 +2735,16 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
     pdl = pdl && ev == nullptr;
     int launches = 0;
     if (ev) cudaEventRecord(ev[0], stream);
+    if (a.ntables) {
+        uint32_t M = 1024u;
+        while (M < a.table_max) M <<= 1;
+        if (a.nsort) {
+            launch_k(table_sort_kernel, a.nsort, kTableThreads, table_smem_bytes(M, a.table_max), stream, false, a);
+            launches++;
+        }
+        launch_k(table_z_kernel, dim3((a.table_max + 63u) / 64u, a.ntables), 64, 0, stream, pdl && a.nsort, a);
+        launches++;
+    }
     if (a.params) {
         launch_k(build_kernel, (a.njobs + 31u) / 32u, 32, 0, stream, false, a);
         launches++;
@@ -2609,7 +2756,7 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
         const uint32_t cap = a.stage_cap < kStageRays ? a.stage_cap : kStageRays;
         // a single-design pass (spans) splits each row's chain over two warps
         launch_k(a.spans ? setup_pair_kernel : setup_kernel, blocks, a.spans ? 64 : 32,
-                 2 * ((cap + 1u) & ~1u) * sizeof(float), stream, false, a);
+                 2 * ((cap + 1u) & ~1u) * sizeof(float), stream, pdl && a.ntables && !a.params, a);
         launches++;
     }
     if (a.adaptive) {
@@ -2708,6 +2855,9 @@ cudaError_t configure_kernels()
         e = cudaFuncSetAttribute(adaptive_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     const int rows_bytes = (int)std::max(rows_smem_bytes(kRowsWarps, kRowsWarps, CPD_MAX_BINS),
                                          rows_smem_bytes(kRowsMaxTeam, 1u, CPD_MAX_BINS));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(table_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)table_smem_bytes(kTableRays, kTableRays));
     const auto rows = {rows_kernel<false, false>, rows_kernel<false, true>, rows_kernel<true, false>, rows_kernel<true, true>};
     for (auto k : rows)
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_bytes);

@@ -233,6 +233,44 @@ CPD_HD double calc_n(const double *c, double w)
 // UniformDistribution::inverse_cdf (distribution.rs:32-34).
 CPD_HD double wavelength(const DevDesign &D, double u) { return add(D.wmin, mul(sub(D.wmax, D.wmin), u)); }
 
+// The GPU point policy: u_i = fract(fma(i, 1/phi, seed)) (kernel.rs:128-130 in f64).
+CPD_HD double seed_point(double seed, uint32_t i)
+{
+    const double v = fma_((double)i, kAlpha, seed);
+    return sub(v, trunc_(v));
+}
+
+// Shaw's inverse normal CDF (erf.rs:27-73).
+CPD_HD double norminv(double u)
+{
+    const double P[8] = {4.3304513840364031401e-8, 0.000036313870818023761224,
+                         0.0034424140686962222423, 0.085838533424158257377,
+                         0.73176759583280610539,   2.3884158540184385711,
+                         3.0333178251950406994,    1.2533141359896652729};
+    const double Q[8] = {1.3141263119543315917e-6, 0.00030617264753008793976,
+                         0.014494272424798068406,  0.2168237095066675527,
+                         1.2356513216582148689,    2.9373357991677046357,
+                         2.9202373175993672857,    1.0};
+    const double t = u > 0.5 ? sub(1.0, u) : u;
+#if defined(__CUDA_ARCH__)
+    const double v = -::log(mul(2.0, t));
+#else
+    const double v = -std::log(2.0 * t);
+#endif
+    double p = P[0], q = Q[0];
+#pragma unroll
+    for (int i = 1; i < 8; i++) {
+        p = fma_(p, v, P[i]);
+        q = fma_(q, v, Q[i]);
+    }
+    const double z = div(mul(v, p), q);
+#if defined(__CUDA_ARCH__)
+    return copysign(z, sub(u, 0.5));
+#else
+    return std::copysign(z, u - 0.5);
+#endif
+}
+
 // GaussianBeam 2-D inverse_cdf (spectrometer.rs:26-30) given z = norminv(u).
 CPD_HD double beam_y(const DevDesign &D, double z) { return sub(D.bym, mul(D.bw, z)); }
 

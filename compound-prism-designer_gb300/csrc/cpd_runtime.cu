@@ -14,7 +14,9 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <thread>
+#include <tuple>
 #include <vector>
 
 #include "cpd_gpu.cuh"
@@ -94,6 +96,8 @@ constexpr uint32_t kSamplingBits = CPD_SAMPLING_ADAPTIVE | CPD_SAMPLING_EXACT;
 // Most rows of a pass whose trace takes equal shares of span slots: every warp scans the
 // blocks' spans (32 per step) to find its share.
 constexpr uint64_t kBalancedMaxRows = 16384;
+// Sizes whose point order a context keeps on the device (at most 64 KiB each).
+constexpr size_t kMaxOrders = 64;
 
 // The kernel node of `fn` in a captured graph (nullptr if none).
 cudaGraphNode_t find_kernel_node(cudaGraph_t g, const void *fn)
@@ -121,7 +125,7 @@ struct PassSlot {
     // inputs (tables, designs, jobs) in one arena, uploaded with one copy; results
     // (DesignOut[n] then HostStatus) written by the kernels into mapped host memory;
     // `in` ends with the device-side Control words
-    DevBuf in, lp, lx, hist, S1, S2, acc, queue, pout;
+    DevBuf in, lp, lx, hist, S1, S2, acc, queue, pout, perm;
     HostBuf h_in, h_outs;
     size_t ctl_off = 0;
     bool hist_dirty = true;
@@ -178,7 +182,7 @@ struct PassSlot {
             if (c.graph) cudaGraphDestroy(c.graph);
         }
         graphs.clear();
-        for (DevBuf *b : {&in, &lp, &lx, &hist, &S1, &S2, &acc, &queue, &pout}) b->release();
+        for (DevBuf *b : {&in, &lp, &lx, &hist, &S1, &S2, &acc, &queue, &pout, &perm}) b->release();
         for (HostBuf *b : {&h_in, &h_outs}) b->release();
         for (cudaEvent_t *ev : {&ev0, &ev1, &done, &kev[0], &kev[1], &kev[2], &kev[3], &kev[4]})
             if (*ev) cudaEventDestroy(*ev), *ev = nullptr;
@@ -210,6 +214,15 @@ struct cpd_context {
     bool use_graphs = true;
     bool autotune = false;
     std::map<RayKey, RayTablePtr> ray_cache;
+    // the order of the sequence's first R points without a seed, per size R (see TableJob): made
+    // when a size comes a second time, kept until the context ends, for kMaxOrders sizes at most
+    struct Order {
+        uint32_t uses = 0;
+        uint32_t *dev = nullptr;
+        std::vector<uint64_t> keys;  // the sorted points, in 2^-64
+    };
+    std::map<uint32_t, Order> orders;
+    std::set<RayKey> host_only;  // tables that a pass could not make on the device
     std::map<RayKey, std::shared_ptr<const std::vector<double>>> lam_cache;  // wavelength u-points per (seed, W)
     // launch shape picked by the autotuner per class of batch
     std::map<std::array<uint64_t, 5>, std::pair<uint32_t, uint32_t>> tune_cache;
@@ -267,15 +280,18 @@ LamPtr lam_points_cached(cpd_context *ctx, double seed, uint32_t W)
     return ctx->lam_cache.emplace(key, v).first->second;
 }
 
-// One design's sampling inputs for a pass. lam_keep / rays_keep: set when lam_u / rays are
-// immutable tables of the context's caches (their device copies may then stay resident).
+// One design's sampling inputs for a pass: the points of a seed, or the caller's own.
 struct PassDesign {
     const DevDesign *dev;      // host copy
     uint32_t W, R;
-    const double *lam_u;       // W wavelength u-points (host), the first W of lam_len
-    const RayTable *rays;
-    std::shared_ptr<const void> lam_keep = nullptr, rays_keep = nullptr;
-    uint32_t lam_len = 0;      // length of the lam_u table (0: W)
+    bool seeded;
+    double seed;
+    const double *lam_u;       // !seeded: W wavelength u-points (host)
+    const double *ray_u;       // !seeded: R ray u-points (host)
+    // the ray table from the host; none: the pass makes it on the device from the points
+    // (rays_keep: a table of the context's cache; its device copy may then stay resident)
+    const RayTable *rays = nullptr;
+    RayTablePtr rays_keep = nullptr, rays_own = nullptr;
     // set instead of dev: the design is built on the device from this record (detector
     // positioned first when acceptance > 0; the same acceptance for every design of a pass)
     const cpd_spectrometer_params *params = nullptr;
@@ -284,8 +300,100 @@ struct PassDesign {
 
 struct PassResult {
     std::vector<DesignOut> outs;
-    bool overflow = false;
+    bool overflow = false;    // the re-trace queue was too small
+    bool bad_table = false;   // a ray table could not be made on the device
 };
+
+// Whether a pass may make the ray table on the device: its points lie in (0, 1), it fits
+// table_sort_kernel, and the trace does not read the f64 table.
+bool device_table(cpd_context *ctx, const PassDesign &p, uint32_t mode)
+{
+    if (p.R > kTableRays || (mode & ~kSamplingBits) == CPD_TRACE_FP64) return false;
+    if (p.seeded) {
+        if (!(p.seed >= 0.0 && p.seed < 1.0)) return false;
+        uint64_t bits;
+        std::memcpy(&bits, &p.seed, 8);
+        std::lock_guard<std::mutex> lk(ctx->cache_mu);
+        return ctx->host_only.empty() || !ctx->host_only.count(RayKey{bits, p.R});
+    }
+    bool in = true;
+    for (uint32_t j = 0; j < p.R; j++) in &= p.ray_u[j] > 0.0 && p.ray_u[j] < 1.0;
+    return in;
+}
+
+// The device's order of the sequence's first R points and, for a seed (in 2^-64), how far the
+// seed turns it; nullptr when the context does not keep this size (yet). The addresses stay
+// valid for the context's life, so passes in flight on any stream may read them.
+const uint32_t *point_order(cpd_context *ctx, uint32_t R, uint64_t seed_fixed, uint32_t &rot)
+{
+    std::lock_guard<std::mutex> lk(ctx->cache_mu);
+    auto it = ctx->orders.find(R);
+    if (it == ctx->orders.end()) {
+        if (ctx->orders.size() >= kMaxOrders) return nullptr;
+        it = ctx->orders.emplace(R, cpd_context::Order()).first;
+    }
+    cpd_context::Order &o = it->second;
+    if (!o.dev) {
+        if (++o.uses < 2u) return nullptr;
+        const uint64_t alpha = (uint64_t)(kAlpha * 18446744073709551616.0);
+        std::vector<std::pair<uint64_t, uint32_t>> kj(R);
+        for (uint32_t j = 0; j < R; j++) kj[j] = {alpha * (j + 1u), j};
+        std::sort(kj.begin(), kj.end());
+        std::vector<uint32_t> order(R);
+        std::vector<uint64_t> keys(R);
+        for (uint32_t i = 0; i < R; i++) {
+            keys[i] = kj[i].first;
+            order[i] = kj[i].second;
+        }
+        uint32_t *dev = nullptr;
+        if (cudaMalloc(&dev, sizeof(uint32_t) * R) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (cudaMemcpy(dev, order.data(), sizeof(uint32_t) * R, cudaMemcpyHostToDevice) != cudaSuccess) {
+            cudaFree(dev);
+            return nullptr;
+        }
+        o.keys.swap(keys);
+        o.dev = dev;
+    }
+    // the points that the seed carries past 1 come first
+    rot = seed_fixed ? (uint32_t)(std::lower_bound(o.keys.begin(), o.keys.end(), 0ull - seed_fixed) - o.keys.begin()) : 0u;
+    if (rot == R) rot = 0u;
+    return o.dev;
+}
+
+// The host's table for a design's points.
+void host_table(cpd_context *ctx, PassDesign &p)
+{
+    if (p.seeded) {
+        p.rays_keep = ray_table_cached(ctx, p.seed, p.R);
+        p.rays = p.rays_keep.get();
+    } else {
+        auto t = std::make_shared<RayTable>();
+        ray_table(p.ray_u, p.R, t->z64, t->z32, &t->rank);
+        p.rays_own = t;
+        p.rays = t.get();
+    }
+}
+
+void choose_table(cpd_context *ctx, PassDesign &p, uint32_t mode)
+{
+    if (!device_table(ctx, p, mode)) host_table(ctx, p);
+}
+
+// After a pass that reported a table the device could not make: its seeds' tables come from
+// the host from now on.
+void mark_host_only(cpd_context *ctx, const std::vector<std::pair<double, uint32_t>> &seeds)
+{
+    std::lock_guard<std::mutex> lk(ctx->cache_mu);
+    if (ctx->host_only.size() > 4096) ctx->host_only.clear();
+    for (const auto &s : seeds) {
+        uint64_t bits;
+        std::memcpy(&bits, &s.first, 8);
+        ctx->host_only.insert(RayKey{bits, s.second});
+    }
+}
 
 uint32_t tile_rows_for(uint32_t B, uint32_t n)
 {
@@ -313,13 +421,17 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     mode &= ~kSamplingBits;
     std::vector<DesignJob> jobs(n);
     std::vector<uint8_t> owns_rays(n, 1);  // designs that share a ray table share its copy
-    std::vector<uint8_t> owns_lam(n, 1);   // likewise for wavelength-point tables
-    std::map<const RayTable *, std::pair<uint64_t, uint64_t>> ray_offs;
+    std::vector<uint8_t> owns_lam(n, 1);   // likewise for the caller's wavelength points
+    // a table's identity: the host table or points it comes from, or its seed and size
+    using TableId = std::tuple<const void *, uint64_t, uint32_t>;
+    std::map<TableId, std::pair<uint64_t, uint64_t>> ray_offs;
     std::map<std::pair<const double *, uint32_t>, uint64_t> lam_offs;
+    std::vector<TableJob> tabs;
     // identity of the tables in upload order (null entries: not from a cache)
     std::vector<const void *> tables_key;
-    bool cacheable = true;
-    uint64_t rows = 0, groups = 0, hist = 0, cells = 0, lam = 0, ray = 0, rnk = 0, accc = 0, items = 0, tiles = 0;
+    bool cacheable = true, any_host = false;
+    uint32_t table_max = 0;
+    uint64_t rows = 0, groups = 0, hist = 0, cells = 0, lam = 0, upts = 0, ray = 0, rnk = 0, accc = 0, items = 0, tiles = 0;
     uint32_t max_B = 0;
     // a coated design under the fixed-N hybrid trace goes through rows_kernel (a device build
     // decides in its record whether the pieces apply; if not, its rays go through fast_ray there)
@@ -340,25 +452,49 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
         std::memset(&J, 0, sizeof(J));
         J.W = p.W;
         J.R = p.R;
-        J.Rz = (uint32_t)p.rays->z64.size();
+        J.Rz = p.rays ? (uint32_t)p.rays->z64.size() : p.R;
+        J.seeded = p.seeded ? 1u : 0u;
+        J.seed = p.seed;
         J.B = on_device ? p.params->bin_count : p.dev->B;
         J.row_off = rows;
-        const uint32_t lam_len = std::max(p.lam_len, p.W);
-        auto lo = lam_offs.emplace(std::make_pair(p.lam_u, lam_len), lam);
-        J.lam_off = lo.first->second;
-        owns_lam[i] = lo.second;
-        if (owns_lam[i]) {
-            lam += lam_len;
-            tables_key.push_back(p.lam_u);
-            cacheable = cacheable && p.lam_keep;
+        owns_lam[i] = 0;
+        if (!p.seeded) {
+            auto lo = lam_offs.emplace(std::make_pair(p.lam_u, p.W), lam);
+            J.lam_off = lo.first->second;
+            owns_lam[i] = lo.second;
+            if (owns_lam[i]) lam += p.W;
+            cacheable = false;  // the caller's points may change in place
         }
-        auto ro = ray_offs.emplace(p.rays, std::make_pair(ray, rnk));
+        uint64_t seed_bits = 0;
+        if (p.seeded) std::memcpy(&seed_bits, &p.seed, 8);
+        const TableId id = p.rays     ? TableId{p.rays, 0, 0}
+                           : p.seeded ? TableId{nullptr, seed_bits, p.R}
+                                      : TableId{p.ray_u, 1, p.R};
+        auto ro = ray_offs.emplace(id, std::make_pair(ray, rnk));
         J.ray_off = ro.first->second.first;
         J.rank_off = ro.first->second.second;
         owns_rays[i] = ro.second;
         if (owns_rays[i]) {
             tables_key.push_back(p.rays);
-            cacheable = cacheable && p.rays_keep;
+            tables_key.push_back(reinterpret_cast<const void *>(seed_bits));
+            tables_key.push_back(reinterpret_cast<const void *>((uintptr_t)p.R));
+            cacheable = cacheable && (!p.rays || p.rays_keep);
+            if (p.rays) {
+                any_host = true;
+            } else {
+                TableJob t{};
+                t.seed = p.seed;
+                t.seed_fixed = p.seeded ? (uint64_t)(p.seed * 18446744073709551616.0) : 0;
+                t.points = p.seeded ? 0u : 1u;
+                t.u_off = upts;
+                t.ray_off = ray;
+                t.rank_off = rnk;
+                t.R = p.R;
+                if (p.seeded) t.order = point_order(ctx, p.R, t.seed_fixed, t.rot);
+                else upts += p.R;
+                table_max = std::max(table_max, p.R);
+                tabs.push_back(t);
+            }
         }
         J.acc_off = accc;
         J.item_off = items;
@@ -385,21 +521,25 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
         if (!J.pieces) items += (uint64_t)((J.W + 31) / 32) * J.nchunk;
         if (!J.pieces) tiles += J.ntiles;
     }
-    // one input arena: wavelength points | z64 | z32 | ranks | designs | jobs (256-byte
-    // sections; the ranks only under adaptive sampling). The tables come first, so their
-    // offsets depend on the tables alone and a pass that finds them resident uploads the
-    // tail from the designs on.
+    // one input arena: z64 (FP64 study mode) | z32 | ranks (adaptive sampling) | wavelength
+    // points | ray points | designs | jobs | parameter records | table jobs | Control words, in
+    // 256-byte sections. A pass uploads its tail: from the z tables on where the host made one,
+    // from the points on where the caller gave them, else from the designs on; the tables that
+    // it makes on the device, and those resident from the previous pass, are not uploaded.
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t o_lam = 0;
-    const size_t o_z64 = o_lam + al(sizeof(double) * lam);
-    const size_t o_z32 = o_z64 + al(sizeof(double) * ray);
+    const bool f64 = mode == CPD_TRACE_FP64;
+    const size_t o_z64 = 0;
+    const size_t o_z32 = o_z64 + (f64 ? al(sizeof(double) * ray) : 0);
     const size_t o_rank = o_z32 + al(2 * sizeof(float) * ray);
-    const size_t o_des = o_rank + al(sizeof(uint32_t) * rnk);
+    const size_t o_lam = o_rank + al(sizeof(uint32_t) * rnk);
+    const size_t o_u = o_lam + al(sizeof(double) * lam);
+    const size_t o_des = o_u + al(sizeof(double) * upts);
     const size_t o_job = o_des + al(sizeof(DevDesign) * n);
     const size_t o_par = o_job + al(sizeof(DesignJob) * n);  // parameter records (device builds)
+    const size_t o_tab = o_par + (on_device ? al(sizeof(cpd_spectrometer_params) * n) : 0);
     // the pass's Control words close the arena: uploaded as zeros with the inputs (one copy
     // node instead of a copy and a memset ahead of the first kernel)
-    const size_t o_ctl = o_par + (on_device ? al(sizeof(cpd_spectrometer_params) * n) : 0);
+    const size_t o_ctl = o_tab + al(sizeof(TableJob) * tabs.size());
     const size_t in_bytes = o_ctl + sizeof(Control);
     const size_t ctl_off = al(sizeof(DesignOut) * n);
     const size_t out_bytes = ctl_off + sizeof(HostStatus);
@@ -409,42 +549,51 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     CPD_TRY(S.in.ensure(in_bytes));
     // the tables already on the device from the previous pass of this slot
     tables_key.push_back(adaptive ? &kSamplingBits : nullptr);  // the rank section
+    tables_key.push_back(f64 ? &kSamplingBits : nullptr);       // the z64 section
     tables_key.push_back(S.in.p);
     const bool resident = cacheable && S.in.p == in_before && tables_key == S.tables_key;
     // a device build writes the design records itself: they are not uploaded
-    const size_t up_off = resident ? (on_device ? o_job : o_des) : 0, up_bytes = in_bytes - up_off;
+    const size_t up_off = any_host && !resident ? 0 : lam || upts ? o_lam : on_device ? o_job : o_des;
+    const size_t up_bytes = in_bytes - up_off;
     char *hin = S.h_in.as<char>();
     std::memset(hin + o_ctl, 0, sizeof(Control));
     for (uint32_t i = 0; i < n; i++) {
         if (on_device) reinterpret_cast<cpd_spectrometer_params *>(hin + o_par)[i] = *ds[i].params;
         else reinterpret_cast<DevDesign *>(hin + o_des)[i] = *ds[i].dev;
         reinterpret_cast<DesignJob *>(hin + o_job)[i] = jobs[i];
-        if (resident) continue;
         if (owns_lam[i])
-            std::memcpy(reinterpret_cast<double *>(hin + o_lam) + jobs[i].lam_off, ds[i].lam_u,
-                        sizeof(double) * std::max(ds[i].lam_len, ds[i].W));
-        if (!owns_rays[i]) continue;
-        std::memcpy(reinterpret_cast<double *>(hin + o_z64) + jobs[i].ray_off, ds[i].rays->z64.data(),
-                    sizeof(double) * jobs[i].Rz);
+            std::memcpy(reinterpret_cast<double *>(hin + o_lam) + jobs[i].lam_off, ds[i].lam_u, sizeof(double) * jobs[i].W);
+        if (resident || !owns_rays[i]) continue;
+        if (!ds[i].rays) continue;
+        if (f64)
+            std::memcpy(reinterpret_cast<double *>(hin + o_z64) + jobs[i].ray_off, ds[i].rays->z64.data(),
+                        sizeof(double) * jobs[i].Rz);
         std::memcpy(reinterpret_cast<float *>(hin + o_z32) + 2 * jobs[i].ray_off, ds[i].rays->z32.data(),
                     2 * sizeof(float) * jobs[i].Rz);
         if (adaptive)
             std::memcpy(reinterpret_cast<uint32_t *>(hin + o_rank) + jobs[i].rank_off, ds[i].rays->rank.data(),
                         sizeof(uint32_t) * jobs[i].R);
     }
+    if (resident) tabs.clear();
+    const uint32_t nsort =
+        (uint32_t)(std::stable_partition(tabs.begin(), tabs.end(), [](const TableJob &t) { return !t.order; }) - tabs.begin());
+    if (!tabs.empty()) std::memcpy(hin + o_tab, tabs.data(), sizeof(TableJob) * tabs.size());
+    for (uint32_t i = 0; i < n; i++)
+        if (owns_rays[i] && !ds[i].rays && !ds[i].seeded)
+            for (const TableJob &t : tabs)
+                if (t.points && t.ray_off == jobs[i].ray_off)
+                    std::memcpy(reinterpret_cast<double *>(hin + o_u) + t.u_off, ds[i].ray_u, sizeof(double) * t.R);
     if (cacheable) {
         S.tables_key = tables_key;
         S.tables_refs.clear();
-        for (const PassDesign &p : ds) {
-            S.tables_refs.push_back(p.lam_keep);
-            S.tables_refs.push_back(p.rays_keep);
-        }
+        for (const PassDesign &p : ds)
+            if (p.rays_keep) S.tables_refs.push_back(p.rays_keep);
     } else {
         S.tables_key.clear();
         S.tables_refs.clear();
     }
     // device buffers (a reallocation retires the captured graphs that hold the old addresses)
-    const void *bufs_before[] = {S.lp.p, S.lx.p, S.hist.p, S.S1.p, S.S2.p, S.acc.p, S.queue.p, S.h_in.p, S.h_outs.p, in_before};
+    const void *bufs_before[] = {S.lp.p, S.lx.p, S.hist.p, S.S1.p, S.S2.p, S.acc.p, S.queue.p, S.h_in.p, S.h_outs.p, S.perm.p, in_before};
     const size_t hist_bytes = sizeof(unsigned long long) * std::max<uint64_t>(hist, 1);
     const size_t old_hist = S.hist.cap;
     // the LamParams, then (single-design passes) one span per 32-row block
@@ -457,9 +606,10 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     CPD_TRY(S.acc.ensure(sizeof(DesignAcc) * n));
     CPD_TRY(S.queue.ensure(sizeof(QEntry) * S.qcap));
     if (p_out_host) CPD_TRY(S.pout.ensure(sizeof(double) * cells));
+    CPD_TRY(S.perm.ensure(sizeof(uint32_t) * std::max<uint64_t>(nsort ? ray : 1, 1)));
     S.ctl_off = ctl_off;
     {
-        const void *after[] = {S.lp.p, S.lx.p, S.hist.p, S.S1.p, S.S2.p, S.acc.p, S.queue.p, S.h_in.p, S.h_outs.p, S.in.p};
+        const void *after[] = {S.lp.p, S.lx.p, S.hist.p, S.S1.p, S.S2.p, S.acc.p, S.queue.p, S.h_in.p, S.h_outs.p, S.perm.p, S.in.p};
         if (!std::equal(std::begin(after), std::end(after), std::begin(bufs_before))) S.buf_gen++;
     }
 
@@ -485,6 +635,12 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     a.lam_u = reinterpret_cast<const double *>(din + o_lam);
     a.z64 = reinterpret_cast<const double *>(din + o_z64);
     a.z32 = reinterpret_cast<const float *>(din + o_z32);
+    a.tables = reinterpret_cast<const TableJob *>(din + o_tab);
+    a.ntables = (uint32_t)tabs.size();
+    a.nsort = nsort;
+    a.table_max = tabs.empty() ? 0u : table_max;
+    a.ray_u = reinterpret_cast<const double *>(din + o_u);
+    a.perm = S.perm.as<uint32_t>();
     a.rank = adaptive ? reinterpret_cast<const uint32_t *>(din + o_rank) : nullptr;
     a.adaptive = adaptive ? (all_exact ? 2u : 1u) : 0u;
     a.max_B = max_B;
@@ -522,6 +678,7 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
         a.fc = ds[0].dev->fc;
         a.fl = fast_limits(a.fc, a.guards);
         a.one = jobs[0];
+        a.one.seed = 0.0;  // not part of the graph: read from the uploaded job
     }
     a.p_out = p_out_host ? S.pout.as<double>() : nullptr;
     a.logtab = ctx->logtab.as<float>();
@@ -535,14 +692,14 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     // timing events around the kernels -- is one graph, captured once per signature.
     // The design constants of a single-design pass are not part of the key: the cached
     // graph's trace node gets them per call.
-    std::vector<uint8_t> key(sizeof(a) + 8 * sizeof(uint64_t));
+    std::vector<uint8_t> key(sizeof(a) + 9 * sizeof(uint64_t));
     {
         LaunchArgs ka = a;
         std::memset(&ka.fc, 0, sizeof(ka.fc));
         std::memset(&ka.fl, 0, sizeof(ka.fl));
         std::memcpy(key.data(), &ka, sizeof(ka));
     }
-    const uint64_t extra[8] = {n, ctx->warps_per_cta, (uint64_t)ctx->num_sms, (in_bytes << 1) | (resident ? 1u : 0u),
+    const uint64_t extra[9] = {n, ctx->warps_per_cta, (uint64_t)ctx->num_sms, in_bytes, up_off,
                                out_bytes, fresh ? accc + 1 : 0, S.buf_gen, (uint64_t)(uintptr_t)S.h_in.p};
     std::memcpy(key.data() + sizeof(a), extra, sizeof(extra));
     auto record = [&](cudaStream_t st, bool capturing) -> int {
@@ -632,8 +789,10 @@ int pass_finish(PassSlot &S, PassResult &res)
             S.kernel_ms[i] = km;
         }
     const HostStatus *c = reinterpret_cast<const HostStatus *>(S.h_outs.as<char>() + S.ctl_off);
-    res.overflow = c->overflow != 0 || c->queue_count > S.qcap;
-    if (res.overflow) S.hist_dirty = true;
+    res.overflow = (c->overflow & kOverflowQueue) != 0 || c->queue_count > S.qcap;
+    res.bad_table = (c->overflow & kOverflowTable) != 0;
+    if (res.overflow || res.bad_table) S.hist_dirty = true;
+    if (res.bad_table) S.tables_key.clear();
     res.outs.assign(S.h_outs.as<DesignOut>(), S.h_outs.as<DesignOut>() + S.n);
     return CPD_OK;
 }
@@ -688,15 +847,28 @@ bool valid_item(const cpd_batch_item &it)
 // Runs one pass on `S` to completion, growing the re-trace queue and re-running the
 // pass if it overflowed. A pass that overflowed leaves the persistent accumulators
 // untouched (the entropy kernel skips such a pass), so the re-run is exact.
-int run_pass_checked(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds, uint32_t mode, bool fresh,
+int run_pass_checked(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &pds, uint32_t mode, bool fresh,
                      double *p_out, PassResult &res, bool use_graph)
 {
-    for (int attempt = 0; attempt < 6; attempt++) {
+    std::vector<PassDesign> by_host;  // the same designs with the host's tables
+    for (int attempt = 0; attempt < 7; attempt++) {
+        const std::vector<PassDesign> &ds = by_host.empty() ? pds : by_host;
         int e = pass_issue(ctx, S, ds, mode, fresh, p_out, use_graph, ctx->profiling);
         if (!e) e = pass_finish(S, res);
         if (e) {
             S.hist_dirty = true;
             return e;
+        }
+        if (res.bad_table) {
+            std::vector<std::pair<double, uint32_t>> seeds;
+            by_host = pds;
+            for (PassDesign &p : by_host) {
+                if (p.rays) continue;
+                if (p.seeded) seeds.emplace_back(p.seed, p.R);
+                host_table(ctx, p);
+            }
+            mark_host_only(ctx, seeds);
+            continue;
         }
         if (!res.overflow) return CPD_OK;
         S.qcap *= 4;
@@ -747,7 +919,7 @@ int tune_pass(cpd_context *ctx, const std::vector<PassDesign> &ds, uint32_t mode
         uint64_t blocks = 0, rays = 0;
         for (const PassDesign &p : ds) {
             blocks += (p.W + 31) / 32;
-            rays += (uint64_t)((p.W + 31) / 32) * p.rays->z64.size();
+            rays += (uint64_t)((p.W + 31) / 32) * (p.rays ? p.rays->z64.size() : p.R);
         }
         const uint64_t warps = trace_resident_warps(ctx->num_sms, w);
         for (uint64_t k = 2; k <= 6 && blocks; k++) {
@@ -784,21 +956,28 @@ int tune_pass(cpd_context *ctx, const std::vector<PassDesign> &ds, uint32_t mode
     return CPD_OK;
 }
 
+// A pass's design under the seed policy.
+PassDesign seeded_design(cpd_context *ctx, const DevDesign *dev, double seed, uint32_t W, uint32_t R, uint32_t mode)
+{
+    PassDesign p{};
+    p.dev = dev;
+    p.W = W;
+    p.R = R;
+    p.seeded = true;
+    p.seed = seed;
+    choose_table(ctx, p, mode);
+    return p;
+}
+
 // Builds the pass inputs of a batch (host copies kept alive by the caller's vectors).
-void batch_inputs(cpd_context *ctx, const cpd_design *designs, const cpd_batch_item *items, uint32_t n,
-                  std::vector<DevDesign> &devs, std::vector<LamPtr> &lams, std::vector<RayTablePtr> &rts,
-                  std::vector<PassDesign> &ds)
+void batch_inputs(cpd_context *ctx, const cpd_design *designs, const cpd_batch_item *items, uint32_t n, uint32_t mode,
+                  std::vector<DevDesign> &devs, std::vector<PassDesign> &ds)
 {
     devs.resize(n);
-    lams.resize(n);
-    rts.resize(n);
-    ds.resize(n);
+    ds.reserve(n);
     for (uint32_t i = 0; i < n; i++) {
         design_to_dev(designs[i], devs[i]);
-        lams[i] = lam_points_cached(ctx, items[i].seed, items[i].max_n);
-        rts[i] = ray_table_cached(ctx, items[i].seed, items[i].max_eval);
-        ds[i] = PassDesign{&devs[i], items[i].max_n, items[i].max_eval, lams[i]->data(), rts[i].get(), lams[i], rts[i],
-                           (uint32_t)lams[i]->size()};
+        ds.push_back(seeded_design(ctx, &devs[i], items[i].seed, items[i].max_n, items[i].max_eval, mode));
     }
 }
 
@@ -863,10 +1042,18 @@ void srv_complete(cpd_server *sv, size_t i)
     int e = pass_finish(S, res);
     std::lock_guard<std::mutex> lk(sv->mu);
     auto &work = sv->slot_work[i];
-    if (!e && res.overflow) e = CPD_NO_CAPACITY;  // re-queued below with a larger queue
+    if (!e && (res.overflow || res.bad_table)) e = CPD_NO_CAPACITY;  // re-queued below
     if (e == CPD_NO_CAPACITY && S.qcap < (1u << 26)) {
-        // grow the re-trace queue and run the same designs again
-        S.qcap *= 4;
+        // run the same designs again, with a larger re-trace queue or the host's tables
+        if (res.overflow) S.qcap *= 4;
+        if (res.bad_table) {
+            std::vector<std::pair<double, uint32_t>> seeds;
+            for (const SrvWork &wk : work) {
+                auto rit = sv->reqs.find(wk.req);
+                if (rit != sv->reqs.end()) seeds.emplace_back(rit->second.items[wk.idx].seed, rit->second.items[wk.idx].max_eval);
+            }
+            mark_host_only(sv->ctx, seeds);
+        }
         for (auto it = work.rbegin(); it != work.rend(); ++it) {
             sv->in_use -= it->bytes;
             sv->pending.push_front(*it);
@@ -916,8 +1103,6 @@ void srv_loop(cpd_server *sv)
         for (size_t i = 0; i < sv->slots.size(); i++) {
             std::vector<SrvWork> take;
             std::vector<DevDesign> devs;
-            std::vector<LamPtr> lams;
-            std::vector<RayTablePtr> rays;
             uint32_t mode = 0;
             {
                 std::lock_guard<std::mutex> lk(sv->mu);
@@ -949,8 +1134,6 @@ void srv_loop(cpd_server *sv)
             // host preparation and issue without the lock (the slot belongs to the worker)
             std::vector<PassDesign> ds(take.size());
             devs.resize(take.size());
-            lams.resize(take.size());
-            rays.resize(take.size());
             for (size_t k = 0; k < take.size(); k++) {
                 const SrvRequest *r;
                 {
@@ -959,10 +1142,7 @@ void srv_loop(cpd_server *sv)
                 }
                 const cpd_batch_item &it = r->items[take[k].idx];
                 if (r->params.empty()) design_to_dev(r->designs[take[k].idx], devs[k]);
-                lams[k] = lam_points_cached(sv->ctx, it.seed, it.max_n);
-                rays[k] = ray_table_cached(sv->ctx, it.seed, it.max_eval);
-                ds[k] = PassDesign{&devs[k], it.max_n, it.max_eval, lams[k]->data(), rays[k].get(), lams[k], rays[k],
-                                   (uint32_t)lams[k]->size()};
+                ds[k] = seeded_design(sv->ctx, &devs[k], it.seed, it.max_n, it.max_eval, mode);
                 if (!r->params.empty()) {
                     ds[k].dev = nullptr;
                     ds[k].params = &r->params[take[k].idx];
@@ -1039,6 +1219,8 @@ void cpd_context_destroy(cpd_context *ctx)
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     ctx->main.destroy();
+    for (auto &o : ctx->orders)
+        if (o.second.dev) cudaFree(o.second.dev);
     for (DevBuf *b : {&ctx->tp_design, &ctx->tp_lam, &ctx->tp_z, &ctx->tp_out, &ctx->tp_rays})
         b->release();
     for (DevBuf *b : {&ctx->bld_params, &ctx->bld_out, &ctx->bld_status, &ctx->pair_design, &ctx->pair_lam,
@@ -1113,9 +1295,13 @@ int cpd_fitness_gpu_points(cpd_context *ctx, const cpd_design *d, const double *
     CPD_SYNC_ENTRY(ctx);
     DevDesign D;
     design_to_dev(*d, D);
-    RayTable rt;
-    ray_table(ray_u, R, rt.z64, rt.z32, &rt.rank);
-    std::vector<PassDesign> ds{PassDesign{&D, W, R, lam_u, &rt}};
+    std::vector<PassDesign> ds(1);
+    ds[0].dev = &D;
+    ds[0].W = W;
+    ds[0].R = R;
+    ds[0].lam_u = lam_u;
+    ds[0].ray_u = ray_u;
+    choose_table(ctx, ds[0], trace_mode);
     PassResult res;
     int e = run_pass_checked(ctx, ctx->main, ds, trace_mode, true, p_out, res, ctx->use_graphs);
     if (e) return e;
@@ -1146,10 +1332,7 @@ int cpd_fitness_gpu_ex(cpd_context *ctx, const cpd_design *d, const double *seed
     PassResult res;
     uint64_t rays = 0;
     for (uint32_t s = 0; s < nseeds; s++) {
-        const auto lam = lam_points_cached(ctx, seeds[s], max_n);
-        RayTablePtr rt = ray_table_cached(ctx, seeds[s], max_eval);
-        std::vector<PassDesign> ds{
-            PassDesign{&D, max_n, max_eval, lam->data(), rt.get(), lam, rt, (uint32_t)lam->size()}};
+        const std::vector<PassDesign> ds{seeded_design(ctx, &D, seeds[s], max_n, max_eval, mode)};
         if (tune && s == 0) {
             // the autotuner replaces the reference's nwarp hint
             auto it = ctx->tune_cache.find(tune_class(ds, mode));
@@ -1178,10 +1361,8 @@ int cpd_fitness_gpu_batch(cpd_context *ctx, const cpd_design *designs, const cpd
         if (!valid_design(&designs[i]) || !valid_item(items[i])) return CPD_INVALID_ARGUMENT;
     CPD_SYNC_ENTRY(ctx);
     std::vector<DevDesign> devs;
-    std::vector<LamPtr> lams;
-    std::vector<RayTablePtr> rts;
     std::vector<PassDesign> ds;
-    batch_inputs(ctx, designs, items, n, devs, lams, rts, ds);
+    batch_inputs(ctx, designs, items, n, trace_mode, devs, ds);
     if (ctx->autotune && !ctx->profiling && !is_adaptive(trace_mode)) {
         auto it = ctx->tune_cache.find(tune_class(ds, trace_mode));
         if (it != ctx->tune_cache.end()) {
@@ -1210,14 +1391,12 @@ int cpd_fitness_gpu_batch_params(cpd_context *ctx, const cpd_spectrometer_params
     for (uint32_t i = 0; i < n; i++)
         if (!valid_params(params[i]) || !valid_item(items[i])) return CPD_INVALID_ARGUMENT;
     CPD_SYNC_ENTRY(ctx);
-    std::vector<LamPtr> lams(n);
-    std::vector<RayTablePtr> rts(n);
-    std::vector<PassDesign> ds(n);
+    std::vector<PassDesign> ds;
+    ds.reserve(n);
     for (uint32_t i = 0; i < n; i++) {
-        lams[i] = lam_points_cached(ctx, items[i].seed, items[i].max_n);
-        rts[i] = ray_table_cached(ctx, items[i].seed, items[i].max_eval);
-        ds[i] = PassDesign{nullptr, items[i].max_n, items[i].max_eval, lams[i]->data(), rts[i].get(), lams[i], rts[i],
-                           (uint32_t)lams[i]->size(), &params[i], acceptance};
+        ds.push_back(seeded_design(ctx, nullptr, items[i].seed, items[i].max_n, items[i].max_eval, trace_mode));
+        ds[i].params = &params[i];
+        ds[i].acceptance = acceptance;
     }
     if (ctx->autotune && !ctx->profiling && !is_adaptive(trace_mode)) {
         auto it = ctx->tune_cache.find(tune_class(ds, trace_mode));
@@ -1269,10 +1448,8 @@ int cpd_autotune_batch(cpd_context *ctx, const cpd_design *designs, const cpd_ba
         if (!valid_design(&designs[i]) || !valid_item(items[i])) return CPD_INVALID_ARGUMENT;
     CPD_SYNC_ENTRY(ctx);
     std::vector<DevDesign> devs;
-    std::vector<LamPtr> lams;
-    std::vector<RayTablePtr> rts;
     std::vector<PassDesign> ds;
-    batch_inputs(ctx, designs, items, n, devs, lams, rts, ds);
+    batch_inputs(ctx, designs, items, n, trace_mode, devs, ds);
     const int e = tune_pass(ctx, ds, trace_mode, best_ms);
     if (e) return e;
     if (ray_tile) *ray_tile = ctx->ray_tile;
