@@ -587,6 +587,16 @@ CPD_HDN inline bool trace_df_(const DevDesign &D, const LamDF &E, float zh, floa
     return false;
 }
 
+// 2^31 t of every ray of a wavelength that meets the coated exit face at cos > 0.5: what
+// trace_df_exact gives each of them.
+CPD_HDN inline uint32_t coated_tfix(const LamDF &E)
+{
+    using namespace df;
+    const F2 ar99{0.99f, -9.5367431640625e-09f};  // 0.99 = hi + lo to ~1e-17
+    const F2 s = add(mul(F2{E.ts, E.ts_lo}, ar99), mul(F2{E.tp, E.tp_lo}, ar99));
+    return t_fixed64(0.5 * ((double)s.hi + (double)s.lo));
+}
+
 // The re-trace of a flagged ray: bin and an FP32 transmittance.
 CPD_HDN inline bool trace_df(const DevDesign &D, const LamDF &E, float zh, float zl, uint32_t &bin, float &t)
 {

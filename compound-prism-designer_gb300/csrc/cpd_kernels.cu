@@ -1159,12 +1159,504 @@ __device__ bool adaptive_row1(const LaunchArgs &a, uint64_t row, unsigned long l
     return false;
 }
 
+// One wavelength row under adaptive sampling by one warp, for a design with certified pieces
+// (cpd_piece.h): the rounds and decisions of adaptive_row1 with the row's core range cut into up
+// to 31 pieces of 2^k sorted rays once, so that a ray's bin is a quadratic of its piece (~25
+// instructions against ~100 of fast_ray) and every such hit has the same transmittance. A bin's
+// Welford state is then its samples n and hits h alone, the test is sem_quick_equal, and the
+// shared-memory sums of q and q^2 drop out. The rays that the float-float trace decides hit with
+// a transmittance of its own: for p(d|lambda) the difference is summed apart (ox), and while it is
+// within kTqDelta quanta the test's error bound covers it.
+// kExact: every hit with the float-float transmittance (coated_tfix), the test without an error
+// bound. Returns ROW_DONE; ROW_UNSURE when the bound leaves a decision open (the caller redoes the
+// row with kExact); or ROW_OTHER when a hit's transmittance is another (an exit face met at
+// cos <= 0.5): the general exact path takes the row.
+enum : int { ROW_DONE = 0, ROW_UNSURE = 1, ROW_OTHER = 2 };
+struct Adapt1Pieces {
+    LamParams P;
+    FastConst C;
+    // the pieces, then the eighths of up to three pieces without a bound
+    float4 rec_a[32 + 24];  // z of the left end (hi, lo), v0, v1; of a cut piece its first eighth's place
+    float2 rec_b[32 + 24];  // v2, e (kCutPiece: cut)
+};
+constexpr float kCutPiece = 2e30f;  // an error beyond that of piece_uniform's pieces without a bound
+// per bin: ox, samples and hits
+constexpr size_t adapt1p_smem_bytes(uint32_t B) { return sizeof(Adapt1Pieces) + 16u * (size_t)B; }
+
+// A row for adaptive_exact_kernel.
+__device__ __forceinline__ void queue_row(const LaunchArgs &a, uint64_t row)
+{
+    const uint32_t d = find_job<F_ROW>(a.jobs, a.njobs, row);
+    const unsigned long long pos = atomicAdd(&a.ctl->queue_count, 1ull);
+    if (pos < a.qcap) a.queue[pos] = QEntry{d, (uint32_t)(row - a.jobs[d].row_off), 0u, 0u};
+    else atomicOr(&a.ctl->overflow, kOverflowQueue);
+}
+
+// The records of a row's pieces, by one warp.
+__device__ __forceinline__ void adapt_pieces(const LaunchArgs &a, Adapt1Pieces &w, const PieceConst &K,
+                                             const float2 *__restrict__ zt, uint32_t lo, uint32_t hi, uint32_t ks,
+                                             uint32_t lane)
+{
+    const LamParams &P = w.P;
+    const FastConst &C = w.C;
+    // the pieces, and then again the pieces without a bound in eighths (nine ends each): of
+    // 81 rays in such pieces per row of 7591, nine in ten are decided
+    uint32_t j0 = lo + (lane << ks), cut = 0u;
+    for (int level = 0; level < 2; level++) {
+        if (level) {
+            const uint32_t g = lane / 9u, t = lane - 9u * g;
+            uint32_t m = cut;
+            for (uint32_t i = 0; i < g; i++) m &= m - 1u;
+            const uint32_t p = g < 3u && m ? (uint32_t)__ffs(m) - 1u : 0u;
+            j0 = min(lo + (p << ks) + (t << (ks - 3u)), min(lo + ((p + 1u) << ks), hi - 1u));
+        }
+        const float2 z = __ldg(zt + min(j0, hi - 1u));
+        const PieceEnd e = piece_end(C, fast_limits(C, a.guards), K, P, a.guards, z.x, z.y);
+        PieceEnd o = e;
+        o.dz = __shfl_down_sync(0xffffffffu, e.dz, 1);
+        o.v = __shfl_down_sync(0xffffffffu, e.v, 1);
+        o.gv = __shfl_down_sync(0xffffffffu, e.gv, 1);
+        o.ci = __shfl_down_sync(0xffffffffu, e.ci, 1);
+        o.cr = __shfl_down_sync(0xffffffffu, e.cr, 1);
+        o.cid = __shfl_down_sync(0xffffffffu, e.cid, 1);
+        o.gn = __shfl_down_sync(0xffffffffu, e.gn, 1);
+        o.px = __shfl_down_sync(0xffffffffu, e.px, 1);
+        o.py = __shfl_down_sync(0xffffffffu, e.py, 1);
+        o.cls = __shfl_down_sync(0xffffffffu, e.cls, 1);
+        const Piece f = piece_fit(C, K, P, e, o);
+        const Piece q = piece_uniform(K, f);
+        if (level == 0) {
+            w.rec_a[lane] = make_float4(z.x, z.y, q.v0, q.v1);
+            w.rec_b[lane] = make_float2(q.v2, q.e);
+            cut = ks >= 3u ? __ballot_sync(0xffffffffu, lane < 31u && j0 < hi && f.cls == PIECE_RAYS) : 0u;
+            if (!cut) break;
+            // their records point to their eighths
+            const uint32_t place = __popc(cut & ((1u << lane) - 1u));
+            __syncwarp();
+            if ((cut >> lane & 1u) && place < 3u) {
+                w.rec_a[lane].x = __uint_as_float(32u + 8u * place);
+                w.rec_b[lane].y = kCutPiece;
+            }
+        } else {
+            const uint32_t g = lane / 9u, t = lane - 9u * g;
+            if (g < 3u && t < 8u) {
+                w.rec_a[32u + 8u * g + t] = make_float4(z.x, z.y, q.v0, q.v1);
+                w.rec_b[32u + 8u * g + t] = make_float2(q.v2, q.e);
+            }
+        }
+    }
+}
+
+// A core ray (sorted position s) on its piece: piece_ray's outcome and the bin.
+__device__ __forceinline__ int adapt_ray(const Adapt1Pieces &w, const PieceConst &K, uint32_t B, uint32_t s, uint32_t lo,
+                                         uint32_t ks, float2 z, uint32_t &bin)
+{
+    const uint32_t i = (s - lo) >> ks;
+    float4 ra = w.rec_a[i];
+    float2 rb = w.rec_b[i];
+    if (rb.y >= kCutPiece) {
+        const uint32_t c = __float_as_uint(ra.x) + ((s - lo) >> (ks - 3u) & 7u);
+        ra = w.rec_a[c];
+        rb = w.rec_b[c];
+    }
+    return piece_ray(K, B, 0.f, ra.z, ra.w, rb.x, rb.y, (ra.x - z.x) + (ra.y - z.y), bin);
+}
+
+// A ray that the pieces leave: fast_ray in the core, and the float-float trace. False when it hits
+// with another transmittance than the row's (tfast by fast_ray, tfix in float-float, which is what
+// a float-float hit gives); add: what its hit adds to the bin beside tfast (kExact: nothing).
+template <bool kExact>
+__device__ __forceinline__ bool adapt_left(const LaunchArgs &a, const DevDesign &D, const Adapt1Pieces &w, const LamDF &E,
+                                           bool core, float2 z, uint32_t tfast, uint32_t tfix, uint32_t &bin,
+                                           bool &used_df, long long &add)
+{
+    int r = RAY_FLAG;
+    if (core) {
+        uint32_t b = 0u;
+        float t = 0.f;
+        r = fast_ray(w.C, w.P, a.guards, z.x, z.y, b, t);
+        if (r == RAY_HIT) {
+            bin = b;
+            return t_fixed(t) == tfast;
+        }
+    }
+    if (r != RAY_FLAG) return true;
+    const uint2 x = trace_df_exact_call(D, E, z.x, z.y);
+    bin = x.x;
+    used_df = true;
+    if (bin == 0xffffffffu) return true;
+    if (!kExact) add = (long long)x.y - (long long)tfast;
+    return x.y == tfix;
+}
+
+template <bool kExact>
+__device__ __forceinline__ int adaptive_row1_pieces(const LaunchArgs &a, uint64_t row, uint32_t d,
+                                                         const DesignJob &J, unsigned long long *smem, uint32_t lane)
+{
+    const uint32_t k = (uint32_t)(row - J.row_off);
+    const uint32_t B = J.B, R = J.R;
+    const DevDesign &D = a.designs[d];
+    Adapt1Pieces &w = *reinterpret_cast<Adapt1Pieces *>(smem);
+    LamParams &P = w.P;
+    FastConst &C = w.C;
+    unsigned long long *ox = reinterpret_cast<unsigned long long *>(&w + 1);
+    uint2 *st = reinterpret_cast<uint2 *>(ox + B);  // samples, hits
+    const LamDF &E = a.lx[row];
+    static_assert(sizeof(Adapt1Pieces) % 16 == 0, "bin arrays follow");
+    if (lane < sizeof(LamParams) / 16)
+        reinterpret_cast<uint4 *>(&P)[lane] = reinterpret_cast<const uint4 *>(a.lp + row)[lane];
+    else if (lane < (sizeof(LamParams) + sizeof(FastConst)) / 16)
+        reinterpret_cast<uint4 *>(&C)[lane - sizeof(LamParams) / 16] =
+            reinterpret_cast<const uint4 *>(&D.fc)[lane - sizeof(LamParams) / 16];
+    for (uint32_t b = lane; b < B; b += 32u) {
+        st[b] = make_uint2(0u, 0u);
+        ox[b] = 0ull;
+    }
+    __syncwarp();
+    const uint32_t *rank = a.rank + J.rank_off;
+    const float2 *__restrict__ zt = reinterpret_cast<const float2 *>(a.z32) + J.ray_off;
+    const PieceConst K = piece_const(C);
+    const uint32_t lo = P.core_lo, hi = P.all_exact ? P.core_lo : P.core_hi, band_lo = P.band_lo, band_hi = P.band_hi;
+    const uint32_t ks = piece_shift(hi - lo);
+    if (hi > lo) adapt_pieces(a, w, K, zt, lo, hi, ks, lane);
+    __syncwarp();
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    const uint32_t tfast = piece_tfix(P), tfix = coated_tfix(E), tfx = kExact ? tfix : tfast, tq = tfx >> kTqShift;
+    constexpr uint32_t delta = kExact ? 0u : kTqDelta;
+    if (!kExact && (tfix >> kTqShift) - tq + kTqDelta > 2u * kTqDelta) return ROW_OTHER;
+    const SemEqual se = sem_equal(tq, delta);
+    uint32_t count = R, ndf = 0;  // the same in every lane
+    // no ray clears the flat faces: every round runs without a hit
+    const uint32_t g_start = band_lo >= band_hi ? R : 0u;
+    // the ray this lane traces in the next round and its start height, loaded while the current
+    // one is decided; its place in the table a round before that (the second load's address)
+    uint32_t s_n1 = 0xffffffffu, s_n2 = 0xffffffffu;
+    float2 z_n1 = make_float2(0.f, 0.f);
+    const auto place = [&](uint32_t g) { return g + lane < R ? __ldg(rank + g + lane) : 0xffffffffu; };
+    const auto height = [&](uint32_t s) { return s >= band_lo && s < band_hi ? __ldg(zt + s) : make_float2(0.f, 0.f); };
+    if (g_start < R) {
+        s_n1 = place(g_start);
+        s_n2 = place(g_start + kRoundRays);
+        z_n1 = height(s_n1);
+    }
+    for (uint32_t g0 = g_start; g0 < R; g0 += kRoundRays) {
+        uint32_t bin = 0xffffffffu;
+        const uint32_t s = s_n1;
+        const float2 z = z_n1;
+        s_n1 = s_n2;
+        z_n1 = height(s_n1);
+        s_n2 = place(g0 + 2u * kRoundRays);
+        int res = RAY_LOST;
+        const bool core = s >= lo && s < hi;
+        if (core) {
+            uint32_t b = 0u;
+            res = adapt_ray(w, K, B, s, lo, ks, z, b);
+            if (res == RAY_HIT) bin = b;
+        } else if (s >= band_lo && s < band_hi) {
+            res = RAY_FLAG;
+        }
+        bool used_df = false;
+        const uint32_t left = __ballot_sync(0xffffffffu, res == RAY_FLAG);
+        if (left) {
+            // the rays that the pieces leave
+            bool same = true;
+            long long add = 0;
+            if (res == RAY_FLAG) same = adapt_left<kExact>(a, D, w, E, core, z, tfast, tfix, bin, used_df, add);
+            if (!__all_sync(0xffffffffu, same)) return ROW_OTHER;
+            if (add) atomicAdd(ox + bin, (unsigned long long)add);
+        }
+        const bool hit = bin != 0xffffffffu;
+        const uint32_t hm = __ballot_sync(0xffffffffu, hit);
+        const uint32_t rn = min(kRoundRays, R - g0);  // samples of this round
+        const uint32_t grp = __match_any_sync(0xffffffffu, bin);
+        const bool leader = hit && (grp & lt_mask) == 0u;
+        int verdict = SEM_PASS;
+        uint32_t cn = 0u, ch = 0u;
+        if (leader) {
+            const uint2 v = st[bin];
+            cn = v.x + rn;
+            ch = v.y + (uint32_t)__popc(grp);
+            st[bin] = make_uint2(cn, ch);
+            verdict = sem_quick_equal(cn, ch, se);
+        }
+        if (kExact) ndf += (uint32_t)__popc(__ballot_sync(0xffffffffu, s >= band_lo && s < band_hi));
+        else if (left) ndf += (uint32_t)__popc(__ballot_sync(0xffffffffu, used_df));
+        // the row goes on when a bin fails (most rounds), or no ray hit
+        if (!hm || __any_sync(0xffffffffu, verdict == SEM_FAIL)) continue;
+        if (verdict < 0) verdict = sem_test(cn, ch, (uint64_t)ch * tq, (uint64_t)ch * tq * tq, delta);
+        if (!__any_sync(0xffffffffu, verdict == SEM_FAIL)) {
+            if (__any_sync(0xffffffffu, verdict == SEM_UNSURE)) return ROW_UNSURE;
+            count = g0 + rn;
+            break;
+        }
+    }
+    __syncwarp();
+    uint32_t hits = 0u;
+    unsigned long long *hrow = a.hist + J.hist_off + (uint64_t)k * B;
+    for (uint32_t b = lane; b < B; b += 32u) {
+        const uint32_t h = st[b].y;
+        hits += h;
+        if (h) hrow[b] = rescale_cell((unsigned long long)h * tfx + ox[b], R, count);
+    }
+    hits = __reduce_add_sync(0xffffffffu, hits);
+    if (lane == 0) {
+        const uint32_t sp = (uint32_t)(row % (uint64_t)kSpread);
+        atomicAdd(&a.acc[d].fast[sp], (unsigned long long)count);
+        if (hits) atomicAdd(&a.acc[d].hits[sp], (unsigned long long)hits);
+        if (ndf) atomicAdd(&a.acc[d].retraced[sp], (unsigned long long)ndf);
+    }
+    return ROW_DONE;
+}
+
 #ifndef CPD_ADAPT_KW_MANY
 #define CPD_ADAPT_KW_MANY 1  // warps per row when at least 8 rows per SM (1: adaptive1_kernel)
 #endif
 #ifndef CPD_ADAPT_KW_SOME
 #define CPD_ADAPT_KW_SOME 4  // warps per row at 2 to 7 rows per SM
 #endif
+// ------------------------------------------------------------------ adaptive sampling, few rows
+
+constexpr uint32_t kAdaptRounds = 256;       // rounds decided at once, and
+constexpr uint32_t kAdaptCounts = 64u * 1024u;  // the bytes of their hit counts
+// Counts of one round in bytes, and rounds per group, for a B-bin detector.
+__host__ __device__ constexpr uint32_t adapt_stride(uint32_t B) { return (B + 3u) & ~3u; }
+__host__ __device__ constexpr uint32_t adapt_rounds(uint32_t B)
+{
+    return kAdaptCounts / adapt_stride(B) < kAdaptRounds ? kAdaptCounts / adapt_stride(B) & ~15u : kAdaptRounds;
+}
+constexpr uint32_t kAdaptOdd = 128;  // such hits listed per group of rounds (more: the general exact path)
+struct AdaptBlock {
+    Adapt1Pieces w;
+    uint2 part[32 * kMaxAdaptWarps];   // samples and hits of one bin over one stretch of rounds
+    uint8_t hit[kAdaptRounds], test[kAdaptRounds], df[kAdaptRounds];  // test: 1 a bin failed
+    uint32_t other, ndf, nodd, pad;
+    uint32_t unsure[kAdaptRounds / 32];
+    uint4 odd[kAdaptOdd];  // hits of the float-float trace: round, bin, what they add beside tfast
+};
+// per bin: ox, samples and hits so far, then the counts
+constexpr size_t adapt_block_smem_bytes(uint32_t B)
+{
+    return sizeof(AdaptBlock) + 16u * (size_t)B + (size_t)adapt_rounds(B) * adapt_stride(B);
+}
+
+// One wavelength row under adaptive sampling by one block, for a design with certified pieces
+// (the form for passes with few rows: the plain call). With the pieces a round costs ~70
+// instructions, so the block bins up to kAdaptRounds rounds first (a round per warp at a time)
+// and decides them afterwards: counts[round][bin] holds each round's hits; a thread takes one bin
+// over a stretch of rounds, adds up the stretches before its own, and tests the bin after every
+// round that hit it; the row stops after the first round with a hit and no failed test. Three
+// barriers for 256 rounds instead of three for 16, and no round waits for the one before.
+// The rays of the float-float trace past the stop would leave their differences in ox, so those
+// are listed with their round and added at the end. Returns as adaptive_row1_pieces.
+template <bool kExact>
+__device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t row, unsigned long long *smem)
+{
+    const uint32_t d = find_job<F_ROW>(a.jobs, a.njobs, row);
+    const DesignJob &J = a.jobs[d];
+    const uint32_t k = (uint32_t)(row - J.row_off), B = J.B, R = J.R;
+    const DevDesign &D = a.designs[d];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nthr = blockDim.x, nwarps = nthr >> 5;
+    AdaptBlock &S = *reinterpret_cast<AdaptBlock *>(smem);
+    Adapt1Pieces &w = S.w;
+    unsigned long long *ox = reinterpret_cast<unsigned long long *>(&S + 1);
+    uint2 *base = reinterpret_cast<uint2 *>(ox + B);
+    uint8_t *counts = reinterpret_cast<uint8_t *>(base + B);
+    const uint32_t stride = adapt_stride(B), C = adapt_rounds(B);
+    const LamDF &E = a.lx[row];
+    if (tid < sizeof(LamParams) / 4)
+        reinterpret_cast<uint32_t *>(&w.P)[tid] = reinterpret_cast<const uint32_t *>(a.lp + row)[tid];
+    if (tid < sizeof(FastConst) / 4)
+        reinterpret_cast<uint32_t *>(&w.C)[tid] = reinterpret_cast<const uint32_t *>(&D.fc)[tid];
+    for (uint32_t b = tid; b < B; b += nthr) {
+        base[b] = make_uint2(0u, 0u);
+        ox[b] = 0ull;
+    }
+    if (tid == 0) S.other = S.ndf = S.nodd = 0u;
+    __syncthreads();
+    const uint32_t *rank = a.rank + J.rank_off;
+    const float2 *__restrict__ zt = reinterpret_cast<const float2 *>(a.z32) + J.ray_off;
+    const PieceConst K = piece_const(w.C);
+    const uint32_t lo = w.P.core_lo, hi = w.P.all_exact ? w.P.core_lo : w.P.core_hi;
+    const uint32_t band_lo = w.P.band_lo, band_hi = w.P.band_hi, ks = piece_shift(hi - lo);
+    if (warp == 0u && hi > lo) adapt_pieces(a, w, K, zt, lo, hi, ks, lane);
+    __syncthreads();
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    const uint32_t tfast = piece_tfix(w.P), tfix = coated_tfix(E), tfx = kExact ? tfix : tfast, tq = tfx >> kTqShift;
+    constexpr uint32_t delta = kExact ? 0u : kTqDelta;
+    if (!kExact && (tfix >> kTqShift) - tq + kTqDelta > 2u * kTqDelta) return ROW_OTHER;
+    const SemEqual se = sem_equal(tq, delta);
+    const uint32_t rounds = band_lo >= band_hi ? 0u : (R + kRoundRays - 1u) / kRoundRays;
+    uint32_t stop = rounds;  // rounds taken
+    const auto place = [&](uint32_t r) {
+        const uint32_t j = r * kRoundRays + lane;
+        return r < rounds && j < R ? __ldg(rank + j) : 0xffffffffu;
+    };
+    const auto height = [&](uint32_t s) { return s >= band_lo && s < band_hi ? __ldg(zt + s) : make_float2(0.f, 0.f); };
+    for (uint32_t r0 = 0; r0 < rounds; r0 += C) {
+        const uint32_t nr = min(C, rounds - r0);
+        if (tid < kAdaptRounds / 32) S.unsure[tid] = 0u;
+        // 1. every round's hits per bin
+        uint32_t s_n1 = place(r0 + warp), s_n2 = place(r0 + warp + nwarps);
+        float2 z_n1 = height(s_n1);
+        for (uint32_t q = warp; q < nr; q += nwarps) {
+            uint32_t bin = 0xffffffffu;
+            const uint32_t s = s_n1;
+            const float2 z = z_n1;
+            s_n1 = s_n2;
+            z_n1 = height(s_n1);
+            s_n2 = place(r0 + q + 2u * nwarps);
+            uint32_t *cw = reinterpret_cast<uint32_t *>(counts + q * stride);
+            for (uint32_t i = lane; i < stride / 4u; i += 32u) cw[i] = 0u;
+            __syncwarp();
+            int res = RAY_LOST;
+            const bool core = s >= lo && s < hi;
+            if (core) {
+                uint32_t b = 0u;
+                res = adapt_ray(w, K, B, s, lo, ks, z, b);
+                if (res == RAY_HIT) bin = b;
+            } else if (s >= band_lo && s < band_hi) {
+                res = RAY_FLAG;
+            }
+            bool used_df = false;
+            long long add = 0;
+            if (res == RAY_FLAG && !adapt_left<kExact>(a, D, w, E, core, z, tfast, tfix, bin, used_df, add)) S.other = 1u;
+            if (add) {
+                const uint32_t i = atomicAdd(&S.nodd, 1u);
+                if (i < kAdaptOdd) S.odd[i] = make_uint4(r0 + q, bin, (uint32_t)add, (uint32_t)(add >> 32));
+                else S.other = 1u;
+            }
+            if (kExact) used_df = s >= band_lo && s < band_hi;
+            const uint32_t grp = __match_any_sync(0xffffffffu, bin);
+            const uint32_t ndf = __popc(__ballot_sync(0xffffffffu, used_df));
+            const bool any = __any_sync(0xffffffffu, bin != 0xffffffffu);
+            if (bin != 0xffffffffu && (grp & lt_mask) == 0u) counts[q * stride + bin] = (uint8_t)__popc(grp);
+            if (lane == 0u) {
+                S.hit[q] = any ? 1u : 0u;
+                S.test[q] = 0u;
+                S.df[q] = (uint8_t)ndf;
+            }
+        }
+        __syncthreads();
+        if (S.other) return ROW_OTHER;
+        // 2. the tests, up to nthr bins at a time
+        for (uint32_t b0 = 0; b0 < B; b0 += nthr) {
+            uint32_t width = 1u;
+            while (width < min(B - b0, nthr)) width <<= 1;
+            const uint32_t np = nthr / width, p = tid / width, b = b0 + (tid & (width - 1u));
+            const uint32_t len = (nr + np - 1u) / np, qa = min(p * len, nr), qb = min(qa + len, nr);
+            const bool act = b < B;
+            uint32_t n = 0u, h = 0u;
+            for (uint32_t q = qa; q < qb && act; q++) {
+                const uint32_t c = counts[q * stride + b];
+                if (c) n += min(kRoundRays, R - (r0 + q) * kRoundRays);
+                h += c;
+            }
+            S.part[tid] = make_uint2(n, h);
+            __syncthreads();
+            if (act) {
+                const uint2 v = base[b];
+                n = v.x;
+                h = v.y;
+                for (uint32_t i = 0; i < p; i++) {
+                    const uint2 o = S.part[i * width + (b - b0)];
+                    n += o.x;
+                    h += o.y;
+                }
+                for (uint32_t q = qa; q < qb; q++) {
+                    const uint32_t c = counts[q * stride + b];
+                    if (!c) continue;
+                    n += min(kRoundRays, R - (r0 + q) * kRoundRays);
+                    h += c;
+                    int verdict = sem_quick_equal(n, h, se);
+                    if (verdict < 0) verdict = sem_test(n, h, (uint64_t)h * tq, (uint64_t)h * tq * tq, delta);
+                    if (verdict == SEM_FAIL) S.test[q] = 1u;  // a failed bin settles the round
+                    else if (verdict == SEM_UNSURE) atomicOr(&S.unsure[q >> 5], 1u << (q & 31u));
+                }
+            }
+            __syncthreads();
+        }
+        // 3. the first round that stops the row
+        uint32_t last = nr;
+        for (uint32_t q0 = 0; q0 < nr; q0 += 32u) {
+            const uint32_t q = q0 + lane;
+            const uint32_t m = __ballot_sync(0xffffffffu, q < nr && S.hit[q] && !S.test[q]);
+            if (m) {
+                last = q0 + (uint32_t)__ffs(m) - 1u;
+                break;
+            }
+        }
+        if (last < nr && (S.unsure[last >> 5] >> (last & 31u) & 1u)) return ROW_UNSURE;
+        const uint32_t taken = last < nr ? last + 1u : nr;
+        // the states through it, and the float-float rays
+        for (uint32_t b0 = 0; b0 < B; b0 += nthr) {
+            uint32_t width = 1u;
+            while (width < min(B - b0, nthr)) width <<= 1;
+            const uint32_t np = nthr / width, p = tid / width, b = b0 + (tid & (width - 1u));
+            if (b >= B) continue;
+            uint32_t n = 0u, h = 0u;
+            for (uint32_t q = p; q < taken; q += np) {
+                const uint32_t c = counts[q * stride + b];
+                if (c) n += min(kRoundRays, R - (r0 + q) * kRoundRays);
+                h += c;
+            }
+            if (n) atomicAdd(&base[b].x, n);
+            if (h) atomicAdd(&base[b].y, h);
+        }
+        for (uint32_t i = tid; i < S.nodd; i += nthr) {
+            const uint4 o = S.odd[i];
+            if (o.x < r0 + taken) atomicAdd(ox + o.y, (unsigned long long)o.w << 32 | o.z);
+        }
+        if (warp == 0u) {
+            uint32_t v = 0u;
+            for (uint32_t q = lane; q < taken; q += 32u) v += S.df[q];
+            v = __reduce_add_sync(0xffffffffu, v);
+            if (lane == 0u) S.ndf += v;
+        }
+        __syncthreads();
+        if (last < nr) {
+            stop = r0 + last + 1u;
+            break;
+        }
+        if (tid == 0) S.nodd = 0u;
+        __syncthreads();
+    }
+    const uint32_t count = rounds ? min(R, stop * kRoundRays) : R;
+    uint32_t hits = 0u;
+    unsigned long long *hrow = a.hist + J.hist_off + (uint64_t)k * B;
+    for (uint32_t b = tid; b < B; b += nthr) {
+        const uint32_t h = base[b].y;
+        hits += h;
+        if (h) hrow[b] = rescale_cell((unsigned long long)h * tfx + ox[b], R, count);
+    }
+    hits = __reduce_add_sync(0xffffffffu, hits);
+    const uint32_t sp = (uint32_t)(row % (uint64_t)kSpread);
+    if (lane == 0u && hits) atomicAdd(&a.acc[d].hits[sp], (unsigned long long)hits);
+    if (tid == 0u) {
+        atomicAdd(&a.acc[d].fast[sp], (unsigned long long)count);
+        if (S.ndf) atomicAdd(&a.acc[d].retraced[sp], (unsigned long long)S.ndf);
+    }
+    return ROW_DONE;
+}
+
+__device__ __noinline__ int adaptive_row_redo(const LaunchArgs &a, unsigned long long *smem)
+{
+    __syncthreads();
+    return adaptive_row_pieces<true>(a, blockIdx.x, smem);
+}
+
+// Passes with fewer rows than adaptive1_kernel's: one row per block (rows of designs without
+// pieces are adaptive_kernel's).
+__global__ void __launch_bounds__(32 * kMaxAdaptWarps, 2) adaptive_block_kernel(const LaunchArgs a)
+{
+    extern __shared__ __align__(16) unsigned long long adapt_smem[];
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();  // the setup's LamParams and LamDF
+    if (a.adapt_pieces != 1u && !a.designs[find_job<F_ROW>(a.jobs, a.njobs, blockIdx.x)].fc.pieces) return;
+    int r = adaptive_row_pieces<false>(a, blockIdx.x, adapt_smem);
+    if (r == ROW_UNSURE) r = adaptive_row_redo(a, adapt_smem);
+    if (r == ROW_OTHER && threadIdx.x == 0) queue_row(a, blockIdx.x);
+}
+
 #ifndef CPD_ADAPT_MIN_BLOCKS
 #define CPD_ADAPT_MIN_BLOCKS 2  // 64 registers at kMaxAdaptWarps warps per block
 #endif
@@ -1176,10 +1668,25 @@ __global__ void __launch_bounds__(32 * kMaxAdaptWarps, CPD_ADAPT_MIN_BLOCKS) ada
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();  // the setup's LamParams and LamDF
     const uint32_t kw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    if (a.adapt_pieces && a.designs[find_job<F_ROW>(a.jobs, a.njobs, blockIdx.x)].fc.pieces) return;
     // a row whose stop decision the FP32 transmittances cannot settle is redone here, on
     // the float-float path from its first round, while other blocks go on with theirs
     if (adaptive_row<false>(a, blockIdx.x, adapt_smem, kw, warp, lane))
         adaptive_row<true>(a, blockIdx.x, adapt_smem, kw, warp, lane);
+}
+
+// Out of line: rows of designs without pieces, and the rare ones that the pieces leave (exact:
+// every form of a pass takes those to the exact path, so that a design's result does not depend on
+// what shares its pass).
+__device__ __noinline__ void adaptive_row1_rest(const LaunchArgs &a, unsigned long long *smem, bool exact)
+{
+    if (exact || adaptive_row1<false>(a, blockIdx.x, smem, threadIdx.x))
+        adaptive_row1<true>(a, blockIdx.x, smem, threadIdx.x);
+}
+
+__device__ __noinline__ int adaptive_row1_redo(const LaunchArgs &a, uint32_t d, unsigned long long *smem)
+{
+    return adaptive_row1_pieces<true>(a, blockIdx.x, d, a.jobs[d], smem, threadIdx.x);
 }
 
 #ifndef CPD_ADAPT1_MIN_BLOCKS
@@ -1193,6 +1700,30 @@ __global__ void __launch_bounds__(32, CPD_ADAPT1_MIN_BLOCKS) adaptive1_kernel(co
     cudaGridDependencySynchronize();  // the setup's LamParams and LamDF
     if (adaptive_row1<false>(a, blockIdx.x, adapt_smem, threadIdx.x))
         adaptive_row1<true>(a, blockIdx.x, adapt_smem, threadIdx.x);
+}
+
+// The same for passes of designs with certified pieces, or some of them (a kernel of its own:
+// with the general form out of line, rows without pieces take 9% longer here).
+__global__ void __launch_bounds__(32, CPD_ADAPT1_MIN_BLOCKS) adaptive1_pieces_kernel(const LaunchArgs a)
+{
+    extern __shared__ __align__(16) unsigned long long adapt_smem[];
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();  // the setup's LamParams and LamDF
+    const uint32_t d = find_job<F_ROW>(a.jobs, a.njobs, blockIdx.x);
+    const bool pieces = a.designs[d].fc.pieces;
+    if (pieces) {
+        int r = adaptive_row1_pieces<false>(a, blockIdx.x, d, a.jobs[d], adapt_smem, threadIdx.x);
+        __syncwarp();
+        if (r == ROW_UNSURE) r = adaptive_row1_redo(a, d, adapt_smem);
+        if (r == ROW_DONE) return;
+    }
+    __syncwarp();
+    if (a.adapt_pieces == 1u) {
+        // a pass of such designs alone has no room for the general form's states
+        if (threadIdx.x == 0) queue_row(a, blockIdx.x);
+        return;
+    }
+    adaptive_row1_rest(a, adapt_smem, pieces);
 }
 
 // The queued rows: the float-float path from the first round on, one row per block of
@@ -2718,12 +3249,15 @@ static uint32_t rows_blocks_per_sm(uint32_t warps, uint32_t B)
 RowsPlan plan_rows(uint64_t rows, uint32_t R, uint32_t max_B, int num_sms)
 {
     RowsPlan p;
-    const uint64_t resident = (uint64_t)num_sms * rows_blocks_per_sm(kRowsWarps, max_B) * kRowsWarps;
-    // several warps per row while all of them are resident at once and each half-warp keeps
-    // 32 rays or more
+    // several warps per row while all teams are resident at once (a second wave would double the
+    // time) and each half-warp keeps 32 rays or more
     p.team = 1u;
-    while (p.team < kRowsMaxTeam && rows * p.team * 2u <= resident && R >= 128u * p.team) p.team *= 2u;
+    for (uint32_t T = 2u; T <= kRowsMaxTeam && R >= 64u * T; T *= 2u) {
+        const uint32_t warps = std::max(kRowsWarps, T);
+        if (rows <= (uint64_t)num_sms * rows_blocks_per_sm(warps, max_B) * (warps / T)) p.team = T;
+    }
     // two rows or more per warp once every warp has one
+    const uint64_t resident = (uint64_t)num_sms * rows_blocks_per_sm(kRowsWarps, max_B) * kRowsWarps;
     p.group = rows <= resident ? 1u : (uint32_t)std::min<uint64_t>(kRowsGroup, std::max<uint64_t>(2u, rows / resident));
     return p;
 }
@@ -2768,9 +3302,22 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
             // decide that many rounds at once
             const uint64_t per_sm = a.total_rows / (uint64_t)num_sms;
             const uint32_t kw = per_sm >= 8 ? CPD_ADAPT_KW_MANY : per_sm >= 2 ? CPD_ADAPT_KW_SOME : kMaxAdaptWarps;
-            launch_k(kw == 1u ? adaptive1_kernel : adaptive_kernel, (unsigned)a.total_rows, 32 * kw,
-                     kw == 1u ? adapt1_smem_bytes(maxB) : adapt_smem_bytes(kw, maxB), stream, pdl, a);
-            launches++;
+            if (kw == 1u) {
+                const size_t smem = adapt1p_smem_bytes(maxB);
+                launch_k(a.adapt_pieces ? adaptive1_pieces_kernel : adaptive1_kernel, (unsigned)a.total_rows, 32,
+                         a.adapt_pieces == 1u ? smem : std::max(smem, adapt1_smem_bytes(maxB)), stream, pdl, a);
+                launches++;
+            } else {
+                if (a.adapt_pieces) {
+                    launch_k(adaptive_block_kernel, (unsigned)a.total_rows, 32 * kMaxAdaptWarps,
+                             adapt_block_smem_bytes(maxB), stream, pdl, a);
+                    launches++;
+                }
+                if (a.adapt_pieces != 1u) {
+                    launch_k(adaptive_kernel, (unsigned)a.total_rows, 32 * kw, adapt_smem_bytes(kw, maxB), stream, pdl, a);
+                    launches++;
+                }
+            }
         }
         if (ev) cudaEventRecord(ev[2], stream);
         const uint32_t kwe = a.total_rows / (uint64_t)num_sms >= 8 ? 1u : kMaxAdaptWarps;
@@ -2849,10 +3396,17 @@ cudaError_t configure_kernels()
     const int bytes = (int)adapt_smem_bytes(kMaxAdaptWarps, CPD_MAX_BINS);
     cudaError_t e = cudaFuncSetAttribute(adaptive_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(adaptive1_pieces_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)std::max(adapt1_smem_bytes(CPD_MAX_BINS), adapt1p_smem_bytes(CPD_MAX_BINS)));
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute(adaptive1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)adapt1_smem_bytes(CPD_MAX_BINS));
+                                 (int)std::max(adapt1_smem_bytes(CPD_MAX_BINS), adapt1p_smem_bytes(CPD_MAX_BINS)));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(adaptive_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    size_t block_bytes = 0;
+    for (uint32_t B = 1; B <= CPD_MAX_BINS; B++) block_bytes = std::max(block_bytes, adapt_block_smem_bytes(B));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(adaptive_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_bytes);
     const int rows_bytes = (int)std::max(rows_smem_bytes(kRowsWarps, kRowsWarps, CPD_MAX_BINS),
                                          rows_smem_bytes(kRowsMaxTeam, 1u, CPD_MAX_BINS));
     if (e == cudaSuccess)

@@ -549,6 +549,28 @@ CPD_HD int sem_quick(uint32_t N, uint32_t h, uint64_t q1, uint64_t q2, uint32_t 
     return -1;
 }
 
+// sem_quick when every hit has t_q = q (within delta of its exact value): q1 = h q, q2 = h q^2, so
+// lhs = 40000 q^2 h (N - h) and err = 40000 h (N d (2^21 + d) + d h (2 q + d)). The constants:
+struct SemEqual {
+    float c;       // 40000 q^2
+    float e1, e2;  // 40000 d (2^21 + d), 40000 d (2 q + d)
+};
+CPD_HD SemEqual sem_equal(uint32_t q, uint32_t delta)
+{
+    const float f = (float)q, d = (float)delta;
+    return SemEqual{40000.f * f * f, 40000.f * (d * (0x1p21f + d)), 40000.f * (d * (2.f * f + d))};
+}
+// Every product and sum rounds by at most 2^-24 relative and none cancels (N and h are exact), so
+// each side is within 8 2^-24 of its value: margins of 2^-18 settle the test, else -1.
+CPD_HD int sem_quick_equal(uint32_t N, uint32_t h, const SemEqual &s)
+{
+    const float n = f32_small(N), f = f32_small(h);
+    const float L = s.c * f * (n - f), E = f * (n * s.e1 + f * s.e2), Y = n * n * (n - 1.f) * 0x1p40f;
+    if ((L + E) * (1.f + 0x1p-18f) < Y * (1.f - 0x1p-18f)) return SEM_PASS;
+    if (L * (1.f - 0x1p-18f) >= (Y + E) * (1.f + 0x1p-18f)) return SEM_FAIL;
+    return -1;
+}
+
 // A cell's sum of t over `count` rays rescaled to the pass's common divisor R:
 // round(s1 R / count), so that p = cell 2^-31 / R everywhere downstream.
 CPD_HD uint64_t rescale_cell(uint64_t s1, uint32_t R, uint32_t count)

@@ -319,8 +319,26 @@ CPD_HD EdgeRays edge_rays(uint32_t p0, uint32_t p1, float sg, float e, const At 
     return r;
 }
 
-// Rays per piece for a range of n rays: at most 31 pieces (32 ends), in steps of 32 rays.
-CPD_HD uint32_t piece_len(uint32_t n) { return 32u * ((n + 991u) / 992u); }
+// log2 of the rays per piece that cut n rays into at most 31 pieces (32 ends).
+CPD_HD uint32_t piece_shift(uint32_t n)
+{
+    uint32_t k = 0;
+    while ((31u << k) < n) k++;
+    return k;
+}
+
+// A piece as a quadratic and an error that make piece_ray give every ray the piece's outcome: a
+// piece in one bin or lost whole is a constant in the bin's sensitive part or off the detector, a
+// piece without a bound has an error beyond every bin.
+CPD_HD Piece piece_uniform(const PieceConst &K, Piece q)
+{
+    if (q.cls == PIECE_MIXED) return q;
+    q.v1 = q.v2 = q.e = 0.f;
+    q.v0 = q.cls == PIECE_BIN ? (float)q.bin + 0.5f * ((K.fs < 0.5f ? K.fs : 0.5f) - 0.5f)
+                              : K.vmid + 2.f * K.vhalf + 1.f;
+    if (q.cls == PIECE_RAYS) q.e = 1e30f;
+    return q;
+}
 
 // 2^31 t of every hit of a certified piece: fast_ray's coated transmittance.
 CPD_HD uint32_t piece_tfix(const LamParams &P) { return t_fixed(mulr(addr(P.ts, P.tp), 0.495f)); }

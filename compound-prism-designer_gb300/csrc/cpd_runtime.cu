@@ -643,6 +643,15 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     a.perm = S.perm.as<uint32_t>();
     a.rank = adaptive ? reinterpret_cast<const uint32_t *>(din + o_rank) : nullptr;
     a.adaptive = adaptive ? (all_exact ? 2u : 1u) : 0u;
+    if (adaptive && !all_exact) {
+        // (a device build decides in its record)
+        uint32_t with = 0, maybe = 0;
+        for (const PassDesign &p : ds) {
+            with += p.dev && p.dev->fc.pieces;
+            maybe += p.params && p.params->ar_coated;
+        }
+        a.adapt_pieces = with == n ? 1u : with || maybe ? 2u : 0u;
+    }
     a.max_B = max_B;
     a.lp = S.lp.as<LamParams>();
     a.lx = S.lx.as<LamDF>();

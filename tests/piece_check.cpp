@@ -51,7 +51,7 @@ int main(int argc, char **argv)
         LamDF E;
         lambda_setup_df(D, lu[k], z32.data(), (uint32_t)z64.size(), P, kYGuardRel, &E);
         if (P.all_exact || P.core_hi <= P.core_lo) continue;
-        const uint32_t lo = P.core_lo, hi = P.core_hi, n = hi - lo, L = piece_len(n);
+        const uint32_t lo = P.core_lo, hi = P.core_hi, n = hi - lo, L = (n + 14u) / 15u;
         const uint32_t T = piece_tfix(P);
         rays += n;
         for (uint32_t j0 = lo; j0 < hi; j0 += L) {
@@ -61,6 +61,17 @@ int main(int argc, char **argv)
             Piece q = piece_fit(D.fc, K, P, a, b);
             if (!D.fc.pieces) q.cls = PIECE_RAYS;
             pieces++;
+            // the same piece as one quadratic for piece_ray (adaptive sampling)
+            {
+                const Piece u = piece_uniform(K, q);
+                for (uint32_t j = j0; j < j1; j++) {
+                    const float dz = (P.zref_hi - z32[2 * j]) + (P.zref_lo - z32[2 * j + 1]);
+                    uint32_t bin = 0;
+                    const int r = piece_ray(K, D.B, u.dz0, u.v0, u.v1, u.v2, u.e, dz, bin);
+                    const int want = q.cls == PIECE_BIN ? RAY_HIT : q.cls == PIECE_LOST ? RAY_LOST : RAY_FLAG;
+                    if (q.cls != PIECE_MIXED && (r != want || (r == RAY_HIT && bin != q.bin))) wrong++;
+                }
+            }
             // the outcome of every ray of the piece: its bin, -1 lost, -2 left to fast_ray
             std::vector<int> out(j1 - j0, q.cls == PIECE_BIN ? (int)q.bin : q.cls == PIECE_LOST ? -1 : -2);
             if (q.cls == PIECE_RAYS) whole += j1 - j0;
