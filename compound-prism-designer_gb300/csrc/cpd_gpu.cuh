@@ -338,6 +338,26 @@ void launch_trace_pairs(const DevDesign *d, const double *lam_u, const double *z
 void launch_tp_adaptive(const DevDesign *d, uint32_t B, const double *lambdas, uint32_t n, const double *z64,
                         uint32_t max_m, double *out, uint32_t *rays_out, cudaStream_t stream);
 
+// The same for a design with certified pieces, up to kTpMaxRays rays.
+constexpr uint32_t kTpMaxRays = 65536;  // rays of the sorted table and the tables of counts
+struct TpArgs {
+    const DevDesign *d;       // wavelength bounds (0, 1): a point is its wavelength
+    const double *lambdas;
+    uint32_t n, max_m;
+    const double *z64;        // in ray order
+    const float2 *z32;        // sorted
+    const uint32_t *rank;     // ray -> sorted position
+    const double2 *cnt;       // by count c: 1/c and c
+    LamParams *lp;
+    double *t64;              // per wavelength
+    double *out;
+    uint32_t *rays_out;
+    Guards guards;
+    uint32_t Rz;
+};
+
+void launch_tp_pieces(const TpArgs &a, uint32_t B, cudaStream_t stream);
+
 // FP32 FMA throughput probe.
 void launch_fma_peak(float *out, uint32_t iters, int blocks, int threads, cudaStream_t stream);
 // SFU (MUFU) throughput probe: 8 x 16 reciprocal-square-root estimates per thread and iteration.

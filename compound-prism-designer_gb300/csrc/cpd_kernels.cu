@@ -1193,7 +1193,7 @@ __device__ __forceinline__ void queue_row(const LaunchArgs &a, uint64_t row)
 }
 
 // The records of a row's pieces, by one warp.
-__device__ __forceinline__ void adapt_pieces(const LaunchArgs &a, Adapt1Pieces &w, const PieceConst &K,
+__device__ __forceinline__ void adapt_pieces(const Guards &g, Adapt1Pieces &w, const PieceConst &K,
                                              const float2 *__restrict__ zt, uint32_t lo, uint32_t hi, uint32_t ks,
                                              uint32_t lane)
 {
@@ -1204,14 +1204,14 @@ __device__ __forceinline__ void adapt_pieces(const LaunchArgs &a, Adapt1Pieces &
     uint32_t j0 = lo + (lane << ks), cut = 0u;
     for (int level = 0; level < 2; level++) {
         if (level) {
-            const uint32_t g = lane / 9u, t = lane - 9u * g;
+            const uint32_t pc = lane / 9u, t = lane - 9u * pc;
             uint32_t m = cut;
-            for (uint32_t i = 0; i < g; i++) m &= m - 1u;
-            const uint32_t p = g < 3u && m ? (uint32_t)__ffs(m) - 1u : 0u;
+            for (uint32_t i = 0; i < pc; i++) m &= m - 1u;
+            const uint32_t p = pc < 3u && m ? (uint32_t)__ffs(m) - 1u : 0u;
             j0 = min(lo + (p << ks) + (t << (ks - 3u)), min(lo + ((p + 1u) << ks), hi - 1u));
         }
         const float2 z = __ldg(zt + min(j0, hi - 1u));
-        const PieceEnd e = piece_end(C, fast_limits(C, a.guards), K, P, a.guards, z.x, z.y);
+        const PieceEnd e = piece_end(C, fast_limits(C, g), K, P, g, z.x, z.y);
         PieceEnd o = e;
         o.dz = __shfl_down_sync(0xffffffffu, e.dz, 1);
         o.v = __shfl_down_sync(0xffffffffu, e.v, 1);
@@ -1238,10 +1238,10 @@ __device__ __forceinline__ void adapt_pieces(const LaunchArgs &a, Adapt1Pieces &
                 w.rec_b[lane].y = kCutPiece;
             }
         } else {
-            const uint32_t g = lane / 9u, t = lane - 9u * g;
-            if (g < 3u && t < 8u) {
-                w.rec_a[32u + 8u * g + t] = make_float4(z.x, z.y, q.v0, q.v1);
-                w.rec_b[32u + 8u * g + t] = make_float2(q.v2, q.e);
+            const uint32_t pc = lane / 9u, t = lane - 9u * pc;
+            if (pc < 3u && t < 8u) {
+                w.rec_a[32u + 8u * pc + t] = make_float4(z.x, z.y, q.v0, q.v1);
+                w.rec_b[32u + 8u * pc + t] = make_float2(q.v2, q.e);
             }
         }
     }
@@ -1318,7 +1318,7 @@ __device__ __forceinline__ int adaptive_row1_pieces(const LaunchArgs &a, uint64_
     const PieceConst K = piece_const(C);
     const uint32_t lo = P.core_lo, hi = P.all_exact ? P.core_lo : P.core_hi, band_lo = P.band_lo, band_hi = P.band_hi;
     const uint32_t ks = piece_shift(hi - lo);
-    if (hi > lo) adapt_pieces(a, w, K, zt, lo, hi, ks, lane);
+    if (hi > lo) adapt_pieces(a.guards, w, K, zt, lo, hi, ks, lane);
     __syncwarp();
     const uint32_t lt_mask = (1u << lane) - 1u;
     const uint32_t tfast = piece_tfix(P), tfix = coated_tfix(E), tfx = kExact ? tfix : tfast, tq = tfx >> kTqShift;
@@ -1478,7 +1478,7 @@ __device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t
     const PieceConst K = piece_const(w.C);
     const uint32_t lo = w.P.core_lo, hi = w.P.all_exact ? w.P.core_lo : w.P.core_hi;
     const uint32_t band_lo = w.P.band_lo, band_hi = w.P.band_hi, ks = piece_shift(hi - lo);
-    if (warp == 0u && hi > lo) adapt_pieces(a, w, K, zt, lo, hi, ks, lane);
+    if (warp == 0u && hi > lo) adapt_pieces(a.guards, w, K, zt, lo, hi, ks, lane);
     __syncthreads();
     const uint32_t lt_mask = (1u << lane) - 1u;
     const uint32_t tfast = piece_tfix(w.P), tfix = coated_tfix(E), tfx = kExact ? tfix : tfast, tq = tfx >> kTqShift;
@@ -2795,6 +2795,249 @@ __global__ void __launch_bounds__(kTpRays) tp_adaptive_kernel(const DevDesign *_
     if (tid == 0 && rays_out) rays_out[blockIdx.x] = count;
 }
 
+// The same estimator for a design with certified pieces (cpd_piece.h), bit for bit. What bounds
+// the kernel above is FP64: a warp instruction takes its scheduler ~64 cycles, a trace of 256 rays
+// ~28k cycles, and a hit's Welford update three divisions. Here
+//  * the bins come from the wavelength's pieces, fast_ray and, for the few rays in its guard
+//    bands, the exact f64 trace; every ray's transmittance is the same f64 value, formed once per
+//    wavelength by the trace's own operations (tp_setup_kernel);
+//  * a chunk's hits are bits of a mask per bin, so one thread per bin replays its hits in ray order
+//    with all bins of 32 packed in one warp, and runs ahead of the other bins up to the earliest
+//    stop known;
+//  * the divisors are ray counts, whose reciprocals are a table: a division is three FP64
+//    instructions (x::div_by);
+//  * of an update only the mean is replayed in f64 (9 instructions; the result is its bits). The
+//    squared deviations are read by the SEM test alone and have a closed form for hits of one t:
+//    after hit k + 1 at ray n, with c the count before it, they grow by
+//    (k t / n)^2 c (n - c) / n + t^2 (n - k)^2 / (n (n + 1)). In FP32, summed exactly, that is
+//    within 2e-6 of the f64 recurrence; a test within kTpMargin leaves the wavelength to a replay
+//    in full (21 instructions) from the start.
+// A bin that ran past the stop is replayed from the chunk's start.
+constexpr uint32_t kTpList = 1024;
+
+// Per wavelength, by two warps of a block: the setup in float-float, and the transmittance of its
+// hits in the f64 trace's operations (the flat faces and a coated exit face).
+__global__ void __launch_bounds__(64) tp_setup_kernel(const TpArgs a)
+{
+    cudaTriggerProgrammaticLaunchCompletion();
+    const uint32_t i = blockIdx.x * 32u + (threadIdx.x & 31u);
+    if (i >= a.n) return;
+    const DevDesign &D = *a.d;
+    const double lambda = a.lambdas[i];
+    if (threadIdx.x < 32u) {
+        LamParams P;
+        LamDF E;
+        lambda_setup_df(D, lambda, reinterpret_cast<const float *>(a.z32), a.Rz, P, kYGuardRel, &E);
+        a.lp[i] = P;
+    } else {
+        x::Ray r{0.0, 0.0, 1.0, 0.0, 1.0, 1.0};
+        double n1 = 1.0;
+        bool ok = true;
+        for (int k = 0; k < D.G && ok; k++) {
+            const double n2 = x::calc_n(D.glass[k], lambda);
+            ok = x::refract(r, D.pnx[k], D.pny[k], n1, n2, D.ar != 0);
+            n1 = n2;
+        }
+        a.t64[i] = x::mul(x::add(x::mul(r.ts, 0.99), x::mul(r.tp, 0.99)), 0.5);
+    }
+}
+
+constexpr float kTpMargin = 1e-5f;
+// One bin: its mean, squared deviations (fast: an FP32 sum and its error; full: f64), the count
+// and the hits.
+struct TpBin {
+    double m;
+    union {
+        double m2;
+        float2 f2;
+    };
+    uint32_t c, k;
+};
+
+__host__ __device__ constexpr uint32_t tp_chunk(uint32_t B) { return B <= 256u ? 1024u : 256u; }
+constexpr size_t tp_pieces_smem_bytes(uint32_t B)
+{
+    // per bin: the state, its copy at the chunk's start, the mask
+    return sizeof(Adapt1Pieces) + (size_t)B * (2u * sizeof(TpBin) + tp_chunk(B) / 8u) + 8u * kTpList;
+}
+
+__global__ void __launch_bounds__(256) tp_pieces_kernel(const TpArgs a)
+{
+    extern __shared__ __align__(16) unsigned char tp_smem[];
+    __shared__ uint32_t s_stop, s_n1, s_n2, s_open;
+    Adapt1Pieces &w = *reinterpret_cast<Adapt1Pieces *>(tp_smem);
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, nthr = blockDim.x;
+    const DevDesign &D = *a.d;
+    const uint32_t B = D.B, C = tp_chunk(B), words = C / 32u;
+    TpBin *st = reinterpret_cast<TpBin *>(&w + 1), *st0 = st + B;
+    uint32_t *list1 = reinterpret_cast<uint32_t *>(st0 + B), *list2 = list1 + kTpList;
+    uint32_t *mask = list2 + kTpList;  // [bin][word]
+    TpBin zero;
+    zero.m = zero.m2 = 0.0;
+    zero.c = zero.k = 0u;
+    for (uint32_t b = tid; b < B; b += nthr) st[b] = zero;
+    if (tid == 0) s_open = 0u;
+    if (tid < sizeof(FastConst) / 4)
+        reinterpret_cast<uint32_t *>(&w.C)[tid] = reinterpret_cast<const uint32_t *>(&D.fc)[tid];
+    const uint32_t il = blockIdx.x;
+    const double lambda = a.lambdas[il];
+    cudaGridDependencySynchronize();  // tp_setup_kernel
+    if (tid < sizeof(LamParams) / 4)
+        reinterpret_cast<uint32_t *>(&w.P)[tid] = reinterpret_cast<const uint32_t *>(a.lp + il)[tid];
+    __syncthreads();
+    const PieceConst K = piece_const(w.C);
+    const uint32_t lo = w.P.core_lo, hi = w.P.all_exact ? w.P.core_lo : w.P.core_hi;
+    const uint32_t band_lo = w.P.band_lo, band_hi = w.P.band_hi, ks = piece_shift(hi - lo);
+    const uint32_t tfast = piece_tfix(w.P);
+    const double t64 = a.t64[il];
+    if (tid < 32u && hi > lo) adapt_pieces(a.guards, w, K, a.z32, lo, hi, ks, lane);
+    uint32_t count = a.max_m;
+    bool full = false;
+    const float tf = (float)t64, tf2 = tf * tf;
+    // no ray clears the flat faces: no hit
+    for (uint32_t j0 = band_lo >= band_hi ? a.max_m : 0u; j0 < a.max_m; j0 += C) {
+        const uint32_t nj = min(C, a.max_m - j0);
+        for (uint32_t i = tid; i < B * words; i += nthr) mask[i] = 0u;
+        for (uint32_t b = tid; b < B; b += nthr) st0[b] = st[b];
+        if (tid == 0) {
+            s_stop = ~0u;
+            s_n1 = s_n2 = 0u;
+        }
+        __syncthreads();
+        // the rays' bins: their pieces, then fast_ray for what those leave
+        for (uint32_t i = tid; i < nj; i += nthr) {
+            const uint32_t s = __ldg(a.rank + j0 + i);
+            if (s < band_lo || s >= band_hi) continue;
+            uint32_t bin = 0u;
+            int r = RAY_FLAG;
+            if (s >= lo && s < hi) r = adapt_ray(w, K, B, s, lo, ks, __ldg(a.z32 + s), bin);
+            if (r == RAY_HIT) atomicOr(mask + bin * words + (i >> 5), 1u << (i & 31u));
+            else if (r == RAY_FLAG) list1[atomicAdd(&s_n1, 1u)] = i;
+        }
+        __syncthreads();
+        for (uint32_t q = tid; q < s_n1; q += nthr) {
+            const uint32_t i = list1[q], s = __ldg(a.rank + j0 + i);
+            const float2 z = __ldg(a.z32 + s);
+            uint32_t bin = 0u;
+            float t = 0.f;
+            int r = RAY_FLAG;
+            if (s >= lo && s < hi) r = fast_ray(w.C, w.P, a.guards, z.x, z.y, bin, t);
+            if (r == RAY_HIT && t_fixed(t) != tfast) r = RAY_FLAG;  // not the wavelength's transmittance
+            if (r == RAY_HIT) atomicOr(mask + bin * words + (i >> 5), 1u << (i & 31u));
+            else if (r == RAY_FLAG) list2[atomicAdd(&s_n2, 1u)] = i;
+        }
+        __syncthreads();
+        // what fast_ray leaves, in exact f64; a hit with another transmittance would break the
+        // replay's one value, and the wavelength is then left to tp_adaptive_kernel
+        bool other = false;
+        for (uint32_t q = tid; q < s_n2; q += nthr) {
+            const uint32_t i = list2[q];
+            uint32_t bin = 0u;
+            double t = 0.0;
+            if (x::trace(D, lambda, x::beam_y(D, a.z64[j0 + i]), bin, t) == 0) {
+                if (t == t64) atomicOr(mask + bin * words + (i >> 5), 1u << (i & 31u));
+                else other = true;
+            }
+        }
+        if (__syncthreads_or(other)) {
+            if (tid == 0) a.rays_out[il] = 0u;  // no wavelength takes 0 rays: the mark
+            return;
+        }
+        // the bins' updates in ray order, up to the earliest stop
+        const auto replay = [&](uint32_t b, bool last) {
+            TpBin v = last ? st0[b] : st[b];
+            // the hits in ray order; the next one's counts are loaded before the current update
+            // (their latency is as long as its chain)
+            uint32_t q = 0, m = mask[b * words];
+            const auto next = [&]() {
+                while (!m && ++q < words) m = mask[b * words + q];
+                if (!m) return ~0u;
+                const uint32_t i = 32u * q + (uint32_t)__ffs(m) - 1u;
+                m &= m - 1u;
+                return i;
+            };
+            uint32_t ni = next();
+            double2 tn = make_double2(0.0, 0.0), tc = tn;
+            if (ni != ~0u) {
+                tn = __ldg(a.cnt + j0 + ni + 1u);
+                tc = __ldg(a.cnt + j0 + ni + 2u);
+            }
+            double c = (double)v.c;
+            while (ni != ~0u && ni <= *(volatile uint32_t *)&s_stop) {
+                const uint32_t i = ni, n = j0 + i + 1u;  // the ray's number
+                const double rn = tn.x, nd = tn.y, rc = tc.x, cd = tc.y;
+                ni = next();
+                if (ni != ~0u) {
+                    tn = __ldg(a.cnt + j0 + ni + 1u);
+                    tc = __ldg(a.cnt + j0 + ni + 2u);
+                }
+                int pass;
+                if (full) {
+                    if (v.c < n) {  // Welford::skip
+                        v.m = x::div_by(x::mul(c, v.m), nd, rn);
+                        v.m2 = x::add(v.m2, x::div_by(x::mul(x::mul(x::sqr(v.m), c), x::sub(nd, c)), nd, rn));
+                    }
+                    // Welford::next_sample: the count becomes the ray's number plus one
+                    const double dl = x::sub(t64, v.m);
+                    v.m = x::add(v.m, x::div_by(dl, cd, rc));
+                    v.m2 = x::add(v.m2, x::mul(dl, x::sub(t64, v.m)));
+                    pass = v.m2 < x::mul(x::mul(5e-3, 5e-3), x::mul(cd, nd));  // c (c - 1), c = n + 1
+                } else {
+                    if (v.c < n) v.m = x::div_by(x::mul(c, v.m), nd, rn);
+                    v.m = x::add(v.m, x::div_by(x::sub(t64, v.m), cd, rc));
+                    const float nf = (float)n, ir = __fdividef(1.f, nf), kt = (float)v.k * tf * ir, cf = (float)v.c;
+                    const float sk = kt * kt * cf * (float)(n - v.c) * ir;
+                    const float rest = (float)(n - v.k);
+                    const float nx = tf2 * (rest * ir) * __fdividef(rest, nf + 1.f);
+                    const ff::F2 e = ff::two_sum(v.f2.x, sk), f = ff::two_sum(e.hi, nx);
+                    v.f2.x = f.hi;
+                    v.f2.y += e.lo + f.lo;
+                    const float m2 = v.f2.x + v.f2.y, lim = 2.5e-5f * ((nf + 1.f) * nf);
+                    pass = m2 < lim * (1.f - kTpMargin) ? 1 : m2 > lim * (1.f + kTpMargin) ? 0 : 2;
+                }
+                c = cd;
+                v.c = n + 1u;
+                v.k++;
+                if (!last && pass) {
+                    if (pass == 2) s_open = 1u;
+                    atomicMin(&s_stop, i);
+                    break;
+                }
+            }
+            st[b] = v;
+        };
+        for (uint32_t b = tid; b < B; b += nthr) replay(b, false);
+        __syncthreads();
+        const uint32_t stop = s_stop;
+        if (s_open) {
+            // a test too close to call: the wavelength again from its first ray, in full
+            __syncthreads();
+            for (uint32_t b = tid; b < B; b += nthr) st[b] = zero;
+            if (tid == 0) s_open = 0u;
+            full = true;
+            j0 = 0u - C;
+            __syncthreads();
+            continue;
+        }
+        if (stop != ~0u) {
+            // bins that took a ray past the stop: again from the chunk's start
+            for (uint32_t b = tid; b < B; b += nthr)
+                if (st[b].c > j0 + stop + 2u) replay(b, true);
+            __syncthreads();
+            count = j0 + stop + 1u;
+            break;
+        }
+        __syncthreads();
+    }
+    // every bin padded to the final ray count (the reference's closing skip)
+    const double2 fin = a.cnt[count];
+    for (uint32_t b = tid; b < B; b += nthr) {
+        const TpBin v = st[b];
+        a.out[(uint64_t)il * B + b] = v.c < count ? x::div_by(x::mul((double)v.c, v.m), fin.y, fin.x) : v.m;
+    }
+    if (tid == 0) a.rays_out[il] = count;
+}
+
 __global__ void fma_peak_kernel(float *out, uint32_t iters)
 {
     float a0 = threadIdx.x * 1e-7f, a1 = a0 + 1e-7f, a2 = a0 + 2e-7f, a3 = a0 + 3e-7f;
@@ -3212,8 +3455,8 @@ __global__ void __launch_bounds__(kLoopThreads, CPD_LOOP_MIN_BLOCKS) loop_kernel
 // A launch that, with `pdl`, may start before the previous kernel on the stream has
 // finished (programmatic dependent launch): the kernel waits for its predecessor's
 // results in cudaGridDependencySynchronize.
-void launch_k(void (*k)(const LaunchArgs), dim3 grid, unsigned block, size_t smem, cudaStream_t st, bool pdl,
-              const LaunchArgs &a)
+template <class Args>
+void launch_k(void (*k)(const Args), dim3 grid, unsigned block, size_t smem, cudaStream_t st, bool pdl, const Args &a)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -3407,6 +3650,10 @@ cudaError_t configure_kernels()
     for (uint32_t B = 1; B <= CPD_MAX_BINS; B++) block_bytes = std::max(block_bytes, adapt_block_smem_bytes(B));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(adaptive_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_bytes);
+    size_t tp_bytes = 0;
+    for (uint32_t B = 1; B <= CPD_MAX_BINS; B++) tp_bytes = std::max(tp_bytes, tp_pieces_smem_bytes(B));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(tp_pieces_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_bytes);
     const int rows_bytes = (int)std::max(rows_smem_bytes(kRowsWarps, kRowsWarps, CPD_MAX_BINS),
                                          rows_smem_bytes(kRowsMaxTeam, 1u, CPD_MAX_BINS));
     if (e == cudaSuccess)
@@ -3452,6 +3699,13 @@ void launch_tp_adaptive(const DevDesign *d, uint32_t B, const double *lambdas, u
 {
     if (!n) return;
     tp_adaptive_kernel<<<n, kTpRays, 3 * sizeof(double) * B, stream>>>(d, lambdas, z64, max_m, out, rays_out);
+}
+
+void launch_tp_pieces(const TpArgs &a, uint32_t B, cudaStream_t stream)
+{
+    if (!a.n) return;
+    tp_setup_kernel<<<(a.n + 31) / 32, 64, 0, stream>>>(a);
+    launch_k(tp_pieces_kernel, a.n, 256, tp_pieces_smem_bytes(B), stream, true, a);
 }
 
 void launch_mufu_peak(float *out, uint32_t iters, int blocks, int threads, cudaStream_t stream)

@@ -206,8 +206,8 @@ struct cpd_context {
     DevBuf bld_params, bld_out, bld_status;  // cpd_design_build_device
     // cpd_transmission_probability: the design, the wavelengths, the ray table of the
     // reference's ray points (kept while max_m stays the same), the results
-    DevBuf tp_design, tp_lam, tp_z, tp_out, tp_rays;
-    uint32_t tp_m = 0;
+    DevBuf tp_design, tp_lam, tp_z, tp_out, tp_rays, tp_tab, tp_lp, tp_t64;
+    uint32_t tp_m = 0, tp_tab_m = 0, tp_rz = 0;
     uint32_t ray_tile = 32;
     uint32_t warps_per_cta = 8;
     bool profiling = false;
@@ -1230,7 +1230,8 @@ void cpd_context_destroy(cpd_context *ctx)
     ctx->main.destroy();
     for (auto &o : ctx->orders)
         if (o.second.dev) cudaFree(o.second.dev);
-    for (DevBuf *b : {&ctx->tp_design, &ctx->tp_lam, &ctx->tp_z, &ctx->tp_out, &ctx->tp_rays})
+    for (DevBuf *b : {&ctx->tp_design, &ctx->tp_lam, &ctx->tp_z, &ctx->tp_out, &ctx->tp_rays, &ctx->tp_tab, &ctx->tp_lp,
+                      &ctx->tp_t64})
         b->release();
     for (DevBuf *b : {&ctx->bld_params, &ctx->bld_out, &ctx->bld_status, &ctx->pair_design, &ctx->pair_lam,
                       &ctx->pair_z, &ctx->pair_bins, &ctx->pair_ts,
@@ -1513,37 +1514,126 @@ int cpd_transmission_probability_ex(cpd_context *ctx, const cpd_design *d, const
     cudaStream_t s = S.stream;
     DevDesign D;
     design_to_dev(*d, D);
-    if (ctx->tp_m != max_m) {
+    const bool pieces = D.fc.pieces && max_m <= kTpMaxRays;
+    if (ctx->tp_m != max_m || (pieces && ctx->tp_tab_m != max_m)) {
         std::vector<double> z(max_m);
         ref_points(max_m, z.data());
+        std::vector<uint32_t> order;
+        if (pieces) {
+            // the rays by point (spread evenly: a bucket each, then the few that share one)
+            order.resize(max_m);
+            std::vector<uint32_t> at(max_m + 1u, 0u);
+            const auto bucket = [&](double u) { return std::min(max_m - 1u, (uint32_t)(u * max_m)); };
+            for (uint32_t j = 0; j < max_m; j++) at[bucket(z[j]) + 1u]++;
+            for (uint32_t b = 0; b < max_m; b++) at[b + 1u] += at[b];
+            std::vector<uint32_t> next(at.begin(), at.end() - 1);
+            for (uint32_t j = 0; j < max_m; j++) order[next[bucket(z[j])]++] = j;
+            for (uint32_t b = 0; b < max_m; b++)
+                if (at[b + 1u] - at[b] > 1u)
+                    std::sort(order.begin() + at[b], order.begin() + at[b + 1u], [&](uint32_t i, uint32_t j) { return z[i] < z[j]; });
+        }
         for (uint32_t j = 0; j < max_m; j++) z[j] = norminv(z[j]);
-        CPD_TRY(ctx->tp_z.ensure(sizeof(double) * max_m));
-        CPD_TRY(cudaMemcpyAsync(ctx->tp_z.p, z.data(), sizeof(double) * max_m, cudaMemcpyHostToDevice, s));
-        ctx->tp_m = max_m;
-        S.h2d += sizeof(double) * max_m;
+        if (ctx->tp_m != max_m) {
+            ctx->tp_m = 0;
+            CPD_TRY(ctx->tp_z.ensure(sizeof(double) * max_m));
+            CPD_TRY(cudaMemcpyAsync(ctx->tp_z.p, z.data(), sizeof(double) * max_m, cudaMemcpyHostToDevice, s));
+            CPD_TRY(cudaStreamSynchronize(s));  // z is about to go
+            ctx->tp_m = max_m;
+            S.h2d += sizeof(double) * max_m;
+        }
+        if (pieces) {
+            // the counts' reciprocals, and the counts | sorted z | ranks
+            ctx->tp_tab_m = 0;
+            std::vector<double> tab(2u * (max_m + 2u) + (size_t)max_m + (max_m + 1u) / 2u);
+            float *z32 = reinterpret_cast<float *>(tab.data() + 2u * (max_m + 2u));
+            uint32_t *rank = reinterpret_cast<uint32_t *>(z32 + 2u * max_m);
+            uint32_t rz = 0;
+            for (uint32_t i = 0; i < max_m; i++) {
+                const uint32_t j = order[i];
+                rank[j] = 0xffffffffu;
+                if (!std::isfinite(z[j])) continue;
+                split_f32(z[j], z32[2 * rz], z32[2 * rz + 1]);
+                rank[j] = rz++;
+            }
+            for (uint32_t c = 0; c < max_m + 2u; c++) {
+                tab[2u * c] = 1.0 / (double)c;
+                tab[2u * c + 1u] = (double)c;
+            }
+            CPD_TRY(ctx->tp_tab.ensure(sizeof(double) * tab.size()));
+            CPD_TRY(cudaMemcpyAsync(ctx->tp_tab.p, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, s));
+            CPD_TRY(cudaStreamSynchronize(s));
+            ctx->tp_rz = rz;
+            ctx->tp_tab_m = max_m;
+            S.h2d += sizeof(double) * tab.size();
+        }
     }
     const size_t out_bytes = sizeof(double) * (size_t)n * D.B;
-    CPD_TRY(ctx->tp_design.ensure(sizeof(DevDesign)));
-    CPD_TRY(ctx->tp_lam.ensure(sizeof(double) * n));
+    // the design and the wavelengths in one copy
+    const size_t lam_off = (sizeof(DevDesign) + 255) & ~size_t(255), in_bytes = lam_off + sizeof(double) * n;
+    CPD_TRY(S.h_in.ensure(in_bytes));
+    CPD_TRY(ctx->tp_design.ensure(in_bytes));
     CPD_TRY(ctx->tp_out.ensure(out_bytes));
     CPD_TRY(ctx->tp_rays.ensure(sizeof(uint32_t) * n));
-    CPD_TRY(cudaMemcpyAsync(ctx->tp_design.p, &D, sizeof(DevDesign), cudaMemcpyHostToDevice, s));
-    CPD_TRY(cudaMemcpyAsync(ctx->tp_lam.p, wavelengths, sizeof(double) * n, cudaMemcpyHostToDevice, s));
+    std::vector<uint32_t> rays(n);
+    if (pieces) {
+        D.wmin = 0.0;  // a point is its wavelength
+        D.wmax = 1.0;
+        D.dc.wmin = ff::F2{0.f, 0.f};
+        D.dc.wspan = ff::F2{1.f, 0.f};
+    }
+    std::memcpy(S.h_in.p, &D, sizeof(DevDesign));
+    std::memcpy(S.h_in.as<char>() + lam_off, wavelengths, sizeof(double) * n);
+    CPD_TRY(cudaMemcpyAsync(ctx->tp_design.p, S.h_in.p, in_bytes, cudaMemcpyHostToDevice, s));
+    const DevDesign *dd = ctx->tp_design.as<DevDesign>();
+    const double *dl = reinterpret_cast<const double *>(ctx->tp_design.as<char>() + lam_off);
     CPD_TRY(cudaEventRecord(S.ev0, s));
-    launch_tp_adaptive(ctx->tp_design.as<DevDesign>(), D.B, ctx->tp_lam.as<double>(), n, ctx->tp_z.as<double>(),
-                       max_m, ctx->tp_out.as<double>(), ctx->tp_rays.as<uint32_t>(), s);
+    if (pieces) {
+        CPD_TRY(ctx->tp_lp.ensure(sizeof(LamParams) * n));
+        CPD_TRY(ctx->tp_t64.ensure(sizeof(double) * n));
+        TpArgs a{};
+        a.d = dd;
+        a.lambdas = dl;
+        a.n = n;
+        a.max_m = max_m;
+        a.z64 = ctx->tp_z.as<double>();
+        a.cnt = ctx->tp_tab.as<double2>();
+        a.z32 = reinterpret_cast<const float2 *>(a.cnt + max_m + 2u);
+        a.rank = reinterpret_cast<const uint32_t *>(a.z32 + max_m);
+        a.lp = ctx->tp_lp.as<LamParams>();
+        a.t64 = ctx->tp_t64.as<double>();
+        a.out = ctx->tp_out.as<double>();
+        a.rays_out = ctx->tp_rays.as<uint32_t>();
+        a.guards = default_guards();
+        a.Rz = ctx->tp_rz;
+        launch_tp_pieces(a, D.B, s);
+    } else {
+        launch_tp_adaptive(dd, D.B, dl, n, ctx->tp_z.as<double>(), max_m, ctx->tp_out.as<double>(),
+                           ctx->tp_rays.as<uint32_t>(), s);
+    }
     CPD_TRY(cudaGetLastError());
     CPD_TRY(cudaEventRecord(S.ev1, s));
     CPD_TRY(cudaMemcpyAsync(out, ctx->tp_out.p, out_bytes, cudaMemcpyDeviceToHost, s));
-    if (rays_out)
-        CPD_TRY(cudaMemcpyAsync(rays_out, ctx->tp_rays.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s));
+    CPD_TRY(cudaMemcpyAsync(rays.data(), ctx->tp_rays.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s));
     CPD_TRY(cudaStreamSynchronize(s));
+    S.launches = pieces ? 2 : 1;
+    // wavelengths with hits of more than one transmittance, by the general kernel
+    for (uint32_t i = 0; i < n; i++)
+        if (rays[i] == 0u) {
+            launch_tp_adaptive(dd, D.B, dl + i, 1, ctx->tp_z.as<double>(), max_m, ctx->tp_out.as<double>() + (size_t)i * D.B,
+                               ctx->tp_rays.as<uint32_t>() + i, s);
+            CPD_TRY(cudaGetLastError());
+            CPD_TRY(cudaMemcpyAsync(out + (size_t)i * D.B, ctx->tp_out.as<double>() + (size_t)i * D.B, sizeof(double) * D.B,
+                                    cudaMemcpyDeviceToHost, s));
+            CPD_TRY(cudaMemcpyAsync(&rays[i], ctx->tp_rays.as<uint32_t>() + i, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+            CPD_TRY(cudaStreamSynchronize(s));
+            S.launches++;
+        }
+    if (rays_out) std::memcpy(rays_out, rays.data(), sizeof(uint32_t) * n);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, S.ev0, S.ev1);
     S.last_ms = ms;
-    S.launches = 1;
-    S.h2d += sizeof(DevDesign) + sizeof(double) * n;
-    S.d2h += out_bytes + (rays_out ? sizeof(uint32_t) * n : 0);
+    S.h2d += in_bytes;
+    S.d2h += out_bytes + sizeof(uint32_t) * n;
     return CPD_OK;
 }
 
