@@ -1,6 +1,7 @@
 """transmission_probability by certified pieces: rays consumed and p(d|lambda) bits equal the
 oracle's, over designs that lose rays in every way, budgets around the chunk and the limit of the
 tables (beyond it, and without a coating, the general kernel), and detectors of few and many bins.
+"""
 import numpy as np
 import pytest
 
