@@ -2332,10 +2332,11 @@ __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
                 const float sg = ra.w > 0.f ? -1.f : 1.f;  // the rays' dz fall with their index
                 uint32_t jb = 0u, je = 0u;
                 if (act) {
-                    const EdgeRays er = edge_rays(rc.x, rc.y, sg, rb.y, [&](uint32_t j) {
+                    const float a0 = sg * (ra.z - ed.v), a1 = sg * ra.w, a2 = sg * rb.x;
+                    const EdgeRays er = edge_rays(rc.x, rc.y, rb.y, [&](uint32_t j) {
                         const float2 z = __ldg(zt + j);
                         const float dd = (ra.x - z.x) + (ra.y - z.y);
-                        return ra.z + dd * (ra.w + dd * rb.x) - ed.v;
+                        return a0 + dd * (a1 + dd * a2);
                     });
                     jb = er.jb;
                     je = er.je;

@@ -28,7 +28,7 @@
 // A mixed piece's bins come from its edges when it has at least this many rays per bin it
 // crosses: finding two edges by bisection costs about as much as binning that many rays.
 #ifndef CPD_EDGE_RAYS
-#define CPD_EDGE_RAYS 8
+#define CPD_EDGE_RAYS 4
 #endif
 
 namespace cpd {
@@ -298,24 +298,36 @@ CPD_HD Edge piece_edge(const PieceConst &K, int q, bool ext, bool up)
 }
 
 // The rays [jb, je) of [p0, p1) within e of an edge, by bisection: at(j) is ray j's v less the
-// edge's, sg +-1 the sign that makes sg at(j) rise with j. Rays before jb and from je on lie on
-// their side of the edge.
+// edge's, with the sign that makes it rise with j. Rays before jb and from je on lie on their side
+// of the edge. The bracket keeps both ends' values, so that the window costs nothing more unless a
+// ray is in it.
 struct EdgeRays {
     uint32_t jb, je;
 };
 template <class At>
-CPD_HD EdgeRays edge_rays(uint32_t p0, uint32_t p1, float sg, float e, const At &at)
+CPD_HD EdgeRays edge_rays(uint32_t p0, uint32_t p1, float e, const At &at)
 {
-    uint32_t base = p0;
-    for (uint32_t n = p1 - p0; n > 1u;) {
-        const uint32_t half = n >> 1;
-        base = sg * at(base + half) < 0.f ? base + half : base;
-        n -= half;
+    uint32_t lo = p0 - 1u, hi = p1;  // at(lo) < 0 <= at(hi); the ends stand outside the piece
+    float alo = -1e30f, ahi = 1e30f;
+    while (hi - lo > 1u) {
+        const uint32_t m = lo + ((hi - lo) >> 1);
+        const float a = at(m);
+        const bool before = a < 0.f;
+        lo = before ? m : lo;
+        alo = before ? a : alo;
+        hi = before ? hi : m;
+        ahi = before ? ahi : a;
     }
     EdgeRays r;
-    r.jb = r.je = sg * at(base) < 0.f ? base + 1u : base;
-    while (r.jb > p0 && fabs_f(at(r.jb - 1u)) < e) r.jb--;
-    while (r.je < p1 && fabs_f(at(r.je)) < e) r.je++;
+    r.jb = r.je = hi;
+    if (-alo < e) {
+        r.jb = lo;
+        while (r.jb > p0 && fabs_f(at(r.jb - 1u)) < e) r.jb--;
+    }
+    if (ahi < e) {
+        r.je = hi + 1u;
+        while (r.je < p1 && fabs_f(at(r.je)) < e) r.je++;
+    }
     return r;
 }
 

@@ -94,9 +94,10 @@ int main(int argc, char **argv)
                     EdgeRays r[2];
                     for (int up = 0; up < 2; up++) {
                         const Edge ed = piece_edge(K, bq, ext, up);
-                        r[up] = edge_rays(j0, j1, sg, q.e, [&](uint32_t j) {
+                        const float a0 = sg * (q.v0 - ed.v), a1 = sg * q.v1, a2 = sg * q.v2;
+                        r[up] = edge_rays(j0, j1, q.e, [&](uint32_t j) {
                             const float dd = dz_of(j) - q.dz0;
-                            return q.v0 + dd * (q.v1 + dd * q.v2) - ed.v;
+                            return a0 + dd * (a1 + dd * a2);
                         });
                         for (uint32_t j = r[up].jb; j < r[up].je && ed.emit; j++) {
                             if (out[j - j0] == -2) wrong++;  // listed twice
@@ -123,7 +124,7 @@ int main(int argc, char **argv)
             }
         }
     }
-    std::printf("rays %ld decided %ld wrong %ld edge %ld whole %ld mixed %ld pieces %ld by_edges %ld\n", rays, decided, wrong,
-                edge, whole, mixed, pieces, by_edges);
+    std::printf("rays %ld decided %ld wrong %ld edge %ld whole %ld mixed %ld pieces %ld by_edges %ld\n",
+                rays, decided, wrong, edge, whole, mixed, pieces, by_edges);
     return 0;
 }
