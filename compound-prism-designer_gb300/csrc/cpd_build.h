@@ -117,8 +117,9 @@ CPD_HD void source(const cpd_spectrometer_params &p, cpd_design &d)
     d.beam_y_mean = p.beam_y_mean;
 }
 
-// f64 tables -> device record (exact part copied, FP32 fast-path constants derived in f64).
-CPD_HDN inline void to_dev(const cpd_design &d, DevDesign &D)
+// f64 tables -> device record but for the float-float copies: the exact part copied, the FP32
+// fast-path constants derived in f64.
+CPD_HDN inline void to_dev_exact(const cpd_design &d, DevDesign &D)
 {
     memset(&D, 0, sizeof(D));
     D.G = d.nglass;
@@ -185,47 +186,63 @@ CPD_HDN inline void to_dev(const cpd_design &d, DevDesign &D)
                            finite(D.intercept) && finite(D.bin_size);
         f.pieces = D.ar && circle && frame && sizes ? 1u : 0u;
     }
-    DFConst &c = D.dc;
-    auto sp = [](double v) {
-        ff::F2 r;
-        ff::split(v, r.hi, r.lo);
-        return r;
-    };
-    for (int k = 0; k < CPD_MAX_GLASS; k++) {
-        for (int i = 0; i < 6; i++) c.glass[k][i] = sp(D.glass[k][i]);
-        c.ppx[k] = sp(D.ppx[k]);
-        c.ppy[k] = sp(D.ppy[k]);
-        c.pnx[k] = sp(D.pnx[k]);
-        c.pny[k] = sp(D.pny[k]);
+}
+
+// The i-th value of the float-float copies (DFConst's fields in order) of a record whose exact part
+// is set.
+CPD_HDN inline double dev_value(const DevDesign &D, int i)
+{
+    if (i < CPD_MAX_GLASS * 6) return (&D.glass[0][0])[i];
+    i -= CPD_MAX_GLASS * 6;
+    if (i < CPD_MAX_GLASS) return D.ppx[i];
+    i -= CPD_MAX_GLASS;
+    if (i < CPD_MAX_GLASS) return D.ppy[i];
+    i -= CPD_MAX_GLASS;
+    if (i < CPD_MAX_GLASS) return D.pnx[i];
+    i -= CPD_MAX_GLASS;
+    if (i < CPD_MAX_GLASS) return D.pny[i];
+    i -= CPD_MAX_GLASS;
+    switch (i) {
+    case 0: return D.height;
+    case 1: return D.ccx;
+    case 2: return D.ccy;
+    case 3: return x::mul(D.crad, D.crad);
+    case 4: return x::div(1.0, D.crad);
+    case 5: return D.cbx;
+    case 6: return D.cby;
+    case 7: return D.cbr2;
+    case 8: return x::sub(D.cbx, D.ccx);
+    case 9: return x::sub(D.cby, D.ccy);
+    case 10: return D.bin_size;
+    case 11: return D.slope;
+    case 12: return x::div(1.0, D.slope);
+    case 13: return D.intercept;
+    case 14: return D.min_ci;
+    case 15: return D.L;
+    case 16: return D.dnx;
+    case 17: return D.dny;
+    case 18: return D.dpx;
+    case 19: return D.dpy;
+    case 20: return D.dux;
+    case 21: return D.duy;
+    case 22: return x::sub(D.dpx, D.cbx);
+    case 23: return x::sub(D.dpy, D.cby);
+    case 24: return D.wmin;
+    case 25: return x::sub(D.wmax, D.wmin);
+    case 26: return D.bw;
+    default: return D.bym;
     }
-    c.height = sp(D.height);
-    c.ccx = sp(D.ccx);
-    c.ccy = sp(D.ccy);
-    c.rc2 = sp(x::mul(D.crad, D.crad));
-    c.irc = sp(x::div(1.0, D.crad));
-    c.cbx = sp(D.cbx);
-    c.cby = sp(D.cby);
-    c.cbr2 = sp(D.cbr2);
-    c.vx = sp(x::sub(D.cbx, D.ccx));
-    c.vy = sp(x::sub(D.cby, D.ccy));
-    c.bin_size = sp(D.bin_size);
-    c.slope = sp(D.slope);
-    c.islope = sp(x::div(1.0, D.slope));
-    c.intercept = sp(D.intercept);
-    c.min_ci = sp(D.min_ci);
-    c.L = sp(D.L);
-    c.dnx = sp(D.dnx);
-    c.dny = sp(D.dny);
-    c.dpx = sp(D.dpx);
-    c.dpy = sp(D.dpy);
-    c.dux = sp(D.dux);
-    c.duy = sp(D.duy);
-    c.qx = sp(x::sub(D.dpx, D.cbx));
-    c.qy = sp(x::sub(D.dpy, D.cby));
-    c.wmin = sp(D.wmin);
-    c.wspan = sp(x::sub(D.wmax, D.wmin));
-    c.bw = sp(D.bw);
-    c.bym = sp(D.bym);
+}
+static_assert(sizeof(DFConst) == sizeof(ff::F2) * (CPD_MAX_GLASS * 10 + 28), "dev_value lists DFConst's fields");
+
+CPD_HDN inline void to_dev(const cpd_design &d, DevDesign &D)
+{
+    to_dev_exact(d, D);
+    for (int i = 0; i < CPD_MAX_GLASS * 10 + 28; i++) {
+        ff::F2 v;
+        ff::split(dev_value(D, i), v.hi, v.lo);
+        reinterpret_cast<ff::F2 *>(&D.dc)[i] = v;
+    }
 }
 
 // detector_array_positioning (spectrometer.rs:322-364) with fit_ray_difference_surface

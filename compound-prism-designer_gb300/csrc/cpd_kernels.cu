@@ -80,32 +80,228 @@ __device__ __forceinline__ void push_ranges(const LaunchArgs &a, uint32_t d, uin
     }
 }
 
-// Designs built on the device from parameter records (CPD_BUILD_ON_DEVICE): one thread
-// per design, the f64 construction of cpd_build.h (positioning first when the pass's
-// acceptance is positive), written straight into the pass's design records. A design whose
-// construction fails keeps its status in the record; the setup then loses all its rays.
+// Designs built on the device from parameter records: the f64 construction of cpd_build.h, eight
+// lanes to a design. FP64 bounds it: a warp instruction takes its scheduler ~64 cycles whatever its
+// active lanes, so what counts is the length of one design's program. The lanes take a face's sine
+// and cosine each, the positioning's two traces run on two of them, and the device record's ~95
+// float splits are spread over all; the rest every lane does alike. (One thread per design, which
+// also built the prism twice: 330 us for 512 designs.)
+constexpr uint32_t kBuildLanes = 8;
+constexpr uint32_t kBuildPerWarp = 32 / kBuildLanes;
+struct BuildScratch {
+    cpd_design d;
+    DevDesign D;
+    double nx[kBuildLanes], ny[kBuildLanes], off[kBuildLanes];
+};
+
+__device__ __forceinline__ double shfl_d(double v, uint32_t src)
+{
+    return __longlong_as_double(__shfl_sync(0xffffffffu, __double_as_longlong(v), (int)src));
+}
+
+// build::design_positioned of record p into S.d (zero-filled on an error), by lane l of the
+// design's eight. The operations and their order are those of build::prism, position and design.
+__device__ __forceinline__ int build_design(const cpd_spectrometer_params &p, double acceptance, BuildScratch &S, uint32_t l,
+                                            uint32_t lane)
+{
+    using build::V2;
+    cpd_design &d = S.d;
+    for (uint32_t i = l; i < sizeof(cpd_design) / 4; i += kBuildLanes) reinterpret_cast<uint32_t *>(&d)[i] = 0u;
+    const int G0 = p.nglass, G = G0 < 1 ? 1 : G0 > CPD_MAX_GLASS ? CPD_MAX_GLASS : G0;
+    const double height = p.height, h2 = x::mul(height, 0.5);
+    // face l's normal and the length it takes; the last lane: the detector's normal
+    const V2 nl = build::rot180(build::angled((int)l <= G && l < kBuildLanes - 1u ? p.angles[l] : p.det_angle));
+    S.nx[l] = nl.x;
+    S.ny[l] = nl.y;
+    S.off[l] = x::mul(fabs(x::div(nl.y, nl.x)), h2);
+    __syncwarp();
+    int prism_err = G0 != G || !(height > 0.0) || !(fabs(p.curvature) > 0.0) || !(fabs(p.curvature) <= 1.0)
+                        ? (int)CPD_INVALID_ARGUMENT : 0;
+    // create_joined_trapezoids
+    bool finite = true;
+    double mx = S.off[0];
+    for (int k = 0; k <= G; k++) {
+        if (k) {
+            const bool turn = build::sign_bit(S.ny[k - 1]) != build::sign_bit(S.ny[k]);
+            const double d1 = S.off[k - 1], d2 = S.off[k];
+            mx = x::add(mx, x::add(p.lengths[k - 1], turn ? x::add(d1, d2) : fabs(x::sub(d1, d2))));
+        }
+        if (k < G) {
+            if (l == 0u) {
+                d.face_point[k][0] = mx;
+                d.face_point[k][1] = h2;
+                d.face_normal[k][0] = S.nx[k];
+                d.face_normal[k][1] = S.ny[k];
+            }
+            finite = finite && build::finite(mx) && build::finite(S.nx[k]);
+        }
+    }
+    // CurvedPlane::from_hyperplane
+    const V2 last_pt{mx, h2}, last_n{S.nx[G], S.ny[G]};
+    const double kc = p.curvature;
+    const double chord = fabs(x::div(height, last_n.x));
+    const double radius = x::div(x::mul(chord, 0.5), fabs(kc));
+    const double apothem = x::sqrt_(x::sub(x::mul(radius, radius), x::mul(x::mul(chord, chord), 0.25)));
+    const double sagitta = x::sub(radius, apothem);
+    const V2 c = build::vfma(last_n, copysign(apothem, kc), last_pt), m = build::vfma(last_n, -copysign(sagitta, kc), last_pt);
+    const double r2 = x::add(x::mul(sagitta, sagitta), x::mul(x::mul(chord, chord), 0.25));
+    if (!prism_err && (!finite || !build::finite(radius) || !build::finite(apothem))) prism_err = CPD_INVALID_ARGUMENT;
+    if (l == 0u) {
+        d.nglass = G;
+        d.ar_coated = p.ar_coated ? 1 : 0;
+        d.height = height;
+        d.exit_center[0] = c.x;
+        d.exit_center[1] = c.y;
+        d.exit_radius = radius;
+        d.exit_bound_center[0] = m.x;
+        d.exit_bound_center[1] = m.y;
+        d.exit_bound_r2 = r2;
+        build::source(p, d);
+    }
+    for (uint32_t i = l; i < CPD_MAX_GLASS * 6u; i += kBuildLanes) (&d.glass[0][0])[i] = (&p.glass[0][0])[i];
+    __syncwarp();
+    int e = 0;
+    double pos[2] = {p.det_position[0], p.det_position[1]};
+    int32_t flipped = p.det_flipped;
+    if (acceptance > 0.0) {
+        // detector_array_positioning: the rays of the acceptance band's two ends, one lane each
+        e = acceptance <= 1.0 ? prism_err : (int)CPD_INVALID_ARGUMENT;
+        DevDesign &D = S.D;
+        if (l == 0u) {
+            D.G = G;
+            D.ar = d.ar_coated;
+            D.height = height;
+            D.ccx = c.x;
+            D.ccy = c.y;
+            D.crad = radius;
+            D.cbx = m.x;
+            D.cby = m.y;
+            D.cbr2 = r2;
+            D.wmin = p.wavelength_bounds[0];
+            D.wmax = p.wavelength_bounds[1];
+            D.bym = p.beam_y_mean;
+        }
+        for (uint32_t i = l; i < CPD_MAX_GLASS * 6u; i += kBuildLanes) (&D.glass[0][0])[i] = (&d.glass[0][0])[i];
+        for (uint32_t k = l; k < CPD_MAX_GLASS; k += kBuildLanes) {
+            D.ppx[k] = d.face_point[k][0];
+            D.ppy[k] = d.face_point[k][1];
+            D.pnx[k] = d.face_normal[k][0];
+            D.pny[k] = d.face_normal[k][1];
+        }
+        __syncwarp();
+        const double uh = x::mul(fmax(x::sub(1.0, acceptance), 0.0), 0.5);
+        x::Ray r{0.0, D.bym, 1.0, 0.0, 1.0, 1.0};
+        int er = 0;
+        if (l < 2u && !e) er = x::prism(D, x::wavelength(D, l ? x::sub(1.0, uh) : uh), r);
+        __syncwarp();
+        const uint32_t a0 = lane & ~(kBuildLanes - 1u);
+        const int e0 = __shfl_sync(0xffffffffu, er, (int)a0), e1 = __shfl_sync(0xffffffffu, er, (int)a0 + 1);
+        const double lox = shfl_d(r.ox, a0), loy = shfl_d(r.oy, a0), lodx = shfl_d(r.dx, a0), lody = shfl_d(r.dy, a0);
+        const double upx = shfl_d(r.ox, a0 + 1u), upy = shfl_d(r.oy, a0 + 1u), updx = shfl_d(r.dx, a0 + 1u),
+                     updy = shfl_d(r.dy, a0 + 1u);
+        const double tm = x::mul(x::add(r.ts, r.tp), 0.5), t0 = shfl_d(tm, a0), t1 = shfl_d(tm, a0 + 1u);
+        if (!e) e = e0 ? e0 : e1;
+        if (!e && (t0 <= 1e-3 || t1 <= 1e-3)) e = CPD_RAYTRACE_ANGULAR_RESPONSE_TOO_WEAK;
+        // rot90(angled(det_angle)); S.n? of the last lane is its rot180
+        const V2 spec{x::mul(S.ny[kBuildLanes - 1], p.det_length), x::mul(-S.nx[kBuildLanes - 1], p.det_length)};
+        const double ca = updx, cb = -lodx, cc = updy, dd = -lody;
+        const double det = x::sub(x::mul(ca, dd), x::mul(cb, cc));
+        if (!e && det == 0.0) e = CPD_RAYTRACE_NO_SURFACE_INTERSECTION;
+        const double i10 = x::div(-cc, det), i11 = x::div(ca, det);
+        double tx = x::add(x::sub(spec.x, upx), lox), ty = x::add(x::sub(spec.y, upy), loy);
+        double d2 = x::add(x::mul(i10, tx), x::mul(i11, ty));
+        int32_t fl = 0;
+        if (!(d2 > 0.0)) {
+            tx = x::add(x::sub(-spec.x, upx), lox);
+            ty = x::add(x::sub(-spec.y, upy), loy);
+            d2 = x::add(x::mul(i10, tx), x::mul(i11, ty));
+            if (!e && d2 < 0.0) e = CPD_RAYTRACE_NO_SURFACE_INTERSECTION;
+            fl = 1;
+        }
+        pos[0] = x::fma_(lodx, d2, lox);
+        pos[1] = x::fma_(lody, d2, loy);
+        flipped = fl;
+    }
+    if (!e) {
+        if (p.bin_count == 0 || p.bin_count > CPD_MAX_BINS || !(p.linear_slope > 0.0) || !(p.bin_size > 0.0) ||
+            !(p.det_length > 0.0) || !(p.wavelength_bounds[1] >= p.wavelength_bounds[0]))
+            e = CPD_INVALID_ARGUMENT;
+        else e = prism_err;
+    }
+    const double min_ci = build::cos_(p.max_incident_angle);
+    const V2 n{S.nx[kBuildLanes - 1], S.ny[kBuildLanes - 1]};
+    const V2 u = flipped ? build::rot90(n) : build::rot90ccw(n);
+    const V2 mid = build::vfma(u, x::mul(p.det_length, 0.5), V2{pos[0], pos[1]});
+    const double dx = mid.x, dy = x::sub(mid.y, p.beam_y_mean);
+    const double size = x::sqrt_(x::add(x::mul(dx, dx), x::mul(dy, dy)));
+    const double deviation = fabs(x::div(dy, size));
+    __syncwarp();
+    if (e) {
+        for (uint32_t i = l; i < sizeof(cpd_design) / 4; i += kBuildLanes) reinterpret_cast<uint32_t *>(&d)[i] = 0u;
+    } else if (l == 0u) {
+        d.bin_count = p.bin_count;
+        d.bin_size = p.bin_size;
+        d.linear_slope = p.linear_slope;
+        d.linear_intercept = p.linear_intercept;
+        d.min_ci = min_ci;
+        d.det_length = p.det_length;
+        d.det_normal[0] = n.x;
+        d.det_normal[1] = n.y;
+        d.det_direction[0] = u.x;
+        d.det_direction[1] = u.y;
+        d.det_position[0] = pos[0];
+        d.det_position[1] = pos[1];
+        d.size = size;
+        d.deviation = deviation;
+    }
+    __syncwarp();
+    return e;
+}
+
+// build::to_dev of S.d into S.D, the float-float copies by all eight lanes.
+__device__ __forceinline__ void build_to_dev(BuildScratch &S, uint32_t l)
+{
+    DevDesign &D = S.D;
+    // the exact tables and the FP32 constants, then the values to split in DFConst's order
+    if (l == 0u) build::to_dev_exact(S.d, D);
+    __syncwarp();
+    for (uint32_t i = l; i < sizeof(DFConst) / sizeof(ff::F2); i += kBuildLanes) {
+        ff::F2 v;
+        ff::split(build::dev_value(D, (int)i), v.hi, v.lo);
+        reinterpret_cast<ff::F2 *>(&D.dc)[i] = v;
+    }
+    __syncwarp();
+}
+
+// Written straight into the pass's design records. A design whose construction fails keeps its
+// status in the record; the setup then loses all its rays.
 __global__ void __launch_bounds__(32) build_kernel(const LaunchArgs a)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.njobs) return;
-    cpd_design d;
-    const int e = build::design_positioned(a.params[i], a.build_acceptance, d);
-    DevDesign D;
-    build::to_dev(d, D);
-    D.status = e;
-    if (e) D.B = a.jobs[i].B;
-    const_cast<DevDesign *>(a.designs)[i] = D;
+    __shared__ __align__(16) BuildScratch S[kBuildPerWarp];
+    const uint32_t lane = threadIdx.x, sub = lane / kBuildLanes, l = lane % kBuildLanes;
+    const uint32_t i = min(blockIdx.x * kBuildPerWarp + sub, a.njobs - 1u);  // (a spare group repeats the last design)
+    const int e = build_design(a.params[i], a.build_acceptance, S[sub], l, lane);
+    build_to_dev(S[sub], l);
+    if (l == 0u) {
+        S[sub].D.status = e;
+        if (e) S[sub].D.B = a.jobs[i].B;
+    }
+    __syncwarp();
+    uint4 *out = reinterpret_cast<uint4 *>(const_cast<DevDesign *>(a.designs) + i);
+    for (uint32_t w = l; w < sizeof(DevDesign) / 16; w += kBuildLanes) out[w] = reinterpret_cast<const uint4 *>(&S[sub].D)[w];
 }
 
 // cpd_design records from parameter records, for the host (cpd_design_build_device).
 __global__ void __launch_bounds__(32) build_records_kernel(const cpd_spectrometer_params *p, uint32_t n,
                                                            double acceptance, cpd_design *out, int32_t *status)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    cpd_design d;
-    status[i] = build::design_positioned(p[i], acceptance, d);
-    out[i] = d;
+    __shared__ __align__(16) BuildScratch S[kBuildPerWarp];
+    const uint32_t lane = threadIdx.x, sub = lane / kBuildLanes, l = lane % kBuildLanes;
+    const uint32_t i = min(blockIdx.x * kBuildPerWarp + sub, n - 1u);
+    const int e = build_design(p[i], acceptance, S[sub], l, lane);
+    if (l == 0u) status[i] = e;
+    uint32_t *o = reinterpret_cast<uint32_t *>(out + i);
+    for (uint32_t w = l; w < sizeof(cpd_design) / 4; w += kBuildLanes) o[w] = reinterpret_cast<const uint32_t *>(&S[sub].d)[w];
 }
 
 
@@ -3524,7 +3720,7 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
         launches++;
     }
     if (a.params) {
-        launch_k(build_kernel, (a.njobs + 31u) / 32u, 32, 0, stream, false, a);
+        launch_k(build_kernel, (a.njobs + kBuildPerWarp - 1u) / kBuildPerWarp, 32, 0, stream, false, a);
         launches++;
     }
     if (a.total_rows) {
@@ -3685,7 +3881,7 @@ void launch_build_records(const cpd_spectrometer_params *p, uint32_t n, double a
                           int32_t *status, cudaStream_t stream)
 {
     if (!n) return;
-    build_records_kernel<<<(n + 31) / 32, 32, 0, stream>>>(p, n, acceptance, out, status);
+    build_records_kernel<<<(n + kBuildPerWarp - 1u) / kBuildPerWarp, 32, 0, stream>>>(p, n, acceptance, out, status);
 }
 
 void launch_trace_pairs(const DevDesign *d, const double *lam_u, const double *z64, uint32_t n, uint32_t mode,
