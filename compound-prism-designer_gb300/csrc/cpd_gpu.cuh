@@ -75,6 +75,8 @@ struct Control {
     unsigned int overflow;
     unsigned int tiles_done;  // entropy tiles (rows_kernel: blocks) finished (single-design passes)
     unsigned long long group_counter;  // rows_kernel: groups claimed past each team's first
+    unsigned int heavy_count;          // heavy rows listed by the setup
+    unsigned int pad;
 };
 
 // Bits of Control::overflow: the re-trace queue was too small; a table could not be made on
@@ -87,6 +89,13 @@ struct HostStatus {
     unsigned long long queue_count;
     unsigned int overflow;
     unsigned int pad;
+};
+
+// A wavelength row with many rays for the float-float trace, listed by the setup: its place in
+// the pass and its ranges (LamParams: core, band).
+struct alignas(16) HeavyRow {
+    unsigned long long row, pad;
+    uint4 ranges;
 };
 
 // Copies of each per-design ray counter: thousands of warps add to the counters of one
@@ -174,6 +183,7 @@ struct LaunchArgs {
     uint32_t max_B;       // widest detector of the launch
     uint64_t total_groups;  // groups of rows of the designs with J.pieces
     uint32_t team;          // rows_kernel: warps per group
+    HeavyRow *heavy;        // the rows rows_kernel gives a whole block (teams smaller than one), or nullptr
     Guards guards;
     double yguard_rel;
     double *p_out;        // optional W x B for the single design of the launch
@@ -300,6 +310,10 @@ int loop_ctas_per_sm();
 // its most rows. With 512 cells (6 KB) four warps of a block keep 20 warps per SM resident.
 constexpr uint32_t kRowsCells = 512;
 constexpr uint32_t kRowsGroup = 8;
+constexpr uint32_t kRowsWarps = 4;  // warps per block, at least a team's
+// Rays of a group per warp from which a pass of one design lists its heavy rows: 1.7 us per 32 of
+// them are 2 ms, a thousand times the launch, and about one design in a thousand has such rows.
+constexpr uint32_t kRowsHeavyGroup = 32768;
 // How rows_kernel splits a pass of this many piece rows with tables of up to R rays: warps per
 // group of rows, and rows per group (a detector's cells may allow fewer).
 struct RowsPlan {

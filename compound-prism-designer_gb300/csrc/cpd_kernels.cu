@@ -447,6 +447,11 @@ __device__ __forceinline__ uint2 setup_failed_row(const LaunchArgs &a, uint64_t 
     return make_uint2(0u, 0u);
 }
 
+// A row with this many rays for the float-float trace goes to rows_kernel<HEAVY>. Almost all such
+// rows have no reference ray (their rays miss the exit face or are reflected) and are traced whole.
+constexpr uint32_t kRowsHeavy = 256;
+constexpr uint32_t kNotHere = 0xffffffffu;  // such a row's ranges in its LamParams: empty
+
 // A row's LamParams after lambda_setup_df: its guard-band rays queued as the mode asks, the
 // record written. Returns the row's fast-path range [core_lo, core_hi) (empty: hi <= lo).
 __device__ __forceinline__ uint2 setup_finish(const LaunchArgs &a, uint32_t d, uint32_t k, uint64_t row, LamParams &P,
@@ -457,6 +462,10 @@ __device__ __forceinline__ uint2 setup_finish(const LaunchArgs &a, uint32_t d, u
     } else if (pieces) {
         // rows_kernel re-traces the guard bands itself; without a reference ray, all of the band
         if (P.all_exact) P.core_lo = P.core_hi = P.band_hi;
+        if (a.heavy && P.band_hi - P.band_lo >= P.core_hi - P.core_lo + kRowsHeavy) {
+            a.heavy[atomicAdd(&a.ctl->heavy_count, 1u)] = HeavyRow{row, 0u, {P.core_lo, P.core_hi, P.band_lo, P.band_hi}};
+            P.core_lo = P.core_hi = P.band_lo = P.band_hi = kNotHere;
+        }
     } else if (a.mode == CPD_TRACE_FP64 || (P.all_exact && a.mode == CPD_TRACE_HYBRID)) {
         push_ranges(a, d, k, P.band_lo, P.band_hi, 0u, 0u);
         P.core_lo = P.core_hi = 0;
@@ -2315,7 +2324,6 @@ __global__ void __launch_bounds__(kEntropyThreads, 4) entropy_block_kernel(const
 #ifndef CPD_ROWS_MAXNREG
 #define CPD_ROWS_MAXNREG 96
 #endif
-constexpr uint32_t kRowsWarps = 4;      // warps per block of rows_kernel, at least a team's
 constexpr uint32_t kRowsMaxTeam = 16;   // most warps of a team
 constexpr uint32_t kRowsBrief = 48;     // a range of up to this many rays goes through fast_ray whole
 constexpr uint32_t kRowsPieces = 15;    // pieces per half-warp (16 ends)
@@ -2374,13 +2382,19 @@ __device__ __forceinline__ void team_sync(uint32_t team, uint32_t T)
 //     design's.
 // Outcomes, flags and sums are those of trace_kernel, retrace_kernel and the entropy kernels,
 // integer for integer.
-template <bool PARAM_FC, bool WITH_P>
+//
+// HEAVY: the rows that the setup listed as having many rays for the float-float trace, each by a
+// whole block, ahead of the groups. A warp takes 1.7 us per 32 such rays, and a pass waits for its
+// last group: one design whose rows are re-traced whole (8 rows of 8192 rays in one warp) made a
+// pass of 512 designs x 16 rows 3.5 ms instead of 0.45 (0.50 so). Without such rows the launch
+// costs 2 us, so a pass of one design has it only where a group could keep its warps for 2 ms.
+template <bool PARAM_FC, bool WITH_P, bool HEAVY>
 __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
 {
     cudaTriggerProgrammaticLaunchCompletion();
     extern __shared__ __align__(16) unsigned char rows_smem[];
-    const uint32_t T = a.team, tid = threadIdx.x, lane = tid & 31u, wib = tid >> 5;
-    const uint32_t nwarps = blockDim.x >> 5, teams = nwarps / T, team = wib / T, tw = wib - team * T;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, wib = tid >> 5, nwarps = blockDim.x >> 5;
+    const uint32_t T = HEAVY ? nwarps : a.team, teams = HEAVY ? 1u : nwarps / T, team = HEAVY ? 0u : wib / T, tw = wib - team * T;
     const uint32_t maxc = ((a.max_B > kRowsCells ? a.max_B : kRowsCells) + 3u) & ~3u;
     float *tab = reinterpret_cast<float *>(rows_smem);
     unsigned long long *bs1 = reinterpret_cast<unsigned long long *>(tab + 4 * ff::kLogTable), *bs2 = bs1 + a.max_B;
@@ -2403,11 +2417,14 @@ __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
     const uint32_t sp = (blockIdx.x * nwarps + wib) % (uint32_t)kSpread;
     // a pass whose table could not be made is re-run by the host: nothing is added
     const bool bad = a.ctl->overflow != 0u;
-    for (uint64_t grp = gteam; grp < a.total_groups && !bad;) {
-        const uint32_t d = PARAM_FC ? 0u : find_job<F_GROUP>(a.jobs, a.njobs, grp);
+    const uint64_t total = HEAVY ? (uint64_t)a.ctl->heavy_count : a.total_groups;
+    for (uint64_t grp = gteam; grp < total && !bad;) {
+        const uint64_t at = HEAVY ? a.heavy[grp].row : grp;
+        const uint32_t d = PARAM_FC ? 0u : find_job<HEAVY ? F_ROW : F_GROUP>(a.jobs, a.njobs, at);
         const DesignJob &J = PARAM_FC ? a.one : a.jobs[d];
         const uint32_t B = J.B;
-        const uint32_t k0 = (uint32_t)(grp - J.grp_off) * J.grp_rows, g = min(J.grp_rows, J.W - k0);
+        const uint32_t k0 = HEAVY ? (uint32_t)(at - J.row_off) : (uint32_t)(at - J.grp_off) * J.grp_rows;
+        const uint32_t g = HEAVY ? 1u : min(J.grp_rows, J.W - k0);
         const uint64_t row0 = J.row_off + k0;
         const float2 *__restrict__ zt = reinterpret_cast<const float2 *>(a.z32) + J.ray_off;
         const LamParams *lp = a.lp + row0;
@@ -2418,9 +2435,9 @@ __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
             K = piece_const(PARAM_FC ? a.fc : Cd);
         }
         // the same in every lane: entries of the lists, the next row, and what is left of the
-        // last rows' mixed pieces: tasks [t0, total), records [ir, nrec) from ray js on
+        // last rows' mixed pieces: tasks [t0, ntask), records [ir, nrec) from ray js on
         uint32_t nwait = 0u, nflag = 0u, nsub = 0u, next = 0u;
-        uint32_t t0 = 0u, total = 0u, ir = 0u, nrec = 0u, js = 0u;
+        uint32_t t0 = 0u, ntask = 0u, ir = 0u, nrec = 0u, js = 0u;
         // of the lane's piece: its tasks
         uint32_t incl = 0u, excl = 0u;
         bool by_edge = false;
@@ -2429,7 +2446,7 @@ __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
         // their lists fill, the float-float steps alone would exceed the instruction cache).
         for (;;) {
             const bool rows_left = next < g || nsub != 0u;
-            const bool work_left = t0 < total || ir < nrec || rows_left;
+            const bool work_left = t0 < ntask || ir < nrec || rows_left;
             if (nflag >= 32u || (nflag && !work_left && !nwait)) {
                 // ---- 32 flagged rays re-traced, one per lane
                 __syncwarp();
@@ -2509,14 +2526,14 @@ __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
                 nflag += __popc(f);
                 continue;
             }
-            if (t0 < total) {
+            if (t0 < ntask) {
                 // ---- 16 tasks of the mixed pieces: two lanes per bin, one edge each
                 // the record of task t: those that start after t0 are marked at their first task
                 const uint32_t tau = lane >> 1, t = t0 + tau;
                 const uint32_t first_rec = __popc(__ballot_sync(0xffffffffu, by_edge && incl <= t0));
                 const uint32_t starts =
                     __reduce_or_sync(0xffffffffu, by_edge && excl > t0 && excl < t0 + 16u ? 1u << (excl - t0) : 0u);
-                const bool act = t < total;
+                const bool act = t < ntask;
                 const uint32_t i = act ? first_rec + __popc(starts & ((2u << tau) - 1u)) : 0u;
                 const float4 ra = w.rec_a[i], rb = w.rec_b[i];
                 const uint4 rc = w.rec_c[i];
@@ -2595,7 +2612,7 @@ __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
                 // the half's row, its core range, and the guard bands around it
                 rl = T == 1u ? min(next + half, g - 1u) : 0u;
                 const bool has = T > 1u || next + half < g;
-                const uint4 rg = *reinterpret_cast<const uint4 *>(&lp[rl].core_lo);  // core, band
+                const uint4 rg = HEAVY ? a.heavy[grp].ranges : *reinterpret_cast<const uint4 *>(&lp[rl].core_lo);  // core, band
                 lo = rg.x;
                 hi = rg.y;
                 uint32_t blo = rg.z, b1 = lo, b2 = hi, bhi = rg.w;
@@ -2637,7 +2654,7 @@ __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
                 const FastLimits Ld = PARAM_FC ? FastLimits{} : fast_limits(Cd, a.guards);
                 const FastLimits &Lm = PARAM_FC ? a.fl : Ld;
                 const LamParams P = lp[rl];
-                if (!again && hl == 0u) w.tfix[rl] = piece_tfix(P);
+                if (!again && hl == 0u) w.tfix[rl] = WITH_P && !HEAVY && P.core_lo == kNotHere ? kNotHere : piece_tfix(P);
                 if (n) z = __ldg(zt + min(j0, hi - 1u));
                 const PieceEnd e = piece_end(C, Lm, K, P, a.guards, z.x, z.y);
                 PieceEnd o = e;
@@ -2677,7 +2694,7 @@ __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
             }
             excl = by_edge ? incl - pe.count : 0u;
             t0 = js = 0u;
-            total = __shfl_sync(0xffffffffu, incl, 31);
+            ntask = __shfl_sync(0xffffffffu, incl, 31);
             ir = __popc(me);
             nrec = ir + __popc(mr);
             if (mixed) {
@@ -2716,7 +2733,7 @@ __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
                         q2 += pq;
                         c1 += cv;
                     }
-                    if (WITH_P) a.p_out[(uint64_t)(k0 + r) * B + b] = (double)cv * J.pscale;
+                    if (WITH_P && (HEAVY || tfix[r] != kNotHere)) a.p_out[(uint64_t)(k0 + r) * B + b] = (double)cv * J.pscale;
                 }
                 if (c1) {
                     if (PARAM_FC) {
@@ -2740,8 +2757,8 @@ __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
             }
         }
         team_sync(team, T);  // the cells are clear for the next group
-        if (nteams >= a.total_groups) break;
-        if (T == 1u) {
+        if (nteams >= total) break;
+        if (!HEAVY && T == 1u) {
             unsigned long long c = 0;
             if (lane == 0) c = atomicAdd(&a.ctl->group_counter, 1ull);
             grp = nteams + __shfl_sync(0xffffffffu, c, 0);
@@ -3678,7 +3695,7 @@ static uint32_t rows_blocks_per_sm(uint32_t warps, uint32_t B)
     if (!n) {
         // one-warp teams need the most shared memory of a kRowsWarps block
         int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rows_kernel<false, false>, 32 * warps,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rows_kernel<false, false, false>, 32 * warps,
                                                       rows_smem_bytes(warps, warps <= kRowsWarps ? warps : 1u, B));
         n = per_sm < 1 ? 1u : (uint32_t)per_sm;
         k.store((uint8_t)n, std::memory_order_relaxed);
@@ -3770,8 +3787,13 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
         const uint32_t warps = std::max(kRowsWarps, a.team), teams = warps / a.team;
         const uint64_t need = (a.total_groups + teams - 1u) / teams;
         const uint64_t resident = (uint64_t)num_sms * rows_blocks_per_sm(warps, a.max_B);
-        auto k = a.spans ? (a.p_out ? rows_kernel<true, true> : rows_kernel<true, false>)
-                         : (a.p_out ? rows_kernel<false, true> : rows_kernel<false, false>);
+        if (a.heavy) {
+            launch_k(a.p_out ? rows_kernel<false, true, true> : rows_kernel<false, false, true>, (unsigned)num_sms,
+                     32 * kRowsMaxTeam, rows_smem_bytes(kRowsMaxTeam, 1u, a.max_B), stream, pdl, a);
+            launches++;
+        }
+        auto k = a.spans ? (a.p_out ? rows_kernel<true, true, false> : rows_kernel<true, false, false>)
+                         : (a.p_out ? rows_kernel<false, true, false> : rows_kernel<false, false, false>);
         launch_k(k, (unsigned)std::min(need, resident), 32 * warps, rows_smem_bytes(warps, teams, a.max_B), stream, pdl, a);
         launches++;
     }
@@ -3856,7 +3878,8 @@ cudaError_t configure_kernels()
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(table_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)table_smem_bytes(kTableRays, kTableRays));
-    const auto rows = {rows_kernel<false, false>, rows_kernel<false, true>, rows_kernel<true, false>, rows_kernel<true, true>};
+    const auto rows = {rows_kernel<false, false, false>, rows_kernel<false, true, false>, rows_kernel<true, false, false>,
+                       rows_kernel<true, true, false>, rows_kernel<false, false, true>, rows_kernel<false, true, true>};
     for (auto k : rows)
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_bytes);
     return e;
@@ -3865,8 +3888,8 @@ cudaError_t configure_kernels()
 const void *single_trace_kernel_fn(const LaunchArgs &a)
 {
     if (!a.total_groups) return reinterpret_cast<const void *>(trace_spans_kernel);
-    return a.p_out ? reinterpret_cast<const void *>(rows_kernel<true, true>)
-                   : reinterpret_cast<const void *>(rows_kernel<true, false>);
+    return a.p_out ? reinterpret_cast<const void *>(rows_kernel<true, true, false>)
+                   : reinterpret_cast<const void *>(rows_kernel<true, false, false>);
 }
 
 uint64_t trace_resident_warps(int num_sms, uint32_t warps_per_cta)

@@ -597,7 +597,11 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     const size_t hist_bytes = sizeof(unsigned long long) * std::max<uint64_t>(hist, 1);
     const size_t old_hist = S.hist.cap;
     // the LamParams, then (single-design passes) one span per 32-row block
-    CPD_TRY(S.lp.ensure(sizeof(LamParams) * std::max<uint64_t>(rows, 1) + sizeof(uint2) * ((rows + 31) / 32)));
+    // or, where rows_kernel's teams are small, a HeavyRow for each
+    const bool heavy = groups && plan.team < kRowsWarps &&
+                       (n > 1 || (uint64_t)plan.group * piece_R / plan.team >= kRowsHeavyGroup);
+    CPD_TRY(S.lp.ensure(sizeof(LamParams) * std::max<uint64_t>(rows, 1) + sizeof(uint2) * ((rows + 31) / 32) +
+                        (heavy ? 16u + sizeof(HeavyRow) * rows : 0)));
     CPD_TRY(S.lx.ensure(sizeof(LamDF) * std::max<uint64_t>(rows, 1)));
     CPD_TRY(S.hist.ensure(hist_bytes));
     if (S.hist.cap != old_hist) S.hist_dirty = true;
@@ -655,6 +659,7 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     a.max_B = max_B;
     a.lp = S.lp.as<LamParams>();
     a.lx = S.lx.as<LamDF>();
+    if (heavy) a.heavy = reinterpret_cast<HeavyRow *>(S.lp.as<char>() + ((sizeof(LamParams) * rows + sizeof(uint2) * ((rows + 31) / 32) + 15u) & ~size_t(15)));
     a.hist = S.hist.as<unsigned long long>();
     a.S1 = S.S1.as<unsigned long long>();
     a.S2 = S.S2.as<unsigned long long>();
