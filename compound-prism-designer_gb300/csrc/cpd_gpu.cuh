@@ -89,6 +89,7 @@ struct HostStatus {
     unsigned long long queue_count;
     unsigned int overflow;
     unsigned int pad;
+    unsigned long long t0, t1;  // LaunchArgs::stamp: the global timer at its start and end, ns
 };
 
 // A wavelength row with many rays for the float-float trace, listed by the setup: its place in
@@ -128,6 +129,9 @@ struct DesignOut {
 constexpr uint32_t kTileCells = 512;
 constexpr uint32_t kTileCellsBatch = CPD_TILE_CELLS_BATCH;
 
+// The first kernel of a pass that is timed by the device's own clock.
+enum : uint32_t { STAMP_NONE, STAMP_SORT, STAMP_Z, STAMP_BUILD, STAMP_SETUP };
+
 struct LaunchArgs {
     const DevDesign *designs;
     const DesignJob *jobs;
@@ -153,6 +157,7 @@ struct LaunchArgs {
     DesignOut *out;       // results (mapped host memory in the context's passes)
     Control *ctl;
     HostStatus *status;   // optional (mapped host memory)
+    uint32_t stamp;       // the kernel that writes status->t0 (the finalize writes t1); STAMP_NONE: none
     uint32_t clear_acc;   // the setup kernel zeroes S1, S2 (acc_cells) and acc (njobs) first
     uint64_t acc_cells;
     QEntry *queue;

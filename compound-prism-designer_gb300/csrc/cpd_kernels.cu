@@ -64,6 +64,19 @@ __device__ __forceinline__ void push_ray(const LaunchArgs &a, uint32_t d, uint32
     else atomicOr(&a.ctl->overflow, kOverflowQueue);
 }
 
+__device__ __forceinline__ unsigned long long global_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// The start of a pass that its kernels time themselves (its first kernel is `which`).
+__device__ __forceinline__ void stamp_start(const LaunchArgs &a, uint32_t which)
+{
+    if (a.stamp == which && blockIdx.x == 0u && blockIdx.y == 0u && threadIdx.x == 0u) a.status->t0 = global_ns();
+}
+
 // The rays [j0, j1) and [j2, j3) of row k, queued with one atomic for the whole run (a row's
 // guard bands can hold dozens of rays; one round trip to the queue counter per ray made a
 // serial chain on the setup's critical path).
@@ -277,6 +290,7 @@ __device__ __forceinline__ void build_to_dev(BuildScratch &S, uint32_t l)
 // status in the record; the setup then loses all its rays.
 __global__ void __launch_bounds__(32) build_kernel(const LaunchArgs a)
 {
+    stamp_start(a, STAMP_BUILD);
     __shared__ __align__(16) BuildScratch S[kBuildPerWarp];
     const uint32_t lane = threadIdx.x, sub = lane / kBuildLanes, l = lane % kBuildLanes;
     const uint32_t i = min(blockIdx.x * kBuildPerWarp + sub, a.njobs - 1u);  // (a spare group repeats the last design)
@@ -331,6 +345,7 @@ constexpr size_t table_smem_bytes(uint32_t buckets, uint32_t R) { return 4u * (s
 // seed's points as 64-bit fractions: no FP64 instruction).
 __global__ void __launch_bounds__(kTableThreads) table_sort_kernel(const LaunchArgs a)
 {
+    stamp_start(a, STAMP_SORT);
     cudaTriggerProgrammaticLaunchCompletion();
     extern __shared__ __align__(16) uint32_t table_smem[];
     __shared__ uint32_t warp_sum[kTableThreads / 32u];
@@ -414,6 +429,7 @@ __global__ void __launch_bounds__(kTableThreads) table_sort_kernel(const LaunchA
 // known order this kernel is all a new seed costs, beside the setup's face loop.
 __global__ void __launch_bounds__(64) table_z_kernel(const LaunchArgs a)
 {
+    stamp_start(a, STAMP_Z);
     cudaTriggerProgrammaticLaunchCompletion();
     if (a.nsort) cudaGridDependencySynchronize();  // the order
     const TableJob t = a.tables[blockIdx.y];
@@ -503,6 +519,7 @@ __device__ __forceinline__ uint2 setup_row(const LaunchArgs &a, uint64_t row, ui
 // pads each to an even number of rays).
 __global__ void __launch_bounds__(32) setup_kernel(const LaunchArgs a)
 {
+    stamp_start(a, STAMP_SETUP);
     // lets the trace kernel's blocks become resident now; they wait for this grid's
     // results in cudaGridDependencySynchronize
     cudaTriggerProgrammaticLaunchCompletion();
@@ -579,6 +596,7 @@ __global__ void __launch_bounds__(32) setup_kernel(const LaunchArgs a)
 // plain call is about half as long.
 __global__ void __launch_bounds__(64) setup_pair_kernel(const LaunchArgs a)
 {
+    stamp_start(a, STAMP_SETUP);
     cudaTriggerProgrammaticLaunchCompletion();
     if (a.clear_acc) {
         const uint64_t gt = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -2093,6 +2111,7 @@ __device__ void finalize_design(const LaunchArgs &a, uint32_t d, const DesignJob
         o.status = D.status;
         a.out[d] = o;
         a.acc[d].rows = rows;
+        if (a.stamp != STAMP_NONE && tid == 0u) a.status->t1 = global_ns();
     }
 }
 
@@ -3333,13 +3352,6 @@ __host__ __device__ inline SlabLayout slab_layout(uint32_t rows, uint32_t cells,
     o += (4 * ((size_t)rows + 1) + 255) & ~size_t(255);
     L.bytes = o;
     return L;
-}
-
-__device__ __forceinline__ unsigned long long global_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
 }
 
 __device__ __forceinline__ unsigned long long load_acquire_sys(const unsigned long long *p)

@@ -320,8 +320,10 @@ int cpd_autotune_batch(cpd_context *ctx, const cpd_design *designs, const cpd_ba
  * (cpd_fitness_gpu then ignores its nwarp hint). Off by default. */
 int cpd_set_autotune(cpd_context *ctx, int on);
 
-/* Device time of the last GPU call's kernels (CUDA events on the context stream), ms,
- * and the number of kernel launches it issued. */
+/* Device time of the last GPU call's kernels, ms, and the number of kernel launches it issued.
+ * CUDA events on the context stream; calls that evaluate one design record none (they add 6 us to
+ * 40) until a context's first cpd_last_timing, and that one returns the time between stamps of the
+ * device's global timer by the call's first kernel and its finalize. */
 int cpd_last_timing(cpd_context *ctx, double *kernel_ms, uint32_t *launches);
 
 /* Per-kernel timing: when on, each pass is launched without graph replay and CUDA
