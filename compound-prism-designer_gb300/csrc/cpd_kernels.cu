@@ -497,27 +497,36 @@ __device__ __forceinline__ uint2 setup_finish(const LaunchArgs &a, uint32_t d, u
 
 // The setup of one wavelength row (below): LamParams and LamDF, and the row's guard-band
 // rays queued. Returns the row's fast-path range [core_lo, core_hi) (empty: hi <= lo).
-__device__ __forceinline__ uint2 setup_row(const LaunchArgs &a, uint64_t row, uint32_t d, double u,
-                                           const DevDesign &sD, uint32_t d0, bool stage_z, const float *sz)
+__device__ __forceinline__ void setup_row(const LaunchArgs &a, uint64_t row, uint32_t d, double u,
+                                          const DevDesign &sD, uint32_t d0, bool stage_z, const float *sz)
 {
     const DesignJob &J = a.jobs[d];
     const uint32_t k = (uint32_t)(row - J.row_off);
     const bool staged = d == d0;
     const DevDesign &D = staged ? sD : a.designs[d];
     const float *z32 = staged && stage_z ? sz : a.z32 + 2 * J.ray_off;
-    if (D.status) return setup_failed_row(a, row);
+    if (D.status) {
+        setup_failed_row(a, row);
+        return;
+    }
     LamParams P;
     lambda_setup_df(D, u, z32, J.Rz, P, a.yguard_rel, a.lx + row, a.adaptive != 0);
-    return setup_finish(a, d, k, row, P, J.pieces != 0u);
+    setup_finish(a, d, k, row, P, J.pieces != 0u);
 }
 
-// One warp per block of 32 rows. The block first copies its design record and, for
+// One thread per row; kSetupThreads per block where that leaves every SM as many warps as it holds
+// (below, a warp per block spreads the rows over more SMs). A block's warps run the same code on
+// one design's tables: 2.3 M rows of 1024 designs take 534 us in blocks of 128 at 96 registers (20
+// warps per SM; 528 at 80, which spills), 538 at the compiler's 107, 613 in blocks of 32, where one
+// issue slot in five waits for instructions. FP32 issue bounds it (5400 instructions per warp: 335 us).
+// The block first copies its design record and, for
 // tables of up to a.stage_cap rays, its sorted z table into shared memory with
 // asynchronous 16-byte copies that are all in flight at once (one memory latency
 // instead of a chain of dependent loads), so the per-wavelength program and its binary
 // searches run on shared-memory operands. Ray tables start 16-byte aligned (the host
 // pads each to an even number of rays).
-__global__ void __launch_bounds__(32) setup_kernel(const LaunchArgs a)
+constexpr uint32_t kSetupThreads = 128;
+__global__ void __maxnreg__(96) setup_kernel(const LaunchArgs a)
 {
     stamp_start(a, STAMP_SETUP);
     // lets the trace kernel's blocks become resident now; they wait for this grid's
@@ -563,19 +572,7 @@ __global__ void __launch_bounds__(32) setup_kernel(const LaunchArgs a)
         asm volatile("cp.async.wait_all;" ::: "memory");
     }
     __syncthreads();
-    uint2 core = make_uint2(0u, 0u);
-    if (row < a.total_rows) core = setup_row(a, row, d, u, sD, d0, stage_z, sz);
-    if (a.spans) {
-        // single-design pass: this block's 32 rows are the trace's block blockIdx.x
-        const bool any = core.y > core.x;
-        const uint32_t lo = __reduce_min_sync(0xffffffffu, any ? core.x : 0xffffffffu);
-        const uint32_t hi = __reduce_max_sync(0xffffffffu, any ? core.y : 0u);
-        if (threadIdx.x == 0) {
-            const uint2 s = hi > lo ? make_uint2(lo, hi) : make_uint2(0u, 0u);
-            a.spans[blockIdx.x] = s;
-            if (s.y > s.x) atomicAdd(&a.ctl->item_counter, (unsigned long long)(s.y - s.x));
-        }
-    }
+    if (row < a.total_rows) setup_row(a, row, d, u, sD, d0, stage_z, sz);
 }
 
 
@@ -3753,12 +3750,13 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
         launches++;
     }
     if (a.total_rows) {
-        // one warp per block: each row is one thread's latency-bound float-float chain,
-        // so spreading the rows over every SM matters
-        const uint32_t blocks = (uint32_t)((a.total_rows + 31) / 32);
+        // 16 warps or more per SM: larger blocks; fewer: each row is one thread's latency-bound
+        // float-float chain, so spreading the rows over every SM matters. A single-design pass
+        // (spans) splits each row's chain over two warps.
+        const uint32_t rows = !a.spans && a.total_rows >= (uint64_t)num_sms * 32u * 16u ? kSetupThreads : 32u;
+        const uint32_t blocks = (uint32_t)((a.total_rows + rows - 1u) / rows);
         const uint32_t cap = a.stage_cap < kStageRays ? a.stage_cap : kStageRays;
-        // a single-design pass (spans) splits each row's chain over two warps
-        launch_k(a.spans ? setup_pair_kernel : setup_kernel, blocks, a.spans ? 64 : 32,
+        launch_k(a.spans ? setup_pair_kernel : setup_kernel, blocks, a.spans ? 64 : rows,
                  2 * ((cap + 1u) & ~1u) * sizeof(float), stream, pdl && a.ntables && !a.params, a);
         launches++;
     }
