@@ -1,9 +1,17 @@
 // cpd_kernels.cu -- the GB300 kernels of the fitness path.
 //
-// A pass over a set of designs runs five kernels on one stream:
+// A pass over a set of designs runs on one stream:
+//   tables   (passes whose ray tables are not resident) the points of each table sorted
+//            (table_sort_kernel) and turned into start heights (table_z_kernel)
+//   build    (designs given as parameter records) eight lanes per design, f64
 //   setup    one thread per (design, wavelength): the flat-face chain in float-float
-//            (cpd_df.h) -> LamParams for the fast path and LamDF for the re-trace;
-//            guard-band rays of the y interval go to the re-trace queue
+//            (cpd_df.h) -> LamParams for the fast path and LamDF for the re-trace
+// and then, for designs whose coated exit face admits certified pieces (cpd_piece.h) under the
+// fixed-N hybrid trace,
+//   rows     rows_kernel: a wavelength's trace, re-trace and entropy by one team of warps, its
+//            cells in shared memory; ahead of it, in passes of many designs, rows_kernel<HEAVY>
+//            for rows that are mostly re-traced;
+// for all others (uncoated designs, the FP32 and FP64 study modes),
 //   trace    persistent warps over work items (design, 32-wavelength block, ray
 //            chunk); lane = wavelength; FP32 exit face + detector per ray; hits
 //            accumulate per lane as run-length fixed-point sums (rays are sorted by
@@ -15,13 +23,14 @@
 //   entropy  one warp (many tiles) or one block (few) per (design, row tile): p = sum/R,
 //            p log2 p, per-bin sums of p and p^2 in float-float with fixed-point
 //            accumulation (order independent)
+// and for both
 //   finalize one warp per design: H(D), MI, SEM convergence (in a single-design pass the
-//            entropy block that completes the last tile runs it).
+//            block that completes the last rows or entropy tile runs it).
 // A single-design pass with a fixed ray count (the plain call) runs setup_pair_kernel (two
-// warps per 32 rows) and trace_spans_kernel (equal shares of the ray slots per warp, the
-// design's constants as kernel parameters) in place of the first two. Adaptive sampling
-// replaces trace and retrace with adaptive1_kernel / adaptive_kernel and
-// adaptive_exact_kernel.
+// warps per 32 rows), and trace_spans_kernel (equal shares of the ray slots per warp) in place
+// of trace; its design's constants are kernel parameters. Adaptive sampling replaces trace and
+// retrace with adaptive1_pieces_kernel / adaptive_block_kernel (designs with pieces),
+// adaptive1_kernel / adaptive_kernel (the others) and adaptive_exact_kernel.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -2402,7 +2411,7 @@ __device__ __forceinline__ void team_sync(uint32_t team, uint32_t T)
 // HEAVY: the rows that the setup listed as having many rays for the float-float trace, each by a
 // whole block, ahead of the groups. A warp takes 1.7 us per 32 such rays, and a pass waits for its
 // last group: one design whose rows are re-traced whole (8 rows of 8192 rays in one warp) made a
-// pass of 512 designs x 16 rows 3.5 ms instead of 0.45 (0.50 so). Without such rows the launch
+// pass of 512 designs x 128 rows 3.5 ms instead of 0.45 (0.50 so). Without such rows the launch
 // costs 2 us, so a pass of one design has it only where a group could keep its warps for 2 ms.
 template <bool PARAM_FC, bool WITH_P, bool HEAVY>
 __global__ void __maxnreg__(CPD_ROWS_MAXNREG) rows_kernel(const LaunchArgs a)
@@ -3715,10 +3724,15 @@ static uint32_t rows_blocks_per_sm(uint32_t warps, uint32_t B)
 RowsPlan plan_rows(uint64_t rows, uint32_t R, uint32_t max_B, int num_sms)
 {
     RowsPlan p;
-    // several warps per row while all teams are resident at once (a second wave would double the
-    // time) and each half-warp keeps 32 rays or more
+    // Several warps per row while all teams are resident at once (4096 rows of 1024 rays by teams of
+    // two, in three waves: 69 us a call instead of 52), and each half-warp's share of the row is up
+    // to 64 rays (mostly fast_ray's, whole) or 256 and more: between, its 15 pieces are so short
+    // that a bin's edges cost more than its rays. 512 rows of 1024 rays (a call, four designs): 128
+    // rays 45.6 us, 256 rays 42.0; 128 rows of 4096: 128 rays 44.3, 256 rays 41.8; but 256 rows of
+    // 1024: 64 rays 40.6, 256 rays 41.7; 128 rows of 2048: 40.3, 41.1.
     p.team = 1u;
     for (uint32_t T = 2u; T <= kRowsMaxTeam && R >= 64u * T; T *= 2u) {
+        if (R > 2u * T * 64u && R < 2u * T * 256u) continue;
         const uint32_t warps = std::max(kRowsWarps, T);
         if (rows <= (uint64_t)num_sms * rows_blocks_per_sm(warps, max_B) * (warps / T)) p.team = T;
     }
