@@ -49,21 +49,13 @@ G_PLAIN, B_PLAIN, W_PLAIN, R_PLAIN = 6, 64, 4096, 1024
 PLAIN_SEED = 20261203 + 1
 # The frozen per-ray operation table of the reference's formulation, keyed by prism count.
 OPS_TABLE = os.path.join(ROOT, "roofline", "ops_per_ray.json")
-# FP32 arithmetic of fast_ray on its full path for an anti-reflection-coated design (exit
-# face, refraction, detector, binning and the guard-band thresholds): adds/muls count 1,
-# FMAs 2, comparisons 0; the 5 hardware estimates (2 sqrt, 3 reciprocals) and the floor
-# are not counted. Rays lost early execute fewer, so this is an upper bound per evaluated
-# ray. (102 before the exit-face terms became polynomials in dz and the exit direction was
-# taken along the detector from dp.)
-FLOP_PER_FAST_RAY = 82
-# Special-function-unit results of fast_ray's full path: 2 square-root and 3 reciprocal
-# estimates.
-SFU_PER_FAST_RAY = 5
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one trace_spans_kernel
-# launch of this workload, from the ncu capture summarised in
-# profiles/fitness_pass_plain_g6_b64_w4096_r1024.md (the figure is copied here when the
-# kernel is re-profiled; bench.py reads no profile file).
-TRACE_TRAFFIC_BYTES = 3045888
+# Of one rows_kernel launch of this workload (it decides most rays by certified pieces, without
+# evaluating them one by one), from the ncu capture summarised in
+# profiles/rows_kernel_plain_and_batched.md: DRAM bytes (dram__bytes_read.sum +
+# dram__bytes_write.sum) and warp instructions (smsp__inst_executed.sum). The figures are copied
+# here when the kernel is re-profiled; bench.py reads no profile file.
+TRACE_TRAFFIC_BYTES = 1038336
+TRACE_WARP_INSTRUCTIONS = 13702911
 
 
 def dist_info():
@@ -581,7 +573,7 @@ def plain_config(l2):
     return {"workload": f"plain gpu_fitness call, one design per call: {G_PLAIN} prisms, {B_PLAIN} bins, "
                         f"{W_PLAIN} wavelengths x {R_PLAIN} rays ({W_PLAIN * R_PLAIN} rays)",
             "prisms": G_PLAIN, "bins": B_PLAIN, "wavelengths": W_PLAIN, "rays_per_wavelength": R_PLAIN,
-            "trace": "fp32 fast path; guard-band rays re-traced in float-float",
+            "trace": "fp32 certified pieces and fast path; guard-band rays re-traced in float-float",
             "accumulation": "int64 fixed point; float-float entropy",
             "l2": l2}
 
@@ -686,30 +678,28 @@ def main():
             t_pass = statistics.median(dev_ms) * 1e-3
             alg = rays * ops["flop"] / t_trace / 1e12
             alg_pass = rays * ops["flop"] / t_pass / 1e12
-            executed = fp.fast_rays * FLOP_PER_FAST_RAY / t_trace / 1e12
+            # warp instructions over the issue slots of 152 SMs x 4 schedulers at the SM clock seen
+            slots = 152 * 4 * (clk["sm_mhz"] or 2070.0) * 1e6 * t_trace
             sfu_alg = rays * (ops["div"] + ops["sqrt"] + ops["log"]) / t_trace / 1e9
-            sfu_exec = fp.fast_rays * SFU_PER_FAST_RAY / t_trace / 1e9
             extras["roofline"] = {
                 "bound": "fp32", "achieved": alg, "peak": peak, "unit": "TFLOP/s", "frac": alg / peak,
                 "traffic": TRACE_TRAFFIC_BYTES,
-                "traffic_source": "ncu capture of trace_spans_kernel on this workload (dram__bytes_read.sum + "
-                                  "dram__bytes_write.sum), profiles/fitness_pass_plain_g6_b64_w4096_r1024.md",
-                "kernel": "trace_spans_kernel", "kernel_ms": kt,
+                "traffic_source": "ncu capture of rows_kernel on this workload (dram__bytes_read.sum + "
+                                  "dram__bytes_write.sum), profiles/rows_kernel_plain_and_batched.md",
+                "kernel": "rows_kernel", "kernel_ms": kt,
                 "frac_algorithmic": alg / peak,
                 "frac_algorithmic_pass": alg_pass / peak,
-                "frac_executed": executed / peak,
+                "warp_instructions": TRACE_WARP_INSTRUCTIONS, "frac_issue": TRACE_WARP_INSTRUCTIONS / slots,
                 "flop_per_ray_algorithmic": ops["flop"],
                 "flop_basis": "the design's W x R rays x the frozen per-ray FLOP of the reference's formulation "
-                              f"(roofline/ops_per_ray.json, G={G_PLAIN}), over the trace kernel's time "
-                              "(frac_algorithmic) and over the whole pass (frac_algorithmic_pass); frac_executed: "
-                              f"{FLOP_PER_FAST_RAY} FP32 FLOP per ray the fast path evaluated",
+                              f"(roofline/ops_per_ray.json, G={G_PLAIN}), over the time of rows_kernel, which traces, "
+                              "re-traces and takes the entropies (frac_algorithmic), and over the whole pass "
+                              "(frac_algorithmic_pass); frac_issue: its warp instructions over the issue slots",
                 "sfu": {"peak_gops": sfu_peak, "algorithmic_gops": sfu_alg, "frac_algorithmic": sfu_alg / sfu_peak,
-                        "executed_gops": sfu_exec, "frac_executed": sfu_exec / sfu_peak,
                         "per_ray_algorithmic": ops["div"] + ops["sqrt"] + ops["log"],
-                        "per_fast_ray_executed": SFU_PER_FAST_RAY,
                         "peak_source": "measured live: reciprocal-square-root chains on all SMs "
                                        "(cpd_measure_sfu_peak)"},
-                "fast_rays": fp.fast_rays, "flop_per_fast_ray": FLOP_PER_FAST_RAY,
+                "fast_rays": fp.fast_rays,
                 "peak_source": "measured live: FP32 FMA probe on all SMs (cpd_measure_fp32_peak)",
                 "retraced": fp.retraced, "hits": fp.hits}
         except Exception as e:  # noqa: BLE001

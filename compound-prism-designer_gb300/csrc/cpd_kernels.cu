@@ -107,7 +107,7 @@ __device__ __forceinline__ void push_ranges(const LaunchArgs &a, uint32_t d, uin
 // active lanes, so what counts is the length of one design's program. The lanes take a face's sine
 // and cosine each, the positioning's two traces run on two of them, and the device record's ~95
 // float splits are spread over all; the rest every lane does alike. (One thread per design, which
-// also built the prism twice: 330 us for 512 designs.)
+// also built the prism twice: build and setup of 512 designs took 356 us, now 76.)
 constexpr uint32_t kBuildLanes = 8;
 constexpr uint32_t kBuildPerWarp = 32 / kBuildLanes;
 struct BuildScratch {
@@ -351,7 +351,10 @@ constexpr size_t table_smem_bytes(uint32_t buckets, uint32_t R) { return 4u * (s
 // a scatter), and each bucket's few are put in order by one thread. The points of a seed are
 // spread evenly (the R1 sequence: at most three share a bucket); the caller's own may not be,
 // and a bucket of more than kTableBucket leaves the table to the host. Keys are integers (a
-// seed's points as 64-bit fractions: no FP64 instruction).
+// seed's points as 64-bit fractions: no FP64 instruction). Latency bounds it: one block, ~10 us for
+// 8192 points (the host's sort and f64 quantiles: 400 us; a call on 3001 own points 238 -> 102 us).
+// That is why a size's order is kept from its second use on: a seed only turns it, and a call with
+// a fresh seed, 128 x 8192 rays, takes 51 us with it, 61 sorted anew, 285 by the host's tables.
 __global__ void __launch_bounds__(kTableThreads) table_sort_kernel(const LaunchArgs a)
 {
     stamp_start(a, STAMP_SORT);
@@ -435,7 +438,8 @@ __global__ void __launch_bounds__(kTableThreads) table_sort_kernel(const LaunchA
 // One thread per sorted position: its z in f64 (the host's own operations but for CUDA's log),
 // split into floats, and the ray's rank. blockIdx.y is the table. A warp's f64 instruction
 // takes its scheduler ~64 cycles, so the positions are spread two warps to a block; with a
-// known order this kernel is all a new seed costs, beside the setup's face loop.
+// known order this kernel is all a new seed costs, beside the setup's face loop (FP64
+// issue bounds it).
 __global__ void __launch_bounds__(64) table_z_kernel(const LaunchArgs a)
 {
     stamp_start(a, STAMP_Z);
@@ -1874,7 +1878,9 @@ __device__ __noinline__ int adaptive_row_redo(const LaunchArgs &a, unsigned long
 }
 
 // Passes with fewer rows than adaptive1_kernel's: one row per block (rows of designs without
-// pieces are adaptive_kernel's).
+// pieces are adaptive_kernel's). The chain of a row bounds it: up to 256 rounds are binned at once
+// by all warps and then decided, instead of 16 rounds per three barriers: a call of 128 rows x up
+// to 8192 rays 101 -> 70 us, one whose rows are redone 90 -> 79.
 __global__ void __launch_bounds__(32 * kMaxAdaptWarps, 2) adaptive_block_kernel(const LaunchArgs a)
 {
     extern __shared__ __align__(16) unsigned long long adapt_smem[];
@@ -1932,7 +1938,9 @@ __global__ void __launch_bounds__(32, CPD_ADAPT1_MIN_BLOCKS) adaptive1_kernel(co
 }
 
 // The same for passes of designs with certified pieces, or some of them (a kernel of its own:
-// with the general form out of line, rows without pieces take 9% longer here).
+// with the general form out of line, rows without pieces take 9% longer here). Issue and the rows'
+// states in shared memory bound it: at 2.6 KB a row 32 rows per SM leave the L1 enough (7.7 KB:
+// 2.1 ms). 256 designs x 128 rows x up to 8192 rays: 2.7 ms ray by ray, 1.15 here.
 __global__ void __launch_bounds__(32, CPD_ADAPT1_MIN_BLOCKS) adaptive1_pieces_kernel(const LaunchArgs a)
 {
     extern __shared__ __align__(16) unsigned long long adapt_smem[];
@@ -2346,6 +2354,8 @@ __global__ void __launch_bounds__(kEntropyThreads, 4) entropy_block_kernel(const
 
 // ------------------------------------------------------------------ rows by certified pieces
 
+// 20 warps per SM without spills: 104 registers (16 warps) 5.85 ms, 96 5.45, 80 (24 warps, spills)
+// 6.3, 128 6.2 on the 1024-design pass.
 #ifndef CPD_ROWS_MAXNREG
 #define CPD_ROWS_MAXNREG 96
 #endif
@@ -2407,6 +2417,14 @@ __device__ __forceinline__ void team_sync(uint32_t team, uint32_t T)
 //     design's.
 // Outcomes, flags and sums are those of trace_kernel, retrace_kernel and the entropy kernels,
 // integer for integer.
+//
+// Issue bounds it (2.3 M rows of 1024 rays: 1680 warp instructions a row at 60% of the slots, the
+// ALU pipe at 51%): 20 warps per SM, an edge's dependent bisection steps, and code the size of the
+// instruction cache. 1024 designs, those rows: 10.8 ms trace and 0.97 entropy by the ray-by-ray
+// kernels, 5.45 ms here; 512 designs x 128 rows x 8192 rays 2.33 -> 0.41 ms. (The steps' code
+// inlined where their lists fill: 6.5 ms. One row's pieces through a histogram in memory and
+// separate re-trace and entropy kernels: 6.3 ms. Edges 3.8 of 14 parts of a warp's time, rays of
+// short pieces 3.6, pieces 2.8, entropy 1.5, re-trace 1.1.)
 //
 // HEAVY: the rows that the setup listed as having many rays for the float-float trace, each by a
 // whole block, ahead of the groups. A warp takes 1.7 us per 32 such rays, and a pass waits for its
@@ -3051,7 +3069,9 @@ __global__ void __launch_bounds__(kTpRays) tp_adaptive_kernel(const DevDesign *_
 //    (k t / n)^2 c (n - c) / n + t^2 (n - k)^2 / (n (n + 1)). In FP32, summed exactly, that is
 //    within 2e-6 of the f64 recurrence; a test within kTpMargin leaves the wavelength to a replay
 //    in full (21 instructions) from the start.
-// A bin that ran past the stop is replayed from the chunk's start.
+// A bin that ran past the stop is replayed from the chunk's start. The longest bin's replay bounds
+// it now. 100 wavelengths x up to 16384 rays, device: 119 -> 56 us where they stop early, 1223 -> 425
+// and 2312 -> 761 where some run all rays (every update in full: 641 and 1166).
 constexpr uint32_t kTpList = 1024;
 
 // Per wavelength, by two warps of a block: the setup in float-float, and the transmittance of its

@@ -93,8 +93,9 @@ typedef struct cpd_fitness {
     double max_sem;         /* max over bins of the SEM of p(d|lambda) across wavelengths */
     uint64_t rays;          /* rays evaluated */
     uint64_t hits;          /* rays that reached a detector bin */
-    uint64_t retraced;      /* rays re-traced in exact f64 (guard band) */
-    uint64_t fast_rays;     /* rays evaluated by the FP32 fast path (exit face + detector) */
+    uint64_t retraced;      /* guard-band rays, re-traced in float-float (exact f64 in CPD_TRACE_FP64) */
+    uint64_t fast_rays;     /* the other rays in reach: decided by the FP32 fast path or, coated designs, as
+                               it decides them by certified pieces */
     uint32_t wavelengths;   /* wavelength rows accumulated */
     int32_t status;         /* CPD_OK or CPD_NOT_CONVERGED */
 } cpd_fitness;
@@ -295,12 +296,12 @@ int cpd_fitness_gpu_batch_params(cpd_context *ctx, const cpd_spectrometer_params
                                  uint32_t trace_mode, cpd_fitness *outs);
 
 /* cpd_design_build_batch on the GPU: the same records and status codes (up to the last-bit
- * differences of CUDA's sin/cos), one thread per design. */
+ * differences of CUDA's sin/cos), eight lanes per design. */
 int cpd_design_build_device(cpd_context *ctx, const cpd_spectrometer_params *params, uint32_t n,
                             double acceptance, cpd_design *out, int32_t *status);
 
-/* Launch-shape tuning of the batched/plain kernels (ray tile = rays per lane per
- * work item, warps per CTA). 0 leaves a value unchanged. */
+/* Launch-shape tuning of the batched/plain ray-by-ray trace (ray tile = rays per lane per
+ * work item, warps per CTA): uncoated designs and the FP32 study mode. 0 leaves a value unchanged. */
 int cpd_set_launch_shape(cpd_context *ctx, uint32_t ray_tile, uint32_t warps_per_cta);
 int cpd_get_launch_shape(cpd_context *ctx, uint32_t *ray_tile, uint32_t *warps_per_cta);
 
@@ -310,7 +311,8 @@ int cpd_get_launch_shape(cpd_context *ctx, uint32_t *ray_tile, uint32_t *warps_p
  * the resident warps, and warps per CTA in {2, 4, 8} (captured graph, minimum of two
  * timed passes each), sets the fastest on the context and remembers it for the batch's
  * class: trace mode and the binary orders of magnitude of its design count, wavelength
- * rows, rays and widest detector. Results do not depend on the shape. Fixed-N passes
+ * rows, rays and widest detector. Results do not depend on the shape (coated designs do not use
+ * it: a batch of them is timed at one shape). Fixed-N passes
  * only (a trace mode without CPD_SAMPLING_ADAPTIVE). */
 int cpd_autotune_batch(cpd_context *ctx, const cpd_design *designs, const cpd_batch_item *items,
                        uint32_t n, uint32_t trace_mode, uint32_t *ray_tile, uint32_t *warps_per_cta,
