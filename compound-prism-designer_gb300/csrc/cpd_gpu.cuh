@@ -157,6 +157,7 @@ struct LaunchArgs {
     DesignOut *out;       // results (mapped host memory in the context's passes)
     Control *ctl;
     HostStatus *status;   // optional (mapped host memory)
+    uint32_t max_rounds;  // adaptive passes: rounds of the longest table (the blocks' hit counts)
     uint32_t stamp;       // the kernel that writes status->t0 (the finalize writes t1); STAMP_NONE: none
     uint32_t clear_acc;   // the setup kernel zeroes S1, S2 (acc_cells) and acc (njobs) first
     uint64_t acc_cells;

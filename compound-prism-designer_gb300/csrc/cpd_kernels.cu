@@ -1666,10 +1666,11 @@ struct AdaptBlock {
     uint32_t unsure[kAdaptRounds / 32];
     uint4 odd[kAdaptOdd];  // hits of the float-float trace: round, bin, what they add beside tfast
 };
-// per bin: ox, samples and hits so far, then the counts
-constexpr size_t adapt_block_smem_bytes(uint32_t B)
+// per bin: ox, samples and hits so far, then the counts (of up to `rounds` rounds)
+constexpr size_t adapt_block_smem_bytes(uint32_t B, uint32_t rounds = kAdaptRounds)
 {
-    return sizeof(AdaptBlock) + 16u * (size_t)B + (size_t)adapt_rounds(B) * adapt_stride(B);
+    return sizeof(AdaptBlock) + 16u * (size_t)B +
+           (size_t)(rounds < adapt_rounds(B) ? rounds : adapt_rounds(B)) * adapt_stride(B);
 }
 
 // One wavelength row under adaptive sampling by one block, for a design with certified pieces
@@ -3810,8 +3811,13 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
                 launches++;
             } else {
                 if (a.adapt_pieces) {
-                    launch_k(adaptive_block_kernel, (unsigned)a.total_rows, 32 * kMaxAdaptWarps,
-                             adapt_block_smem_bytes(maxB), stream, pdl, a);
+                    // 2 to 7 rows per SM: 8 warps, four such blocks per SM; 4 warps where more rows
+                    // than that have few rounds. Calls, 16 / 8 / 4 warps: 472 x 602 rays 65 / 57 /
+                    // 62 us, 472 x 4096 97 / 90 / 110, 1000 x 8192 174 / 162 / 193, 700 x 602
+                    // 60 / 55 / 50, 1200 x 1024 110 / 94 / 88
+                    const uint32_t kb = kw == kMaxAdaptWarps ? kw : per_sm >= 4 && a.max_rounds <= 32u ? 4u : 8u;
+                    launch_k(adaptive_block_kernel, (unsigned)a.total_rows, 32 * kb,
+                             adapt_block_smem_bytes(maxB, a.max_rounds), stream, pdl, a);
                     launches++;
                 }
                 if (a.adapt_pieces != 1u) {

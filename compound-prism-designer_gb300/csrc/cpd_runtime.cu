@@ -652,6 +652,7 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     if (adaptive && !all_exact) {
         // (a device build decides in its record)
         uint32_t with = 0, maybe = 0;
+        for (const PassDesign &p : ds) a.max_rounds = std::max(a.max_rounds, (p.R + kRoundRays - 1u) / kRoundRays);
         for (const PassDesign &p : ds) {
             with += p.dev && p.dev->fc.pieces;
             maybe += p.params && p.params->ar_coated;
