@@ -1780,13 +1780,17 @@ __device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t
             const uint32_t len = (nr + np - 1u) / np, qa = min(p * len, nr), qb = min(qa + len, nr);
             const bool act = b < B;
             uint32_t n = 0u, h = 0u;
-            for (uint32_t q = qa; q < qb && act; q++) {
-                const uint32_t c = counts[q * stride + b];
-                if (c) n += min(kRoundRays, R - (r0 + q) * kRoundRays);
-                h += c;
+            if (np > 1u) {
+                // this stretch's share, for the stretches after it (one stretch, every thread a bin of its
+                // own: nothing to pass on; 1200 rows x 1024 rays in 236 bins 57 -> 55 us)
+                for (uint32_t q = qa; q < qb && act; q++) {
+                    const uint32_t c = counts[q * stride + b];
+                    if (c) n += min(kRoundRays, R - (r0 + q) * kRoundRays);
+                    h += c;
+                }
+                S.part[tid] = make_uint2(n, h);
+                __syncthreads();
             }
-            S.part[tid] = make_uint2(n, h);
-            __syncthreads();
             if (act) {
                 const uint2 v = base[b];
                 n = v.x;
@@ -1881,7 +1885,9 @@ __device__ __noinline__ int adaptive_row_redo(const LaunchArgs &a, unsigned long
 // Passes with fewer rows than adaptive1_kernel's: one row per block (rows of designs without
 // pieces are adaptive_kernel's). The chain of a row bounds it: up to 256 rounds are binned at once
 // by all warps and then decided, instead of 16 rounds per three barriers: a call of 128 rows x up
-// to 8192 rays 101 -> 70 us, one whose rows are redone 90 -> 79.
+// to 8192 rays 101 -> 70 us, one whose rows are redone 90 -> 79. With 200 bins and more most rounds
+// have a ray too close to an edge, and its fast_ray costs the round as much as 32: such rows are no
+// faster than ray by ray (900 rows x 2048 rays: 64 bins 53 -> 47 us, 200 bins 63 -> 79).
 __global__ void __launch_bounds__(32 * kMaxAdaptWarps, 2) adaptive_block_kernel(const LaunchArgs a)
 {
     extern __shared__ __align__(16) unsigned long long adapt_smem[];
