@@ -1805,6 +1805,9 @@ __device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t
                     if (!c) continue;
                     n += min(kRoundRays, R - (r0 + q) * kRoundRays);
                     h += c;
+                    // with a thread per bin, a bin that failed has often settled the round already
+                    // (1200 rows x 1024 rays in 236 bins: 55 -> 49 us; with stretches, no gain)
+                    if (np == 1u && *(volatile uint8_t *)&S.test[q]) continue;
                     int verdict = sem_quick_equal(n, h, se);
                     if (verdict < 0) verdict = sem_test(n, h, (uint64_t)h * tq, (uint64_t)h * tq * tq, delta);
                     if (verdict == SEM_FAIL) S.test[q] = 1u;  // a failed bin settles the round
@@ -1885,9 +1888,9 @@ __device__ __noinline__ int adaptive_row_redo(const LaunchArgs &a, unsigned long
 // Passes with fewer rows than adaptive1_kernel's: one row per block (rows of designs without
 // pieces are adaptive_kernel's). The chain of a row bounds it: up to 256 rounds are binned at once
 // by all warps and then decided, instead of 16 rounds per three barriers: a call of 128 rows x up
-// to 8192 rays 101 -> 70 us, one whose rows are redone 90 -> 79. With 200 bins and more most rounds
-// have a ray too close to an edge, and its fast_ray costs the round as much as 32: such rows are no
-// faster than ray by ray (900 rows x 2048 rays: 64 bins 53 -> 47 us, 200 bins 63 -> 79).
+// to 8192 rays 101 -> 70 us, one whose rows are redone 90 -> 79. The tests of step 2 run for 32
+// bins at a time whether one or all were hit: with 64 bins 900 rows x 2048 rays take 47 us (53 ray
+// by ray), with 200, 75 (63).
 __global__ void __launch_bounds__(32 * kMaxAdaptWarps, 2) adaptive_block_kernel(const LaunchArgs a)
 {
     extern __shared__ __align__(16) unsigned long long adapt_smem[];
