@@ -710,9 +710,9 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
         a.build_acceptance = ds[0].acceptance;
     }
 
-    // The device work of a pass, captured once per signature and replayed.
-    // The whole pass -- input upload, accumulator clears, kernels, read-back, and the two
-    // timing events around the kernels -- is one graph, captured once per signature.
+    // The whole pass -- input upload, the kernels (which clear the accumulators and write the
+    // results into mapped host memory) and, where it is timed, the two events around them -- is
+    // one graph, captured once per signature and replayed.
     // The design constants of a single-design pass are not part of the key: the cached
     // graph's trace node gets them per call.
     std::vector<uint8_t> key(sizeof(a) + 9 * sizeof(uint64_t));
