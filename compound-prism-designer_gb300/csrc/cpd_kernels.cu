@@ -1649,14 +1649,6 @@ __device__ __forceinline__ int adaptive_row1_pieces(const LaunchArgs &a, uint64_
 #endif
 // ------------------------------------------------------------------ adaptive sampling, few rows
 
-constexpr uint32_t kAdaptRounds = 256;       // rounds decided at once, and
-constexpr uint32_t kAdaptCounts = 64u * 1024u;  // the bytes of their hit counts
-// Counts of one round in bytes, and rounds per group, for a B-bin detector.
-__host__ __device__ constexpr uint32_t adapt_stride(uint32_t B) { return (B + 3u) & ~3u; }
-__host__ __device__ constexpr uint32_t adapt_rounds(uint32_t B)
-{
-    return kAdaptCounts / adapt_stride(B) < kAdaptRounds ? kAdaptCounts / adapt_stride(B) & ~15u : kAdaptRounds;
-}
 constexpr uint32_t kAdaptOdd = 128;  // such hits listed per group of rounds (more: the general exact path)
 struct AdaptBlock {
     Adapt1Pieces w;
@@ -1666,11 +1658,10 @@ struct AdaptBlock {
     uint32_t unsure[kAdaptRounds / 32];
     uint4 odd[kAdaptOdd];  // hits of the float-float trace: round, bin, what they add beside tfast
 };
-// per bin: ox, samples and hits so far, then the counts (of up to `rounds` rounds)
-constexpr size_t adapt_block_smem_bytes(uint32_t B, uint32_t rounds = kAdaptRounds)
+// then per bin: ox, samples and hits so far, and the counts (adapt_arrays_bytes)
+constexpr size_t adapt_block_smem_bytes(uint32_t max_B, uint32_t max_rounds = kAdaptRounds)
 {
-    return sizeof(AdaptBlock) + 16u * (size_t)B +
-           (size_t)(rounds < adapt_rounds(B) ? rounds : adapt_rounds(B)) * adapt_stride(B);
+    return sizeof(AdaptBlock) + adapt_arrays_bytes(max_B, max_rounds);
 }
 
 // One wavelength row under adaptive sampling by one block, for a design with certified pieces
@@ -1695,7 +1686,7 @@ __device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t
     unsigned long long *ox = reinterpret_cast<unsigned long long *>(&S + 1);
     uint2 *base = reinterpret_cast<uint2 *>(ox + B);
     uint8_t *counts = reinterpret_cast<uint8_t *>(base + B);
-    const uint32_t stride = adapt_stride(B), C = adapt_rounds(B);
+    const uint32_t stride = adapt_stride(B), C = adapt_rounds(B, adapt_arrays_bytes(a.max_B, a.max_rounds));
     const LamDF &E = a.lx[row];
     if (tid < sizeof(LamParams) / 4)
         reinterpret_cast<uint32_t *>(&w.P)[tid] = reinterpret_cast<const uint32_t *>(a.lp + row)[tid];

@@ -591,6 +591,25 @@ CPD_HD uint64_t rescale_cell(uint64_t s1, uint32_t R, uint32_t count)
     return (uint64_t)(((u128)s1 * R + count / 2u) / count);
 }
 
+// A block that decides many rounds of a row at once (adaptive_block_kernel) keeps, behind its fixed
+// part, 16 bytes per bin and the hit counts of those rounds, a byte per round and bin. Passes size
+// them by their widest detector and longest table:
+constexpr uint32_t kAdaptRounds = 256;          // most rounds decided at once, and
+constexpr uint32_t kAdaptCounts = 64u * 1024u;  // the bytes of their hit counts
+CPD_HDN constexpr uint32_t adapt_stride(uint32_t B) { return (B + 3u) & ~3u; }
+CPD_HDN constexpr uint32_t adapt_arrays_bytes(uint32_t max_B, uint32_t max_rounds)
+{
+    const uint32_t fit = kAdaptCounts / adapt_stride(max_B), most = fit < kAdaptRounds ? fit & ~15u : kAdaptRounds;
+    return 16u * max_B + (max_rounds < most ? max_rounds : most) * adapt_stride(max_B);
+}
+// The rounds that a B-bin row of such a pass decides at once: those whose counts lie within the
+// pass's bytes (narrower rows have room for other numbers of rounds, not always for kAdaptCounts).
+CPD_HDN constexpr uint32_t adapt_rounds(uint32_t B, uint32_t bytes)
+{
+    const uint32_t fit = (bytes - 16u * B) / adapt_stride(B);
+    return fit < kAdaptRounds ? fit : kAdaptRounds;
+}
+
 // Splits an f64 into f32 hi + lo parts (hi + lo == v to about 2^-48 relative).
 CPD_HD void split_f32(double v, float &hi, float &lo)
 {
