@@ -22,6 +22,7 @@
 
 #include "cpd_gpu.cuh"
 #include "cpd_host.h"
+#include "cpd_orders.h"
 
 namespace cpd {
 namespace {
@@ -97,8 +98,6 @@ constexpr uint32_t kSamplingBits = CPD_SAMPLING_ADAPTIVE | CPD_SAMPLING_EXACT;
 // Most rows of a pass whose trace takes equal shares of span slots: every warp scans the
 // blocks' spans (32 per step) to find its share.
 constexpr uint64_t kBalancedMaxRows = 16384;
-// Sizes whose point order a context keeps on the device (at most 64 KiB each).
-constexpr size_t kMaxOrders = 64;
 
 // The kernel node of `fn` in a captured graph (nullptr if none).
 cudaGraphNode_t find_kernel_node(cudaGraph_t g, const void *fn)
@@ -216,14 +215,7 @@ struct cpd_context {
     bool use_graphs = true;
     bool autotune = false;
     std::map<RayKey, RayTablePtr> ray_cache;
-    // the order of the sequence's first R points without a seed, per size R (see TableJob): made
-    // when a size comes a second time, kept until the context ends, for kMaxOrders sizes at most
-    struct Order {
-        uint32_t uses = 0;
-        uint32_t *dev = nullptr;
-        std::vector<uint64_t> keys;  // the sorted points, in 2^-64
-    };
-    std::map<uint32_t, Order> orders;
+    PointOrders orders;
     std::set<RayKey> host_only;  // tables that a pass could not make on the device
     std::map<RayKey, std::shared_ptr<const std::vector<double>>> lam_cache;  // wavelength u-points per (seed, W)
     // launch shape picked by the autotuner per class of batch
@@ -323,46 +315,29 @@ bool device_table(cpd_context *ctx, const PassDesign &p, uint32_t mode)
     return in;
 }
 
-// The device's order of the sequence's first R points and, for a seed (in 2^-64), how far the
-// seed turns it; nullptr when the context does not keep this size (yet). The addresses stay
-// valid for the context's life, so passes in flight on any stream may read them.
-const uint32_t *point_order(cpd_context *ctx, uint32_t R, uint64_t seed_fixed, uint32_t &rot)
+// PointOrders' calls, on a slot's stream.
+struct OrderDevice {
+    cudaStream_t stream;
+    uint32_t *alloc(uint32_t n)
+    {
+        uint32_t *p = nullptr;
+        if (cudaMalloc(&p, sizeof(uint32_t) * n) == cudaSuccess) return p;
+        cudaGetLastError();
+        return nullptr;
+    }
+    bool upload(uint32_t *dst, const uint32_t *src, uint32_t n)
+    {
+        return cudaMemcpyAsync(dst, src, sizeof(uint32_t) * n, cudaMemcpyHostToDevice, stream) == cudaSuccess;
+    }
+    bool wait() { return cudaStreamSynchronize(stream) == cudaSuccess; }
+    void free(uint32_t *p) { cudaFree(p); }
+};
+
+const uint32_t *point_order(cpd_context *ctx, cudaStream_t stream, uint32_t R, uint64_t seed_fixed, uint32_t &rot)
 {
     std::lock_guard<std::mutex> lk(ctx->cache_mu);
-    auto it = ctx->orders.find(R);
-    if (it == ctx->orders.end()) {
-        if (ctx->orders.size() >= kMaxOrders) return nullptr;
-        it = ctx->orders.emplace(R, cpd_context::Order()).first;
-    }
-    cpd_context::Order &o = it->second;
-    if (!o.dev) {
-        if (++o.uses < 2u) return nullptr;
-        const uint64_t alpha = (uint64_t)(kAlpha * 18446744073709551616.0);
-        std::vector<std::pair<uint64_t, uint32_t>> kj(R);
-        for (uint32_t j = 0; j < R; j++) kj[j] = {alpha * (j + 1u), j};
-        std::sort(kj.begin(), kj.end());
-        std::vector<uint32_t> order(R);
-        std::vector<uint64_t> keys(R);
-        for (uint32_t i = 0; i < R; i++) {
-            keys[i] = kj[i].first;
-            order[i] = kj[i].second;
-        }
-        uint32_t *dev = nullptr;
-        if (cudaMalloc(&dev, sizeof(uint32_t) * R) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        if (cudaMemcpy(dev, order.data(), sizeof(uint32_t) * R, cudaMemcpyHostToDevice) != cudaSuccess) {
-            cudaFree(dev);
-            return nullptr;
-        }
-        o.keys.swap(keys);
-        o.dev = dev;
-    }
-    // the points that the seed carries past 1 come first
-    rot = seed_fixed ? (uint32_t)(std::lower_bound(o.keys.begin(), o.keys.end(), 0ull - seed_fixed) - o.keys.begin()) : 0u;
-    if (rot == R) rot = 0u;
-    return o.dev;
+    OrderDevice dev{stream};
+    return ctx->orders.get(dev, R, seed_fixed, rot);
 }
 
 // The host's table for a design's points.
@@ -492,7 +467,7 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
                 t.ray_off = ray;
                 t.rank_off = rnk;
                 t.R = p.R;
-                if (p.seeded) t.order = point_order(ctx, p.R, t.seed_fixed, t.rot);
+                if (p.seeded) t.order = point_order(ctx, S.stream, p.R, t.seed_fixed, t.rot);
                 else upts += p.R;
                 table_max = std::max(table_max, p.R);
                 tabs.push_back(t);
@@ -1231,7 +1206,9 @@ int cpd_context_create(int device, cpd_context **out)
     std::vector<float> tab(4 * ff::kLogTable);
     ff::make_log_table(tab.data());
     if (configure_kernels() != cudaSuccess || ctx->main.create() != cudaSuccess || ctx->logtab.ensure(sizeof(float) * tab.size()) != cudaSuccess ||
-        cudaMemcpy(ctx->logtab.p, tab.data(), sizeof(float) * tab.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaMemcpyAsync(ctx->logtab.p, tab.data(), sizeof(float) * tab.size(), cudaMemcpyHostToDevice, ctx->main.stream) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(ctx->main.stream) != cudaSuccess) {  // every slot's stream reads it
         ctx->main.destroy();
         ctx->logtab.release();
         delete ctx;
@@ -1246,8 +1223,10 @@ void cpd_context_destroy(cpd_context *ctx)
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     ctx->main.destroy();
-    for (auto &o : ctx->orders)
-        if (o.second.dev) cudaFree(o.second.dev);
+    {
+        OrderDevice dev{nullptr};
+        ctx->orders.release(dev);
+    }
     for (DevBuf *b : {&ctx->tp_design, &ctx->tp_lam, &ctx->tp_z, &ctx->tp_out, &ctx->tp_rays, &ctx->tp_tab, &ctx->tp_lp,
                       &ctx->tp_t64})
         b->release();
