@@ -10,6 +10,7 @@
 #include <chrono>
 #include <cmath>
 #include <condition_variable>
+#include <cstddef>
 #include <cstring>
 #include <deque>
 #include <map>
@@ -843,16 +844,37 @@ bool valid_item(const cpd_batch_item &it)
     return it.max_n >= 1 && it.max_n <= CPD_MAX_WAVELENGTHS && it.max_eval >= 1 && it.max_eval <= CPD_MAX_RAYS;
 }
 
+// Takes back what a pass that is run again has counted: the ray counters of its designs return to
+// those of the results before it (its trace adds to them as it goes; every other sum of such a pass
+// is left out by the entropy and finalize kernels).
+int restore_counters(PassSlot &S, const std::vector<DesignOut> &before)
+{
+    static_assert(offsetof(DesignAcc, hits) + 3 * sizeof(DesignAcc::hits) == sizeof(DesignAcc), "the counters end the record");
+    for (size_t i = 0; i < before.size(); i++) {
+        DesignAcc c{};
+        c.hits[0] = before[i].hits;
+        c.retraced[0] = before[i].retraced;
+        c.fast[0] = before[i].fast;
+        CPD_TRY(cudaMemcpyAsync(S.acc.as<DesignAcc>()[i].hits, c.hits, 3 * sizeof(c.hits), cudaMemcpyHostToDevice, S.stream));
+    }
+    CPD_TRY(cudaStreamSynchronize(S.stream));
+    return CPD_OK;
+}
+
 // Runs one pass on `S` to completion, growing the re-trace queue and re-running the
-// pass if it overflowed. A pass that overflowed leaves the persistent accumulators
-// untouched (the entropy kernel skips such a pass), so the re-run is exact.
+// pass if it overflowed, or with the host's tables if the device could not make one. Such a
+// pass leaves the persistent accumulators as they were: the entropy kernel skips it, and the
+// ray counters are restored (unless the re-run clears them: fresh).
 int run_pass_checked(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &pds, uint32_t mode, bool fresh,
                      double *p_out, PassResult &res, bool use_graph)
 {
     std::vector<PassDesign> by_host;  // the same designs with the host's tables
+    std::vector<DesignOut> before;
+    if (!fresh) before.assign(S.h_outs.as<DesignOut>(), S.h_outs.as<DesignOut>() + pds.size());
     for (int attempt = 0; attempt < 7; attempt++) {
         const std::vector<PassDesign> &ds = by_host.empty() ? pds : by_host;
-        int e = pass_issue(ctx, S, ds, mode, fresh, p_out, use_graph, ctx->profiling);
+        int e = attempt ? restore_counters(S, before) : (int)CPD_OK;
+        if (!e) e = pass_issue(ctx, S, ds, mode, fresh, p_out, use_graph, ctx->profiling);
         if (!e) e = pass_finish(S, res);
         if (e) {
             S.hist_dirty = true;
