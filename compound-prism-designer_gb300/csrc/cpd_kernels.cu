@@ -1649,12 +1649,12 @@ __device__ __forceinline__ int adaptive_row1_pieces(const LaunchArgs &a, uint64_
 #endif
 // ------------------------------------------------------------------ adaptive sampling, few rows
 
-constexpr uint32_t kAdaptOdd = 128;  // such hits listed per group of rounds (more: the general exact path)
+constexpr uint32_t kAdaptOdd = 128;  // such hits listed per group of rounds (more: traced again once the stop is known)
 struct AdaptBlock {
     Adapt1Pieces w;
     uint2 part[32 * kMaxAdaptWarps];   // samples and hits of one bin over one stretch of rounds
     uint8_t hit[kAdaptRounds], test[kAdaptRounds], df[kAdaptRounds];  // test: 1 a bin failed
-    uint32_t other, ndf, nodd, pad;
+    uint32_t other, ndf, nodd, pad;    // other: the row's first round with a hit for adaptive_exact_kernel
     uint32_t unsure[kAdaptRounds / 32];
     uint4 odd[kAdaptOdd];  // hits of the float-float trace: round, bin, what they add beside tfast
 };
@@ -1662,6 +1662,33 @@ struct AdaptBlock {
 constexpr size_t adapt_block_smem_bytes(uint32_t max_B, uint32_t max_rounds = kAdaptRounds)
 {
     return sizeof(AdaptBlock) + adapt_arrays_bytes(max_B, max_rounds);
+}
+
+// What the float-float hits of rounds [r0, r0 + taken) add beside tfast, where there are more of them
+// than the list holds: their rays traced again (out of line: a row with its rays on a bin's edge).
+__device__ __noinline__ void adapt_odd_again(const LaunchArgs &a, const AdaptBlock &S, uint64_t row, const DevDesign &D,
+                                             const DesignJob &J, unsigned long long *ox, uint32_t r0, uint32_t taken,
+                                             uint32_t tfast, uint32_t tfix)
+{
+    const Adapt1Pieces &w = S.w;
+    const uint32_t *rank = a.rank + J.rank_off;
+    const float2 *__restrict__ zt = reinterpret_cast<const float2 *>(a.z32) + J.ray_off;
+    const PieceConst K = piece_const(w.C);
+    const uint32_t lo = w.P.core_lo, hi = w.P.all_exact ? w.P.core_lo : w.P.core_hi, ks = piece_shift(hi - lo);
+    const uint32_t j1 = min((r0 + taken) * kRoundRays, J.R);
+    for (uint32_t j = r0 * kRoundRays + threadIdx.x; j < j1; j += blockDim.x) {
+        const uint32_t s = __ldg(rank + j);
+        if (s < w.P.band_lo || s >= w.P.band_hi) continue;
+        const float2 z = __ldg(zt + s);
+        const bool core = s >= lo && s < hi;
+        uint32_t bin = 0xffffffffu;
+        if (core && adapt_ray(w, K, J.B, s, lo, ks, z, bin) != RAY_FLAG) continue;
+        bin = 0xffffffffu;
+        bool used_df = false;
+        long long add = 0;
+        adapt_left<false>(a, D, w, a.lx[row], core, z, tfast, tfix, bin, used_df, add);
+        if (add) atomicAdd(ox + bin, (unsigned long long)add);
+    }
 }
 
 // One wavelength row under adaptive sampling by one block, for a design with certified pieces
@@ -1672,7 +1699,8 @@ constexpr size_t adapt_block_smem_bytes(uint32_t max_B, uint32_t max_rounds = kA
 // round that hit it; the row stops after the first round with a hit and no failed test. Three
 // barriers for 256 rounds instead of three for 16, and no round waits for the one before.
 // The rays of the float-float trace past the stop would leave their differences in ox, so those
-// are listed with their round and added at the end. Returns as adaptive_row1_pieces.
+// are listed with their round and added at the end. Returns as adaptive_row1_pieces: what lies past
+// the stop decides nothing.
 template <bool kExact>
 __device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t row, unsigned long long *smem)
 {
@@ -1696,7 +1724,10 @@ __device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t
         base[b] = make_uint2(0u, 0u);
         ox[b] = 0ull;
     }
-    if (tid == 0) S.other = S.ndf = S.nodd = 0u;
+    if (tid == 0) {
+        S.other = 0xffffffffu;
+        S.ndf = S.nodd = 0u;
+    }
     __syncthreads();
     const uint32_t *rank = a.rank + J.rank_off;
     const float2 *__restrict__ zt = reinterpret_cast<const float2 *>(a.z32) + J.ray_off;
@@ -1744,11 +1775,11 @@ __device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t
             }
             bool used_df = false;
             long long add = 0;
-            if (res == RAY_FLAG && !adapt_left<kExact>(a, D, w, E, core, z, tfast, tfix, bin, used_df, add)) S.other = 1u;
+            if (res == RAY_FLAG && !adapt_left<kExact>(a, D, w, E, core, z, tfast, tfix, bin, used_df, add))
+                atomicMin(&S.other, r0 + q);
             if (add) {
                 const uint32_t i = atomicAdd(&S.nodd, 1u);
                 if (i < kAdaptOdd) S.odd[i] = make_uint4(r0 + q, bin, (uint32_t)add, (uint32_t)(add >> 32));
-                else S.other = 1u;
             }
             if (kExact) used_df = s >= band_lo && s < band_hi;
             const uint32_t grp = __match_any_sync(0xffffffffu, bin);
@@ -1762,7 +1793,6 @@ __device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t
             }
         }
         __syncthreads();
-        if (S.other) return ROW_OTHER;
         // 2. the tests, up to nthr bins at a time
         for (uint32_t b0 = 0; b0 < B; b0 += nthr) {
             uint32_t width = 1u;
@@ -1817,8 +1847,9 @@ __device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t
                 break;
             }
         }
-        if (last < nr && (S.unsure[last >> 5] >> (last & 31u) & 1u)) return ROW_UNSURE;
         const uint32_t taken = last < nr ? last + 1u : nr;
+        if (S.other < r0 + taken) return ROW_OTHER;
+        if (last < nr && (S.unsure[last >> 5] >> (last & 31u) & 1u)) return ROW_UNSURE;
         // the states through it, and the float-float rays
         for (uint32_t b0 = 0; b0 < B; b0 += nthr) {
             uint32_t width = 1u;
@@ -1834,7 +1865,9 @@ __device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t
             if (n) atomicAdd(&base[b].x, n);
             if (h) atomicAdd(&base[b].y, h);
         }
-        for (uint32_t i = tid; i < S.nodd; i += nthr) {
+        const uint32_t nodd = S.nodd;
+        if (!kExact && nodd > kAdaptOdd) adapt_odd_again(a, S, row, D, J, ox, r0, taken, tfast, tfix);
+        for (uint32_t i = tid; i < nodd && nodd <= kAdaptOdd; i += nthr) {
             const uint4 o = S.odd[i];
             if (o.x < r0 + taken) atomicAdd(ox + o.y, (unsigned long long)o.w << 32 | o.z);
         }
