@@ -354,9 +354,10 @@ void launch_trace_pairs(const DevDesign *d, const double *lam_u, const double *z
 
 // The reference CPU estimator of p(d|lambda) (p_dets_l_wavelength, src/fitness.rs:5-69) for
 // n explicit wavelengths, one block each: out[n x B] and the rays each consumed. z64 holds
-// norminv of the reference's ray points in ray order (max_m of them).
+// norminv of the reference's ray points in ray order (max_m of them). left_only: the
+// wavelengths that launch_tp_pieces has left (rays_out 0).
 void launch_tp_adaptive(const DevDesign *d, uint32_t B, const double *lambdas, uint32_t n, const double *z64,
-                        uint32_t max_m, double *out, uint32_t *rays_out, cudaStream_t stream);
+                        uint32_t max_m, double *out, uint32_t *rays_out, bool left_only, cudaStream_t stream);
 
 // The same for a design with certified pieces, up to kTpMaxRays rays.
 constexpr uint32_t kTpMaxRays = 65536;  // rays of the sorted table and the tables of counts

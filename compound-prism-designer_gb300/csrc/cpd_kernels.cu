@@ -2993,8 +2993,9 @@ __device__ __forceinline__ void tp_next(TpWelford &w, double v)
 __global__ void __launch_bounds__(kTpRays) tp_adaptive_kernel(const DevDesign *__restrict__ dd,
                                                               const double *__restrict__ lambdas,
                                                               const double *__restrict__ z64, uint32_t max_m,
-                                                              double *out, uint32_t *rays_out)
+                                                              double *out, uint32_t *rays_out, bool left_only)
 {
+    if (left_only && rays_out[blockIdx.x]) return;  // tp_pieces_kernel has done it
     __shared__ __align__(16) DevDesign sD;
     __shared__ uint32_t key[kTpRays];   // (bin << 8) | ray within the round; ~0u: no hit
     __shared__ double tv[kTpRays];      // t of the round's ray i
@@ -3998,10 +3999,10 @@ void launch_trace_pairs(const DevDesign *d, const double *lam_u, const double *z
 }
 
 void launch_tp_adaptive(const DevDesign *d, uint32_t B, const double *lambdas, uint32_t n, const double *z64,
-                        uint32_t max_m, double *out, uint32_t *rays_out, cudaStream_t stream)
+                        uint32_t max_m, double *out, uint32_t *rays_out, bool left_only, cudaStream_t stream)
 {
     if (!n) return;
-    tp_adaptive_kernel<<<n, kTpRays, 3 * sizeof(double) * B, stream>>>(d, lambdas, z64, max_m, out, rays_out);
+    tp_adaptive_kernel<<<n, kTpRays, 3 * sizeof(double) * B, stream>>>(d, lambdas, z64, max_m, out, rays_out, left_only);
 }
 
 void launch_tp_pieces(const TpArgs &a, uint32_t B, cudaStream_t stream)

@@ -1628,7 +1628,7 @@ int cpd_transmission_probability_ex(cpd_context *ctx, const cpd_design *d, const
         launch_tp_pieces(a, D.B, s);
     } else {
         launch_tp_adaptive(dd, D.B, dl, n, ctx->tp_z.as<double>(), max_m, ctx->tp_out.as<double>(),
-                           ctx->tp_rays.as<uint32_t>(), s);
+                           ctx->tp_rays.as<uint32_t>(), false, s);
     }
     CPD_TRY(cudaGetLastError());
     CPD_TRY(cudaEventRecord(S.ev1, s));
@@ -1636,22 +1636,25 @@ int cpd_transmission_probability_ex(cpd_context *ctx, const cpd_design *d, const
     CPD_TRY(cudaMemcpyAsync(rays.data(), ctx->tp_rays.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s));
     CPD_TRY(cudaStreamSynchronize(s));
     S.launches = pieces ? 2 : 1;
-    // wavelengths with hits of more than one transmittance, by the general kernel
-    for (uint32_t i = 0; i < n; i++)
-        if (rays[i] == 0u) {
-            launch_tp_adaptive(dd, D.B, dl + i, 1, ctx->tp_z.as<double>(), max_m, ctx->tp_out.as<double>() + (size_t)i * D.B,
-                               ctx->tp_rays.as<uint32_t>() + i, s);
-            CPD_TRY(cudaGetLastError());
-            CPD_TRY(cudaMemcpyAsync(out + (size_t)i * D.B, ctx->tp_out.as<double>() + (size_t)i * D.B, sizeof(double) * D.B,
-                                    cudaMemcpyDeviceToHost, s));
-            CPD_TRY(cudaMemcpyAsync(&rays[i], ctx->tp_rays.as<uint32_t>() + i, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-            CPD_TRY(cudaStreamSynchronize(s));
-            S.launches++;
-        }
-    if (rays_out) std::memcpy(rays_out, rays.data(), sizeof(uint32_t) * n);
-    float ms = 0.f;
+    float ms = 0.f, left_ms = 0.f;
     cudaEventElapsedTime(&ms, S.ev0, S.ev1);
-    S.last_ms = ms;
+    // wavelengths with hits of more than one transmittance, by the general kernel (glass of an index
+    // near 1 behind a steep exit face; then often every wavelength, so all in one launch)
+    if (std::find(rays.begin(), rays.end(), 0u) != rays.end()) {
+        CPD_TRY(cudaEventRecord(S.ev0, s));
+        launch_tp_adaptive(dd, D.B, dl, n, ctx->tp_z.as<double>(), max_m, ctx->tp_out.as<double>(), ctx->tp_rays.as<uint32_t>(),
+                           true, s);
+        CPD_TRY(cudaGetLastError());
+        CPD_TRY(cudaEventRecord(S.ev1, s));
+        CPD_TRY(cudaMemcpyAsync(out, ctx->tp_out.p, out_bytes, cudaMemcpyDeviceToHost, s));
+        CPD_TRY(cudaMemcpyAsync(rays.data(), ctx->tp_rays.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s));
+        CPD_TRY(cudaStreamSynchronize(s));
+        cudaEventElapsedTime(&left_ms, S.ev0, S.ev1);
+        S.d2h += out_bytes + sizeof(uint32_t) * n;
+        S.launches++;
+    }
+    if (rays_out) std::memcpy(rays_out, rays.data(), sizeof(uint32_t) * n);
+    S.last_ms = ms + left_ms;
     S.h2d += in_bytes;
     S.d2h += out_bytes + sizeof(uint32_t) * n;
     return CPD_OK;
