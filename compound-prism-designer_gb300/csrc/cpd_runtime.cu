@@ -220,7 +220,7 @@ struct cpd_context {
     std::set<RayKey> host_only;  // tables that a pass could not make on the device
     std::map<RayKey, std::shared_ptr<const std::vector<double>>> lam_cache;  // wavelength u-points per (seed, W)
     // launch shape picked by the autotuner per class of batch
-    std::map<std::array<uint64_t, 5>, std::pair<uint32_t, uint32_t>> tune_cache;
+    std::map<std::array<uint64_t, 6>, std::pair<uint32_t, uint32_t>> tune_cache;
 };
 
 namespace {
@@ -897,9 +897,17 @@ int run_pass_checked(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign
     return CPD_NO_CAPACITY;
 }
 
-// The class of a batch for the launch-shape cache: trace mode and the binary orders of
-// magnitude of its design count, wavelength rows, rays and widest detector.
-std::array<uint64_t, 5> tune_class(const std::vector<PassDesign> &ds, uint32_t mode)
+// Whether every design of a batch goes through rows_kernel, which has no launch shape to tune.
+bool all_pieces(const std::vector<PassDesign> &ds, uint32_t mode)
+{
+    return mode == CPD_TRACE_HYBRID && std::all_of(ds.begin(), ds.end(), [](const PassDesign &p) {
+        return p.params ? p.params->ar_coated != 0 : p.dev->fc.pieces != 0;
+    });
+}
+
+// The class of a batch for the launch-shape cache: trace mode, whether it has a shape to tune, and
+// the binary orders of magnitude of its design count, wavelength rows, rays and widest detector.
+std::array<uint64_t, 6> tune_class(const std::vector<PassDesign> &ds, uint32_t mode)
 {
     uint64_t rows = 0, rays = 0, maxB = 0;
     for (const PassDesign &p : ds) {
@@ -912,7 +920,7 @@ std::array<uint64_t, 5> tune_class(const std::vector<PassDesign> &ds, uint32_t m
         while ((1ull << b) < v && b < 63) b++;
         return b;
     };
-    return {mode, lg(ds.size()), lg(rows), lg(rays), lg(maxB)};
+    return {mode, all_pieces(ds, mode), lg(ds.size()), lg(rows), lg(rays), lg(maxB)};
 }
 
 // The autotuner: times every (ray tile, warps per CTA) candidate on the batch itself
@@ -931,9 +939,7 @@ int tune_pass(cpd_context *ctx, const std::vector<PassDesign> &ds, uint32_t mode
     // Besides the powers of two: tiles that make the work items a whole number of rounds
     // of the resident warps (2..6 items per warp), so that the last round is not a tail.
     std::vector<std::pair<uint32_t, uint32_t>> cands;
-    const bool pieces = mode == CPD_TRACE_HYBRID && std::all_of(ds.begin(), ds.end(), [](const PassDesign &p) {
-        return p.params ? p.params->ar_coated != 0 : p.dev->fc.pieces != 0;
-    });
+    const bool pieces = all_pieces(ds, mode);
     if (pieces) cands.push_back({32u, 8u});  // no work items: the shape does not matter
     for (uint32_t w : kWarps) {
         if (pieces) break;
