@@ -940,7 +940,7 @@ int tune_pass(cpd_context *ctx, const std::vector<PassDesign> &ds, uint32_t mode
     // of the resident warps (2..6 items per warp), so that the last round is not a tail.
     std::vector<std::pair<uint32_t, uint32_t>> cands;
     const bool pieces = all_pieces(ds, mode);
-    if (pieces) cands.push_back({32u, 8u});  // no work items: the shape does not matter
+    if (pieces) cands.push_back({rt0, w0});  // no work items: the caller's shape stays
     for (uint32_t w : kWarps) {
         if (pieces) break;
         for (uint32_t rt : kTiles) cands.push_back({rt, w});

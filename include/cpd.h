@@ -312,8 +312,8 @@ int cpd_get_launch_shape(cpd_context *ctx, uint32_t *ray_tile, uint32_t *warps_p
  * timed passes each), sets the fastest on the context and remembers it for the batch's
  * class: trace mode, whether it has a design that uses the shape, and the binary orders of
  * magnitude of its design count, wavelength rows, rays and widest detector. Results do not depend
- * on the shape (coated designs do not use it: a batch of them is timed at one shape). Fixed-N passes
- * only (a trace mode without CPD_SAMPLING_ADAPTIVE). */
+ * on the shape (coated designs do not use it: a batch of them is timed at the context's shape,
+ * which stays). Fixed-N passes only (a trace mode without CPD_SAMPLING_ADAPTIVE). */
 int cpd_autotune_batch(cpd_context *ctx, const cpd_design *designs, const cpd_batch_item *items,
                        uint32_t n, uint32_t trace_mode, uint32_t *ray_tile, uint32_t *warps_per_cta,
                        double *best_ms);

@@ -31,3 +31,11 @@ def test_a_coated_batch_leaves_its_class_untuned(n):
     first, second = uploads(uncoated), uploads(uncoated)
     assert first > 20 * second  # the first call times the candidates, three passes each
     ctx.close()
+
+
+def test_a_coated_batch_keeps_the_callers_shape():
+    ctx = cpd.Context(0)
+    ctx.set_launch_shape(64, 4)
+    rt, w, ms = cpd.autotune_batch(_specs(True), max_n=200, max_eval=512, context=ctx)
+    assert (rt, w) == ctx.launch_shape() == (64, 4) and ms > 0
+    ctx.close()
