@@ -20,16 +20,17 @@ namespace cpd {
 constexpr size_t kMaxOrders = 64;
 
 // An order is made when its size comes a second time and kept until release: passes in flight on
-// any stream may read it. The caller serialises the calls.
+// any stream may read it. Sizes seen once give way to new ones. The caller serialises the calls.
 // Device: uint32_t *alloc(n); bool upload(dst, src, n), which may return before the device has the
 // data, and bool wait(), which does not; void free(p).
 class PointOrders {
     struct Order {
-        uint32_t uses = 0;
+        uint64_t since = 0;  // when the size came first
         uint32_t *dev = nullptr;
         std::vector<uint64_t> keys;  // the sorted points, in 2^-64
     };
     std::map<uint32_t, Order> orders;
+    uint64_t clock = 0;
 
 public:
     // The device's order of the sequence's first R points and, for a seed (in 2^-64), how far the
@@ -39,12 +40,18 @@ public:
     {
         auto it = orders.find(R);
         if (it == orders.end()) {
-            if (orders.size() >= kMaxOrders) return nullptr;
-            it = orders.emplace(R, Order()).first;
+            if (orders.size() >= kMaxOrders) {
+                auto old = orders.end();
+                for (auto i = orders.begin(); i != orders.end(); ++i)
+                    if (!i->second.dev && (old == orders.end() || i->second.since < old->second.since)) old = i;
+                if (old == orders.end()) return nullptr;
+                orders.erase(old);
+            }
+            orders[R].since = ++clock;
+            return nullptr;
         }
         Order &o = it->second;
         if (!o.dev) {
-            if (++o.uses < 2u) return nullptr;
             const uint64_t alpha = (uint64_t)(kAlpha * 18446744073709551616.0);
             std::vector<std::pair<uint64_t, uint32_t>> kj(R);
             for (uint32_t j = 0; j < R; j++) kj[j] = {alpha * (j + 1u), j};

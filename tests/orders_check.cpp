@@ -1,6 +1,8 @@
 // Host check of PointOrders (csrc/cpd_orders.h) on a device whose copies are carried out only when
 // they are waited for.
 // usage: orders_check early    <sizes>...       prints: given <orders handed out> early <before the device had them>
+//        orders_check steady <one-off sizes>   prints: given <calls of a steady size that got an order, of 3 after those>
+//                                                      kept <sizes kept when 100 come twice>
 //        orders_check sorted   <R> <seeds>...   prints: points <n> misplaced <not in ascending order of the seed's points>
 #include <cstdio>
 #include <cstdlib>
@@ -70,6 +72,20 @@ int main(int argc, char **argv)
         }
         orders.release(dev);
         std::printf("given %ld early %ld left %zu\n", given, early, dev.owned.size());
+    } else if (what == "steady" && argc > 2) {
+        const uint32_t n = (uint32_t)std::atoi(argv[2]);
+        uint32_t rot = 0;
+        long given = 0, kept = 0;
+        for (uint32_t i = 0; i < n; i++) orders.get(dev, 100u + i, 0, rot);
+        for (int call = 0; call < 3; call++) given += orders.get(dev, 50u, 0, rot) != nullptr;
+        for (int call = 0; call < 3; call++)
+            for (uint32_t i = 0; i < 100u; i++) {
+                orders.get(dev, 1000u + i, 0, rot);
+                orders.get(dev, 1000u + i, 0, rot);
+            }
+        kept = (long)dev.owned.size();
+        orders.release(dev);
+        std::printf("given %ld kept %ld\n", given, kept);
     } else if (what == "sorted" && argc > 2) {
         const uint32_t R = (uint32_t)std::atoi(argv[2]);
         long n = 0, misplaced = 0;

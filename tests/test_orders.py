@@ -33,6 +33,11 @@ def test_an_order_is_on_the_device_before_it_is_given_out(orders_bin):
     assert r == {"given": 12, "early": 0, "left": 0}
 
 
+@pytest.mark.parametrize("n", [0, 1, 63, 64, 65, 500])
+def test_sizes_seen_once_do_not_keep_a_steady_size_out(orders_bin, n):
+    assert _run(orders_bin, "steady", n) == {"given": 2, "kept": 64}
+
+
 @pytest.mark.parametrize("R", [1, 2, 33, 1000, 16384])
 def test_orders_sort_the_points_of_any_seed(orders_bin, R):
     seeds = [0.0, 0.5, 1e-17, 2.0 ** -53, 0.1234567, 0.381966, 0.9, 1.0 - 2.0 ** -53]
