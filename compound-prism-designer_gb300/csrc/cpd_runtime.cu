@@ -1073,9 +1073,9 @@ void srv_complete(cpd_server *sv, size_t i)
     std::lock_guard<std::mutex> lk(sv->mu);
     auto &work = sv->slot_work[i];
     if (!e && (res.overflow || res.bad_table)) e = CPD_NO_CAPACITY;  // re-queued below
-    if (e == CPD_NO_CAPACITY && S.qcap < (1u << 26)) {
-        // run the same designs again, with a larger re-trace queue or the host's tables
-        if (res.overflow) S.qcap *= 4;
+    if (e == CPD_NO_CAPACITY && (S.qcap < (1u << 26) || res.bad_table)) {
+        // run the same designs again, with a larger re-trace queue (up to a limit) or the host's tables
+        if (res.overflow && S.qcap < (1u << 26)) S.qcap *= 4;
         if (res.bad_table) {
             std::vector<std::pair<double, uint32_t>> seeds;
             for (const SrvWork &wk : work) {

@@ -60,3 +60,15 @@ def test_server_request_with_such_a_seed(adaptive):
             assert (int(o["hits"]), int(o["rays"]), float(o["info"])) == (f.hits, f.rays, f.info)
     sv.close()
     ctx.close()
+
+
+def test_server_whose_queue_is_at_its_limit():
+    # 17 M rays in f64 take the slot's queue to its largest size; such a seed is still served after it
+    (spec, _), = _designs(1)[:1]
+    ctx = cpd.Context(0)
+    with cpd.Server(slots=1, context=ctx) as sv:
+        sv.wait(sv.submit([spec], seeds=0.3, max_n=4096, max_eval=4200, mode=cpd.TRACE_FP64))
+        out = sv.wait(sv.submit([spec], seeds=ZERO, max_n=40, max_eval=300))[0]
+    f = spec.gpu_fitness_full([ZERO], max_n=40, max_eval=300)
+    assert (int(out["hits"][0]), float(out["info"][0])) == (f.hits, f.info)
+    ctx.close()
