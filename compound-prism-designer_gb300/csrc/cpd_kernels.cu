@@ -1005,7 +1005,7 @@ struct RoundSlot {
     uint32_t p[6][32];
     uint32_t df;       // ballot of the rays traced in float-float
     uint32_t nh;       // hits of the round
-    uint32_t verdict;  // 0 go on, 1 stop, 2 unsure
+    uint32_t verdict;  // 0 go on, 1 stop, 2 unsure, 3 a hit of another transmittance (kEqual)
     uint32_t pad;
 };
 static_assert(sizeof(RoundSlot) % 16 == 0, "bin states follow the slots 16-byte aligned");
@@ -1044,10 +1044,15 @@ __device__ __forceinline__ uint32_t lane_entry(const uint4 &w, uint32_t v)
 // the one-round-at-a-time order bit for bit.
 // kExact: every ray by the float-float trace and the exact test. Otherwise a row whose
 // stop decision the FP32 transmittances cannot settle (sem_test: SEM_UNSURE) leaves
-// nothing behind and returns true: the caller redoes it on the exact path. (In the
+// nothing behind and returns ROW_UNSURE: the caller redoes it on the exact path. (In the
 // verification mode every row is queued for adaptive_exact_kernel instead.)
-template <bool kExact>
-__device__ bool adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long long *smem, uint32_t KW,
+// kEqual: a design with certified pieces. Its rows have the arithmetic of adaptive_row1_pieces,
+// decision for decision (one transmittance, states of samples and hits alone, a row with a hit of
+// another transmittance up to its stop returned as ROW_OTHER), so that they come out the same here
+// and there; kExact then concerns the transmittance and the test.
+enum : int { ROW_DONE = 0, ROW_UNSURE = 1, ROW_OTHER = 2 };
+template <bool kExact, bool kEqual = false>
+__device__ int adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long long *smem, uint32_t KW,
                              uint32_t warp, uint32_t lane)
 {
     const uint32_t d = find_job<F_ROW>(a.jobs, a.njobs, row);
@@ -1063,7 +1068,7 @@ __device__ bool adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lo
             if (pos < a.qcap) a.queue[pos] = QEntry{d, k, 0u, 0u};
             else atomicOr(&a.ctl->overflow, kOverflowQueue);
         }
-        return false;
+        return ROW_DONE;
     }
     RoundSlot *slots = reinterpret_cast<RoundSlot *>(smem);
     RoundSlot &my = slots[warp];
@@ -1071,8 +1076,13 @@ __device__ bool adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lo
     const LamParams P = a.lp[row];
     const LamDF &E = a.lx[row];
     const BinStates st(slots + KW, B);
+    const uint32_t tfast = kEqual ? piece_tfix(P) : 0u, tfix = kEqual ? coated_tfix(E) : 0u;
+    const uint32_t tfx = kExact ? tfix : tfast, tq = tfx >> kTqShift;
+    constexpr uint32_t delta = kExact ? 0u : kTqDelta;
+    if (kEqual && !kExact && (tfix >> kTqShift) - tq + kTqDelta > 2u * kTqDelta) return ROW_OTHER;
     for (uint32_t b = tid; b < B; b += nthr) {
-        st.s1[b] = st.q1[b] = st.q2[b] = 0ull;
+        st.s1[b] = 0ull;  // kEqual: what the float-float hits add beside tfast
+        if (!kEqual) st.q1[b] = st.q2[b] = 0ull;
         st.n[b] = st.h[b] = 0u;
         st.lanes[b] = make_uint4(0u, 0u, 0u, 0u);
         st.rounds[b] = 0u;
@@ -1100,19 +1110,20 @@ __device__ bool adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lo
     for (uint32_t g0 = g_start; g0 < R; g0 += KW * kRoundRays) {
         // 1. trace round `warp` of the group; each bin's leader sums the round's hits there
         uint32_t bin = 0xffffffffu, tf = 0u;
-        bool used_df = false;
+        bool used_df = false, other = false;
         {
             const uint32_t s = s_nx;
             if (s >= P.band_lo && s < P.band_hi) {
                 const float2 z = z_nx;
                 int res = RAY_FLAG;
-                if (!kExact && !P.all_exact && s >= P.core_lo && s < P.core_hi) {
+                if ((!kExact || kEqual) && !P.all_exact && s >= P.core_lo && s < P.core_hi) {
                     uint32_t b = 0;
                     float t = 0.f;
                     res = fast_ray(C, P, a.guards, z.x, z.y, b, t);
                     if (res == RAY_HIT) {
                         bin = b;
                         tf = t_fixed(t);
+                        other = kEqual && tf != tfast;
                     }
                 }
                 if (res == RAY_FLAG) {
@@ -1120,7 +1131,9 @@ __device__ bool adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lo
                     bin = r.x;
                     tf = r.y;
                     used_df = true;
+                    other = kEqual && bin != 0xffffffffu && tf != tfix;
                 }
+                if (kEqual && kExact) used_df = true;
             }
         }
         if (g0 + KW * kRoundRays < R) fetch(g0 + KW * kRoundRays);
@@ -1133,7 +1146,10 @@ __device__ bool adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lo
             my.df = dfb;
             my.nh = (uint32_t)__popc(hm);
         }
-        {
+        const bool any_other = kEqual && __any_sync(0xffffffffu, other);
+        if (kEqual) {
+            if (leader) my.p[0][lane] = kExact ? 0u : (uint32_t)__popc(grp & dfb);  // float-float hits
+        } else {
             // the bin's sums over its lanes: shared-memory adds into the leader's slot
             my.p[0][lane] = my.p[1][lane] = my.p[2][lane] = my.p[3][lane] = my.p[4][lane] = 0u;
             __syncwarp();
@@ -1163,28 +1179,38 @@ __device__ bool adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lo
             lw = st.lanes[bin];
             rmask = st.rounds[bin];
             cs1 = st.s1[bin];
-            cq1 = st.q1[bin];
-            cq2 = st.q2[bin];
+            if (!kEqual) {
+                cq1 = st.q1[bin];
+                cq2 = st.q2[bin];
+            }
             cn = st.n[bin];
             ch = st.h[bin];
             for (uint32_t m = rmask & ((2u << warp) - 1u); m; m &= m - 1u) {  // rounds <= warp
                 const uint32_t v = (uint32_t)__ffs(m) - 1u, l = lane_entry(lw, v);
                 const RoundSlot &o = slots[v];
                 const uint32_t sq = o.p[0][l - 1u];
-                cs1 += ((unsigned long long)sq << kTqShift) + o.p[1][l - 1u];
-                cq1 += sq;
-                cq2 += ((unsigned long long)o.p[2][l - 1u] << 20) + ((unsigned long long)o.p[3][l - 1u] << 11) +
-                       o.p[4][l - 1u];
+                if (kEqual) {
+                    cs1 += sq * ((unsigned long long)tfix - tfast);
+                } else {
+                    cs1 += ((unsigned long long)sq << kTqShift) + o.p[1][l - 1u];
+                    cq1 += sq;
+                    cq2 += ((unsigned long long)o.p[2][l - 1u] << 20) + ((unsigned long long)o.p[3][l - 1u] << 11) +
+                           o.p[4][l - 1u];
+                }
                 ch += o.p[5][l - 1u];
                 cn += min(kRoundRays, R - (g0 + v * kRoundRays));
             }
-            verdict = sem_quick(cn, ch, cq1, cq2, kExact ? 0u : kTqDelta);
+            verdict = kEqual ? sem_quick_equal(cn, ch, sem_equal(tq, delta)) : sem_quick(cn, ch, cq1, cq2, delta);
+            if (kEqual) {
+                cq1 = (unsigned long long)ch * tq;
+                cq2 = cq1 * tq;
+            }
         }
         if (__any_sync(0xffffffffu, verdict < 0) && verdict < 0)
-            verdict = sem_test(cn, ch, cq1, cq2, kExact ? 0u : kTqDelta);
+            verdict = sem_test(cn, ch, cq1, cq2, delta);
         const bool fail = __any_sync(0xffffffffu, verdict == SEM_FAIL);
         const bool unsure = __any_sync(0xffffffffu, verdict == SEM_UNSURE);
-        if (lane == 0) my.verdict = (!hm || fail) ? 0u : (!kExact && unsure) ? 2u : 1u;
+        if (lane == 0) my.verdict = any_other ? 3u : (!hm || fail) ? 0u : (!kExact && unsure) ? 2u : 1u;
         __syncthreads();
         // 3. the first round that stops ends the row; the states through it are kept
         // (lane v reads round v's verdict)
@@ -1204,8 +1230,10 @@ __device__ bool adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lo
             const uint32_t earlier = rmask & ((1u << warp) - 1u);
             if (warp <= last && !later) {  // the bin's latest round through `last`
                 st.s1[bin] = cs1;
-                st.q1[bin] = cq1;
-                st.q2[bin] = cq2;
+                if (!kEqual) {
+                    st.q1[bin] = cq1;
+                    st.q2[bin] = cq2;
+                }
                 st.n[bin] = cn;
                 st.h[bin] = ch;
             }
@@ -1218,14 +1246,14 @@ __device__ bool adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lo
         __syncthreads();
         if (flag) break;
     }
-    if (flag == 2u) {
-        // the caller redoes the row on the exact path at once
+    if (flag >= 2u) {
+        // the caller redoes the row on the exact path at once, or queues it
         __syncthreads();
-        return true;
+        return flag == 2u ? ROW_UNSURE : ROW_OTHER;
     } else {
         unsigned long long *hrow = a.hist + J.hist_off + (uint64_t)k * B;
         for (uint32_t b = tid; b < B; b += nthr) {
-            const unsigned long long s1 = st.s1[b];
+            const unsigned long long s1 = st.s1[b] + (kEqual ? (unsigned long long)st.h[b] * tfx : 0ull);
             if (s1) hrow[b] = rescale_cell(s1, R, count);
         }
         if (tid == 0) {
@@ -1236,7 +1264,7 @@ __device__ bool adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lo
         }
     }
     __syncthreads();  // the slots and bin states are reused by the block's next row
-    return false;
+    return ROW_DONE;
 }
 
 // One wavelength row under adaptive sampling by a single warp (the form for passes with
@@ -1404,7 +1432,6 @@ __device__ bool adaptive_row1(const LaunchArgs &a, uint64_t row, unsigned long l
 // bound. Returns ROW_DONE; ROW_UNSURE when the bound leaves a decision open (the caller redoes the
 // row with kExact); or ROW_OTHER when a hit's transmittance is another (an exit face met at
 // cos <= 0.5): the general exact path takes the row.
-enum : int { ROW_DONE = 0, ROW_UNSURE = 1, ROW_OTHER = 2 };
 struct Adapt1Pieces {
     LamParams P;
     FastConst C;
@@ -1803,7 +1830,7 @@ __device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t
             uint32_t n = 0u, h = 0u;
             if (np > 1u) {
                 // this stretch's share, for the stretches after it (one stretch, every thread a bin of its
-                // own: nothing to pass on; 1200 rows x 1024 rays in 236 bins 57 -> 55 us)
+                // own: nothing to pass on; calls of 472 rows x 4096 rays in 200 bins 109 -> 104 us)
                 for (uint32_t q = qa; q < qb && act; q++) {
                     const uint32_t c = counts[q * stride + b];
                     if (c) n += min(kRoundRays, R - (r0 + q) * kRoundRays);
@@ -1827,7 +1854,7 @@ __device__ __forceinline__ int adaptive_row_pieces(const LaunchArgs &a, uint64_t
                     n += min(kRoundRays, R - (r0 + q) * kRoundRays);
                     h += c;
                     // with a thread per bin, a bin that failed has often settled the round already
-                    // (1200 rows x 1024 rays in 236 bins: 55 -> 49 us; with stretches, no gain)
+                    // (the same calls: 107 -> 104 us; with stretches, no gain)
                     if (np == 1u && *(volatile uint8_t *)&S.test[q]) continue;
                     int verdict = sem_quick_equal(n, h, se);
                     if (verdict < 0) verdict = sem_test(n, h, (uint64_t)h * tq, (uint64_t)h * tq * tq, delta);
@@ -1912,9 +1939,9 @@ __device__ __noinline__ int adaptive_row_redo(const LaunchArgs &a, unsigned long
 // Passes with fewer rows than adaptive1_kernel's: one row per block (rows of designs without
 // pieces are adaptive_kernel's). The chain of a row bounds it: up to 256 rounds are binned at once
 // by all warps and then decided, instead of 16 rounds per three barriers: a call of 128 rows x up
-// to 8192 rays 101 -> 70 us, one whose rows are redone 90 -> 79. The tests of step 2 run for 32
-// bins at a time whether one or all were hit: with 64 bins 900 rows x 2048 rays take 47 us (53 ray
-// by ray), with 200, 75 (63).
+// to 8192 rays in 32 bins 101 -> 80 us, some of its rows redone. The tests of step 2 run for 32
+// bins at a time whether one or all were hit, so wide detectors and short tables are not for it
+// (adapt_by_blocks).
 __global__ void __launch_bounds__(32 * kMaxAdaptWarps, 2) adaptive_block_kernel(const LaunchArgs a)
 {
     extern __shared__ __align__(16) unsigned long long adapt_smem[];
@@ -1942,6 +1969,25 @@ __global__ void __launch_bounds__(32 * kMaxAdaptWarps, CPD_ADAPT_MIN_BLOCKS) ada
     // the float-float path from its first round, while other blocks go on with theirs
     if (adaptive_row<false>(a, blockIdx.x, adapt_smem, kw, warp, lane))
         adaptive_row<true>(a, blockIdx.x, adapt_smem, kw, warp, lane);
+}
+
+__device__ __noinline__ int adaptive_equal_redo(const LaunchArgs &a, unsigned long long *smem)
+{
+    return adaptive_row<true, true>(a, blockIdx.x, smem, blockDim.x >> 5, threadIdx.x >> 5, threadIdx.x & 31u);
+}
+
+// The same for the rows of designs with certified pieces, ray by ray: passes with few rows that
+// adaptive_block_kernel is slower for (adapt_by_blocks).
+__global__ void __launch_bounds__(32 * kMaxAdaptWarps, CPD_ADAPT_MIN_BLOCKS) adaptive_equal_kernel(const LaunchArgs a)
+{
+    extern __shared__ __align__(16) unsigned long long adapt_smem[];
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();  // the setup's LamParams and LamDF
+    const uint32_t kw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    if (a.adapt_pieces != 1u && !a.designs[find_job<F_ROW>(a.jobs, a.njobs, blockIdx.x)].fc.pieces) return;
+    int r = adaptive_row<false, true>(a, blockIdx.x, adapt_smem, kw, warp, lane);
+    if (r == ROW_UNSURE) r = adaptive_equal_redo(a, adapt_smem);
+    if (r == ROW_OTHER && threadIdx.x == 0) queue_row(a, blockIdx.x);
 }
 
 // Out of line: rows of designs without pieces, and the rare ones that the pieces leave (exact:
@@ -3797,6 +3843,33 @@ RowsPlan plan_rows(uint64_t rows, uint32_t R, uint32_t max_B, int num_sms)
     return p;
 }
 
+// Whether the rows of designs with pieces go through adaptive_block_kernel (true) or
+// adaptive_equal_kernel, in adaptive passes of fewer than 8 rows per SM. The first bins by pieces, but
+// tests every bin of every round; the second traces ray by ray, 16 (4) rounds at a time, and tests
+// the bins that a round hit. So the first is for long tables and narrow detectors. Calls in us, first /
+// second (three designs each; over 4032 sizes of up to 1024 bins and 1200 rows the lines below are within
+// 0.3 % of the faster of the two on average):
+//   up to 2 rows per SM, 100 rows: 64 bins x 300 rays 47 / 46, x 1024 49 / 50, x 4096 59 / 75; 256 bins
+//     x 2048 61 / 61, x 4096 78 / 80; 800 bins x 1024 64 / 53, x 16384 264 / 163: a round costs the first
+//     more with more bins, and a group of 16 rounds the second hardly more than one;
+//   up to 4, 472 rows: as long as all blocks are resident, 200 bins x 4096 112 / 130, x 8192 (4 rows on
+//     some SM, room for 3) 222 / 206; 512 bins x 8192 314 / 243;
+//   beyond, 900 rows: 64 bins x 300 55 / 53, x 8192 158 / 214; 128 x 16384 315 / 321; 160 x 16384 366 / 259;
+//     512 x 8192 463 / 292: rows wait for a place, and of blocks of the second twice as many fit.
+static bool adapt_by_blocks(uint32_t max_B, uint64_t rows, uint32_t max_rounds, int num_sms)
+{
+    const uint64_t per_sm = rows / (uint64_t)num_sms, setup = (rows + 31u) / 32u;  // setup: its blocks
+    const size_t bytes = adapt_block_smem_bytes(max_B, max_rounds);
+    // Beside a setup block an SM has no room for arrays of 50 KB: from 148 rows on two rows share an SM,
+    // though there is one for each. 236 bins x 16384, 147 rows 156 / 165, 148 rows 193 / 165
+    if (rows <= (uint64_t)num_sms && rows + setup > (uint64_t)num_sms && bytes > 50u * 1024u) return false;
+    if (per_sm < 2) return max_B <= 256u && max_rounds > 20u + max_B / 4u;
+    if (per_sm >= 4) return max_B <= 128u && max_rounds >= 24u && max_rounds * max_B <= 65536u;
+    // (blocks of 8 warps at 64 registers: four)
+    const uint64_t room = std::min<uint64_t>(4u, (227u * 1024u) / (bytes + 1024u));
+    return max_B <= 400u && max_rounds >= 16u && rows <= room * (uint64_t)num_sms;
+}
+
 int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaStream_t stream, cudaEvent_t *ev,
                 bool pdl)
 {
@@ -3844,11 +3917,14 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
                          a.adapt_pieces == 1u ? smem : std::max(smem, adapt1_smem_bytes(maxB)), stream, pdl, a);
                 launches++;
             } else {
-                if (a.adapt_pieces) {
+                if (a.adapt_pieces && !adapt_by_blocks(maxB, a.total_rows, a.max_rounds, num_sms)) {
+                    launch_k(adaptive_equal_kernel, (unsigned)a.total_rows, 32 * kw, adapt_smem_bytes(kw, maxB), stream, pdl, a);
+                    launches++;
+                } else if (a.adapt_pieces) {
                     // 2 to 7 rows per SM: 8 warps, four such blocks per SM; 4 warps where more rows
-                    // than that have few rounds. Calls, 16 / 8 / 4 warps: 472 x 602 rays 65 / 57 /
-                    // 62 us, 472 x 4096 97 / 90 / 110, 1000 x 8192 174 / 162 / 193, 700 x 602
-                    // 60 / 55 / 50, 1200 x 1024 110 / 94 / 88
+                    // than that have few rounds. Calls, 16 / 8 / 4 warps: 472 x 602 rays in 100 bins 57 /
+                    // 52 / 55 us, 472 x 4096 in 200 119 / 103 / 135, 1000 x 8192 in 64 174 / 161 / 181,
+                    // 700 x 1024 in 64 66 / 61 / 57, 1200 x 1024 in 100 92 / 75 / 67
                     const uint32_t kb = kw == kMaxAdaptWarps ? kw : per_sm >= 4 && a.max_rounds <= 32u ? 4u : 8u;
                     launch_k(adaptive_block_kernel, (unsigned)a.total_rows, 32 * kb,
                              adapt_block_smem_bytes(maxB, a.max_rounds), stream, pdl, a);
@@ -3941,6 +4017,7 @@ cudaError_t configure_kernels()
 {
     const int bytes = (int)adapt_smem_bytes(kMaxAdaptWarps, CPD_MAX_BINS);
     cudaError_t e = cudaFuncSetAttribute(adaptive_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(adaptive_equal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(adaptive1_pieces_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)std::max(adapt1_smem_bytes(CPD_MAX_BINS), adapt1p_smem_bytes(CPD_MAX_BINS)));

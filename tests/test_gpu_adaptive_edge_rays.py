@@ -1,19 +1,20 @@
 """Adaptive sampling of rows with more rays at a bin's edge than a block lists (or such rays only
-past the row's stop): rays, hits and p(d|lambda) are those that the same rows have in a pass of many
-rows, where a warp takes a row round by round, and the oracle's."""
+past the row's stop), and of rows whose hits have more than one transmittance: rays, hits and
+p(d|lambda) are those that the same rows have in a pass of many rows, where a warp takes a row round
+by round, and the oracle's."""
 import numpy as np
 import pytest
 
 import compound_prism_designer as cpd
 import oracle as O
 from compound_prism_designer import synth
+from test_gpu_tp_handed_back import _two_sided
 
 pytestmark = pytest.mark.gpu
 MODE = cpd.TRACE_HYBRID | cpd.SAMPLING_ADAPTIVE
-B = 24
 
 
-def _edge_and_middle(spec, d, lam):
+def _edge_and_middle(spec, d, lam, B):
     """Two ray points at wavelength lam: one on the upper edge of a bin, one well inside that bin."""
     (px, py), (ux, uy) = spec.design.det_position, spec.design.det_direction
 
@@ -46,24 +47,26 @@ def _edge_and_middle(spec, d, lam):
     return None
 
 
-def _cases():
+def _cases(B):
     rng = np.random.default_rng(77)
     out = []
     while len(out) < 3:
         spec, d, _ = synth.random_design(rng, 3, B)
         u0 = float(rng.uniform(0.2, 0.8))
         lo, hi = d["wavelength_bounds"]
-        got = _edge_and_middle(spec, d, lo + (hi - lo) * u0)
+        got = _edge_and_middle(spec, d, lo + (hi - lo) * u0, B)
         if got:
             k = np.arange(1300)  # the edge ray hits on one side of u0 and is lost on the other
             out.append((spec, d, u0 + 1e-9 * (1 + k // 2) * (-1.0) ** k, *got))
     return out
 
 
+# few rows of a narrow detector are decided many rounds at once, of a wide one in groups of 16 rounds
+@pytest.mark.parametrize("B", [24, 300])
 @pytest.mark.parametrize("kind", ["all along", "past the stop", "few"])
-def test_rows_alone_equal_rows_among_many(kind):
+def test_rows_alone_equal_rows_among_many(kind, B):
     R = 8192
-    for spec, d, lam, edge, middle in _cases():
+    for spec, d, lam, edge, middle in _cases(B):
         if kind == "all along":  # half of the rays on the edge
             rays = np.tile([edge, middle], R // 2)
         elif kind == "past the stop":  # every ray of the first rounds hits the one bin
@@ -77,4 +80,21 @@ def test_rows_alone_equal_rows_among_many(kind):
         assert np.array_equal(p[:8], q)
         po, st, n = O.fitness_adaptive_points(d, lam[:8], rays, 8)
         assert np.abs(q - po).max() <= 1e-6 and g.rays == int(n.sum()) and g.hits == st["hits"]
-        assert (int(n.sum()) == 8 * 32) == (kind == "past the stop")
+        assert (np.sum(n == 32) >= 4) if kind == "past the stop" else np.any(n > 32)
+
+
+@pytest.mark.parametrize("R", [40, 2000, 8192])
+@pytest.mark.parametrize("B", [8, 100, 300])
+def test_rows_of_two_transmittances(B, R):
+    rng = np.random.default_rng([B, R])
+    for _ in range(3):
+        spec, d = _two_sided(rng, B)
+        lam, rays = rng.uniform(size=1300), rng.uniform(size=R)
+        f, p = spec.gpu_fitness_points(lam, rays, want_p=True, mode=MODE)
+        for n in (5, 330, 700):  # one row per SM at most, two or three, four or more
+            g, q = spec.gpu_fitness_points(lam[:n], rays, want_p=True, mode=MODE)
+            assert np.array_equal(p[:n], q)
+        po, st, count = O.fitness_adaptive_points(d, lam[:200], rays, 8)
+        assert np.abs(p[:200] - po).max() <= 1e-6
+        g, _ = spec.gpu_fitness_points(lam[:200], rays, want_p=True, mode=MODE)
+        assert g.rays == int(count.sum()) and g.hits == st["hits"]
