@@ -436,17 +436,17 @@ __global__ void __launch_bounds__(kTableThreads) table_sort_kernel(const LaunchA
 }
 
 // One thread per sorted position: its z in f64 (the host's own operations but for CUDA's log),
-// split into floats, and the ray's rank. blockIdx.y is the table. A warp's f64 instruction
-// takes its scheduler ~64 cycles, so the positions are spread two warps to a block; with a
-// known order this kernel is all a new seed costs, beside the setup's face loop (FP64
-// issue bounds it).
+// split into floats, and the ray's rank. blockIdx.x is the table (a pass may have more than 65535).
+// A warp's f64 instruction takes its scheduler ~64 cycles, so the positions are spread two warps to
+// a block; with a known order this kernel is all a new seed costs, beside the setup's face loop
+// (FP64 issue bounds it).
 __global__ void __launch_bounds__(64) table_z_kernel(const LaunchArgs a)
 {
     stamp_start(a, STAMP_Z);
     cudaTriggerProgrammaticLaunchCompletion();
     if (a.nsort) cudaGridDependencySynchronize();  // the order
-    const TableJob t = a.tables[blockIdx.y];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const TableJob t = a.tables[blockIdx.x];
+    const uint32_t i = blockIdx.y * blockDim.x + threadIdx.x;
     if (i >= t.R) return;
     const uint32_t at = i + t.rot;
     const uint32_t j = t.order ? t.order[at < t.R ? at : at - t.R] : a.perm[t.ray_off + i];
@@ -3889,7 +3889,7 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
             launch_k(table_sort_kernel, a.nsort, kTableThreads, table_smem_bytes(M, a.table_max), stream, false, a);
             launches++;
         }
-        launch_k(table_z_kernel, dim3((a.table_max + 63u) / 64u, a.ntables), 64, 0, stream, pdl && a.nsort, a);
+        launch_k(table_z_kernel, dim3(a.ntables, (a.table_max + 63u) / 64u), 64, 0, stream, pdl && a.nsort, a);
         launches++;
     }
     if (a.params) {
