@@ -373,6 +373,39 @@ void mark_host_only(cpd_context *ctx, const std::vector<std::pair<double, uint32
     }
 }
 
+// Whether a pass gives its coated designs to rows_kernel (by_rows), the rule for all of them: under
+// the fixed-N hybrid trace, but for short tables on many rows, whose pieces of a few rays save less
+// than their edges cost. The ray-by-ray kernels give the same numbers. us, rows_kernel / ray by ray: 64
+// designs x 4096 rows, 16 bins, 64 rays 538 / 320, 128 496 / 397, 200 475 / 484; 64 bins, 64 rays 649 /
+// 469, 200 691 / 638, 256 698 / 679, 320 692 / 740; 128 designs x 128 rows, 32 bins, 128 rays 243 / 231;
+// 64 x 128 150 / 163; one design x 16384, 16 bins, 128 rays 64 / 57, 256 62 / 66; 64 bins, 128 rays 88 /
+// 73; 100 bins 103 / 107, 256 bins 99 / 153 (a cell's histogram costs the ray-by-ray kernels more).
+struct RowsRule {
+    uint64_t rows = 0, coated_rows = 0, coated_rays = 0;
+    uint32_t n = 0, max_B = 0, max_R = 0;  // max_R: of the coated designs
+    bool on = false;
+};
+bool coated(const PassDesign &p) { return p.params ? p.params->ar_coated != 0 : p.dev->fc.pieces != 0; }
+RowsRule rows_rule(const std::vector<PassDesign> &ds, uint32_t mode)
+{
+    RowsRule r;
+    r.n = (uint32_t)ds.size();
+    for (const PassDesign &p : ds) {
+        r.rows += p.W;
+        r.max_B = std::max(r.max_B, p.params ? p.params->bin_count : p.dev->B);
+        if (!coated(p)) continue;
+        r.coated_rows += p.W;
+        r.coated_rays += (uint64_t)p.W * p.R;
+        r.max_R = std::max(r.max_R, p.R);
+    }
+    const bool many = r.n > 1 ? r.rows >= 16384u : r.rows >= 8192u && r.max_B <= 80u;
+    r.on = mode == CPD_TRACE_HYBRID && r.coated_rows && !(many && r.coated_rays <= 256u * r.coated_rows);
+    return r;
+}
+// A coated design under that rule (a device build decides in its record whether the pieces apply;
+// if not, its rays go through fast_ray there).
+bool by_rows(const PassDesign &p, const RowsRule &r) { return r.on && coated(p); }
+
 uint32_t tile_rows_for(uint32_t B, uint32_t n)
 {
     return std::max<uint32_t>(1u, (n > 1 ? kTileCellsBatch : kTileCells) / B);
@@ -410,20 +443,10 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     bool cacheable = true, any_host = false;
     uint32_t table_max = 0;
     uint64_t rows = 0, groups = 0, hist = 0, cells = 0, lam = 0, upts = 0, ray = 0, rnk = 0, accc = 0, items = 0, tiles = 0;
-    uint32_t max_B = 0;
-    // a coated design under the fixed-N hybrid trace goes through rows_kernel (a device build
-    // decides in its record whether the pieces apply; if not, its rays go through fast_ray there)
-    const auto by_pieces = [&](const PassDesign &p) {
-        return mode == CPD_TRACE_HYBRID && !adaptive && (p.params ? p.params->ar_coated != 0 : p.dev->fc.pieces != 0);
-    };
-    uint64_t piece_rows = 0;
-    uint32_t piece_R = 0;
-    for (const PassDesign &p : ds) {
-        max_B = std::max(max_B, p.params ? p.params->bin_count : p.dev->B);
-        if (by_pieces(p)) piece_rows += p.W, piece_R = std::max(piece_R, p.R);
-    }
+    const RowsRule rule = rows_rule(ds, adaptive ? CPD_SAMPLING_ADAPTIVE : mode);
+    const uint32_t max_B = rule.max_B;
     RowsPlan plan{1u, 1u};
-    if (piece_rows) plan = plan_rows(piece_rows, piece_R, max_B, ctx->num_sms);
+    if (rule.on) plan = plan_rows(rule.coated_rows, rule.max_R, max_B, ctx->num_sms);
     for (uint32_t i = 0; i < n; i++) {
         const PassDesign &p = ds[i];
         DesignJob &J = jobs[i];
@@ -478,7 +501,7 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
         J.item_off = items;
         J.tile_off = tiles;
         J.nchunk = std::max<uint32_t>(1u, (J.Rz + ctx->ray_tile - 1) / ctx->ray_tile);
-        J.pieces = by_pieces(p) ? 1u : 0u;
+        J.pieces = by_rows(p, rule) ? 1u : 0u;
         J.hist_off = hist;
         J.grp_off = groups;
         J.grp_rows = std::min(plan.group, std::max(1u, kRowsCells / J.B));
@@ -577,7 +600,7 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
     // the LamParams, then (single-design passes) one span per 32-row block
     // or, where rows_kernel's teams are small, a HeavyRow for each
     const bool heavy = groups && plan.team < kRowsWarps &&
-                       (n > 1 || (uint64_t)plan.group * piece_R / plan.team >= kRowsHeavyGroup);
+                       (n > 1 || (uint64_t)plan.group * rule.max_R / plan.team >= kRowsHeavyGroup);
     CPD_TRY(S.lp.ensure(sizeof(LamParams) * std::max<uint64_t>(rows, 1) + sizeof(uint2) * ((rows + 31) / 32) +
                         (heavy ? 16u + sizeof(HeavyRow) * rows : 0)));
     CPD_TRY(S.lx.ensure(sizeof(LamDF) * std::max<uint64_t>(rows, 1)));
@@ -898,11 +921,9 @@ int run_pass_checked(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign
 }
 
 // Whether every design of a batch goes through rows_kernel, which has no launch shape to tune.
-bool all_pieces(const std::vector<PassDesign> &ds, uint32_t mode)
+bool all_by_rows(const std::vector<PassDesign> &ds, uint32_t mode)
 {
-    return mode == CPD_TRACE_HYBRID && std::all_of(ds.begin(), ds.end(), [](const PassDesign &p) {
-        return p.params ? p.params->ar_coated != 0 : p.dev->fc.pieces != 0;
-    });
+    return rows_rule(ds, mode).on && std::all_of(ds.begin(), ds.end(), coated);
 }
 
 // The class of a batch for the launch-shape cache: trace mode, whether it has a shape to tune, and
@@ -920,7 +941,7 @@ std::array<uint64_t, 6> tune_class(const std::vector<PassDesign> &ds, uint32_t m
         while ((1ull << b) < v && b < 63) b++;
         return b;
     };
-    return {mode, all_pieces(ds, mode), lg(ds.size()), lg(rows), lg(rays), lg(maxB)};
+    return {mode, all_by_rows(ds, mode), lg(ds.size()), lg(rows), lg(rays), lg(maxB)};
 }
 
 // The autotuner: times every (ray tile, warps per CTA) candidate on the batch itself
@@ -939,7 +960,7 @@ int tune_pass(cpd_context *ctx, const std::vector<PassDesign> &ds, uint32_t mode
     // Besides the powers of two: tiles that make the work items a whole number of rounds
     // of the resident warps (2..6 items per warp), so that the last round is not a tail.
     std::vector<std::pair<uint32_t, uint32_t>> cands;
-    const bool pieces = all_pieces(ds, mode);
+    const bool pieces = all_by_rows(ds, mode);
     if (pieces) cands.push_back({rt0, w0});  // no work items: the caller's shape stays
     for (uint32_t w : kWarps) {
         if (pieces) break;
