@@ -538,10 +538,13 @@ __device__ __forceinline__ void setup_row(const LaunchArgs &a, uint64_t row, uin
 // instead of a chain of dependent loads), so the per-wavelength program and its binary
 // searches run on shared-memory operands. Ray tables start 16-byte aligned (the host
 // pads each to an even number of rays).
+// STAMPED: the pass's first stamp (a branch of its own in front of the trigger below costs passes of
+// several designs 2 to 4 us, though none of them takes it: 8 x 128 rows, adaptive, 66.6 -> 71.1).
 constexpr uint32_t kSetupThreads = 128;
+template <bool STAMPED>
 __global__ void __maxnreg__(96) setup_kernel(const LaunchArgs a)
 {
-    stamp_start(a, STAMP_SETUP);
+    if (STAMPED) stamp_start(a, STAMP_SETUP);
     // lets the trace kernel's blocks become resident now; they wait for this grid's
     // results in cudaGridDependencySynchronize
     cudaTriggerProgrammaticLaunchCompletion();
@@ -3903,7 +3906,7 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
         const uint32_t rows = !a.spans && a.total_rows >= (uint64_t)num_sms * 32u * 16u ? kSetupThreads : 32u;
         const uint32_t blocks = (uint32_t)((a.total_rows + rows - 1u) / rows);
         const uint32_t cap = a.stage_cap < kStageRays ? a.stage_cap : kStageRays;
-        launch_k(a.spans ? setup_pair_kernel : setup_kernel, blocks, a.spans ? 64 : rows,
+        launch_k(a.spans ? setup_pair_kernel : a.stamp == STAMP_SETUP ? setup_kernel<true> : setup_kernel<false>, blocks, a.spans ? 64 : rows,
                  2 * ((cap + 1u) & ~1u) * sizeof(float), stream, pdl && a.ntables && !a.params, a);
         launches++;
     }
