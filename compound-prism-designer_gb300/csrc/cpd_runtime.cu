@@ -380,9 +380,12 @@ void mark_host_only(cpd_context *ctx, const std::vector<std::pair<double, uint32
 // 469, 200 691 / 638, 256 698 / 679, 320 692 / 740; 128 designs x 128 rows, 32 bins, 128 rays 243 / 231;
 // 64 x 128 150 / 163; one design x 16384, 16 bins, 128 rays 64 / 57, 256 62 / 66; 64 bins, 128 rays 88 /
 // 73; 100 bins 103 / 107, 256 bins 99 / 153 (a cell's histogram costs the ray-by-ray kernels more).
+// Beside designs for the ray-by-ray kernels it is one more kernel in the chain (~20 us), which takes
+// 8 M coated rays to win back: 4 coated and 4 uncoated designs of 128 rows, 2.1 M coated rays 119 / 110,
+// 4.2 M 135 / 133, 8.4 M 157 / 175; 32 and 1, 4.2 M 156 / 138, 8.4 M 161 / 161, 16.8 M 177 / 201.
 struct RowsRule {
     uint64_t rows = 0, coated_rows = 0, coated_rays = 0;
-    uint32_t n = 0, max_B = 0, max_R = 0;  // max_R: of the coated designs
+    uint32_t n = 0, others = 0, max_B = 0, max_R = 0;  // others: not coated; max_R: of the coated designs
     bool on = false;
 };
 bool coated(const PassDesign &p) { return p.params ? p.params->ar_coated != 0 : p.dev->fc.pieces != 0; }
@@ -393,13 +396,17 @@ RowsRule rows_rule(const std::vector<PassDesign> &ds, uint32_t mode)
     for (const PassDesign &p : ds) {
         r.rows += p.W;
         r.max_B = std::max(r.max_B, p.params ? p.params->bin_count : p.dev->B);
-        if (!coated(p)) continue;
+        if (!coated(p)) {
+            r.others++;
+            continue;
+        }
         r.coated_rows += p.W;
         r.coated_rays += (uint64_t)p.W * p.R;
         r.max_R = std::max(r.max_R, p.R);
     }
     const bool many = r.n > 1 ? r.rows >= 16384u : r.rows >= 8192u && r.max_B <= 80u;
-    r.on = mode == CPD_TRACE_HYBRID && r.coated_rows && !(many && r.coated_rays <= 256u * r.coated_rows);
+    r.on = mode == CPD_TRACE_HYBRID && r.coated_rows && !(many && r.coated_rays <= 256u * r.coated_rows) &&
+           (!r.others || r.coated_rays >= 1u << 23);
     return r;
 }
 // A coated design under that rule (a device build decides in its record whether the pieces apply;

@@ -35,3 +35,12 @@ def test_batches(rows, R):
     params = cpd.fitness_batch(specs, seeds=0.3, max_n=W, max_eval=R)
     for spec, w, f in zip(specs, W, params):
         _same(f, spec.gpu_fitness_full([0.3], max_n=w, max_eval=R))
+
+
+@pytest.mark.parametrize("W", [511, 512])  # of the coated designs: 8.4 M rays and a few less
+def test_beside_uncoated_designs(W):
+    rng = np.random.default_rng(W)
+    specs = [synth.random_design(rng, 3, B, ar_coated=ar)[0] for B, ar in ((32, True), (64, False), (9, True))]
+    n, R = [W, 40, 512], 8192
+    for spec, w, f in zip(specs, n, cpd.fitness_batch(specs, seeds=0.3, max_n=n, max_eval=R)):
+        _same(f, spec.gpu_fitness_full([0.3], max_n=w, max_eval=R))
