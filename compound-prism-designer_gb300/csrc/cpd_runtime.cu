@@ -299,8 +299,29 @@ struct PassResult {
     bool bad_table = false;   // a ray table could not be made on the device
 };
 
-// Whether a pass may make the ray table on the device: its points lie in (0, 1), it fits
-// table_sort_kernel, and the trace does not read the f64 table.
+// Whether points in (0, 1) crowd in table_sort_kernel's buckets, as far as 64 of them show it (that
+// takes 0.3 us, all of 3000 points 3): a pass that finds a bucket too full is run again with the host's
+// table, 340 instead of 250 us for 4000 points within 1e-9 of each other.
+bool crowded(const double *u, uint32_t R)
+{
+    if (R <= kTableBucket) return false;
+    uint32_t M = 1024u;
+    while (M < R) M <<= 1;
+    const uint32_t n = std::min(R, 64u);
+    uint32_t b[64];
+    for (uint32_t i = 0; i < n; i++) b[i] = (uint32_t)(u[(uint64_t)i * R / n] * M);
+    std::sort(b, b + n);
+    bool suspect = false;  // of 64 points spread evenly, four in one of 1024 buckets: 1 in 1600
+    for (uint32_t i = 3; i < n; i++) suspect |= b[i] == b[i - 3];
+    if (!suspect) return false;
+    std::vector<uint32_t> count(M, 0u);
+    for (uint32_t j = 0; j < R; j++)
+        if (++count[(uint32_t)(u[j] * M)] > kTableBucket) return true;
+    return false;
+}
+
+// Whether a pass may make the ray table on the device: its points lie in (0, 1) and do not crowd, it
+// fits table_sort_kernel, and the trace does not read the f64 table.
 bool device_table(cpd_context *ctx, const PassDesign &p, uint32_t mode)
 {
     if (p.R > kTableRays || (mode & ~kSamplingBits) == CPD_TRACE_FP64) return false;
@@ -313,7 +334,7 @@ bool device_table(cpd_context *ctx, const PassDesign &p, uint32_t mode)
     }
     bool in = true;
     for (uint32_t j = 0; j < p.R; j++) in &= p.ray_u[j] > 0.0 && p.ray_u[j] < 1.0;
-    return in;
+    return in && !crowded(p.ray_u, p.R);
 }
 
 // PointOrders' calls, on a slot's stream.
