@@ -185,7 +185,8 @@ struct LaunchArgs {
     uint32_t stage_cap;
     uint32_t mode;        // CPD_TRACE_*
     uint32_t adaptive;    // per-wavelength SEM stop: 1, or 2 with every row on the exact path
-    uint32_t adapt_pieces;  // adaptive sampling: 1 every design has certified pieces, 2 some may
+    uint32_t adapt_pieces;  // adaptive sampling: 1 every design has certified pieces, 2 every one may
+                            // (device builds decide), 3 some have none
     uint32_t max_B;       // widest detector of the launch
     uint64_t total_groups;  // groups of rows of the designs with J.pieces
     uint32_t team;          // rows_kernel: warps per group

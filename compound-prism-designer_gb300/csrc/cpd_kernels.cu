@@ -1008,7 +1008,7 @@ struct RoundSlot {
     uint32_t p[6][32];
     uint32_t df;       // ballot of the rays traced in float-float
     uint32_t nh;       // hits of the round
-    uint32_t verdict;  // 0 go on, 1 stop, 2 unsure, 3 a hit of another transmittance (kEqual)
+    uint32_t verdict;  // 0 go on, 1 stop, 2 unsure, 3 a hit of another transmittance (ROWS_EQUAL)
     uint32_t pad;
 };
 static_assert(sizeof(RoundSlot) % 16 == 0, "bin states follow the slots 16-byte aligned");
@@ -1049,12 +1049,13 @@ __device__ __forceinline__ uint32_t lane_entry(const uint4 &w, uint32_t v)
 // stop decision the FP32 transmittances cannot settle (sem_test: SEM_UNSURE) leaves
 // nothing behind and returns ROW_UNSURE: the caller redoes it on the exact path. (In the
 // verification mode every row is queued for adaptive_exact_kernel instead.)
-// kEqual: a design with certified pieces. Its rows have the arithmetic of adaptive_row1_pieces,
-// decision for decision (one transmittance, states of samples and hits alone, a row with a hit of
-// another transmittance up to its stop returned as ROW_OTHER), so that they come out the same here
-// and there; kExact then concerns the transmittance and the test.
+// ROWS_EQUAL: a design with certified pieces (ROWS_MIXED: if it has them). Its rows have the
+// arithmetic of adaptive_row1_pieces, decision for decision (one transmittance, states of samples and
+// hits alone, a row with a hit of another transmittance up to its stop returned as ROW_OTHER), so
+// that they come out the same here and there; kExact then concerns the transmittance and the test.
 enum : int { ROW_DONE = 0, ROW_UNSURE = 1, ROW_OTHER = 2 };
-template <bool kExact, bool kEqual = false>
+enum : int { ROWS_GENERAL = 0, ROWS_EQUAL = 1, ROWS_MIXED = 2 };
+template <bool kExact, int kRows = ROWS_GENERAL>
 __device__ int adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long long *smem, uint32_t KW,
                              uint32_t warp, uint32_t lane)
 {
@@ -1063,6 +1064,7 @@ __device__ int adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lon
     const uint32_t k = (uint32_t)(row - J.row_off);
     const uint32_t B = J.B, R = J.R;
     const DevDesign &D = a.designs[d];
+    const bool equal = kRows == ROWS_MIXED ? D.fc.pieces != 0u : kRows == ROWS_EQUAL;
     const uint32_t tid = warp * 32u + lane, nthr = KW * 32u;
     if (!kExact && a.adaptive == 2u) {
         // verification mode: every row on the exact path
@@ -1079,13 +1081,13 @@ __device__ int adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lon
     const LamParams P = a.lp[row];
     const LamDF &E = a.lx[row];
     const BinStates st(slots + KW, B);
-    const uint32_t tfast = kEqual ? piece_tfix(P) : 0u, tfix = kEqual ? coated_tfix(E) : 0u;
+    const uint32_t tfast = equal ? piece_tfix(P) : 0u, tfix = equal ? coated_tfix(E) : 0u;
     const uint32_t tfx = kExact ? tfix : tfast, tq = tfx >> kTqShift;
     constexpr uint32_t delta = kExact ? 0u : kTqDelta;
-    if (kEqual && !kExact && (tfix >> kTqShift) - tq + kTqDelta > 2u * kTqDelta) return ROW_OTHER;
+    if (equal && !kExact && (tfix >> kTqShift) - tq + kTqDelta > 2u * kTqDelta) return ROW_OTHER;
     for (uint32_t b = tid; b < B; b += nthr) {
-        st.s1[b] = 0ull;  // kEqual: what the float-float hits add beside tfast
-        if (!kEqual) st.q1[b] = st.q2[b] = 0ull;
+        st.s1[b] = 0ull;  // equal: what the float-float hits add beside tfast
+        if (!equal) st.q1[b] = st.q2[b] = 0ull;
         st.n[b] = st.h[b] = 0u;
         st.lanes[b] = make_uint4(0u, 0u, 0u, 0u);
         st.rounds[b] = 0u;
@@ -1119,14 +1121,14 @@ __device__ int adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lon
             if (s >= P.band_lo && s < P.band_hi) {
                 const float2 z = z_nx;
                 int res = RAY_FLAG;
-                if ((!kExact || kEqual) && !P.all_exact && s >= P.core_lo && s < P.core_hi) {
+                if ((!kExact || equal) && !P.all_exact && s >= P.core_lo && s < P.core_hi) {
                     uint32_t b = 0;
                     float t = 0.f;
                     res = fast_ray(C, P, a.guards, z.x, z.y, b, t);
                     if (res == RAY_HIT) {
                         bin = b;
                         tf = t_fixed(t);
-                        other = kEqual && tf != tfast;
+                        other = equal && tf != tfast;
                     }
                 }
                 if (res == RAY_FLAG) {
@@ -1134,9 +1136,9 @@ __device__ int adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lon
                     bin = r.x;
                     tf = r.y;
                     used_df = true;
-                    other = kEqual && bin != 0xffffffffu && tf != tfix;
+                    other = equal && bin != 0xffffffffu && tf != tfix;
                 }
-                if (kEqual && kExact) used_df = true;
+                if (equal && kExact) used_df = true;
             }
         }
         if (g0 + KW * kRoundRays < R) fetch(g0 + KW * kRoundRays);
@@ -1149,8 +1151,8 @@ __device__ int adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lon
             my.df = dfb;
             my.nh = (uint32_t)__popc(hm);
         }
-        const bool any_other = kEqual && __any_sync(0xffffffffu, other);
-        if (kEqual) {
+        const bool any_other = equal && __any_sync(0xffffffffu, other);
+        if (equal) {
             if (leader) my.p[0][lane] = kExact ? 0u : (uint32_t)__popc(grp & dfb);  // float-float hits
         } else {
             // the bin's sums over its lanes: shared-memory adds into the leader's slot
@@ -1182,7 +1184,7 @@ __device__ int adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lon
             lw = st.lanes[bin];
             rmask = st.rounds[bin];
             cs1 = st.s1[bin];
-            if (!kEqual) {
+            if (!equal) {
                 cq1 = st.q1[bin];
                 cq2 = st.q2[bin];
             }
@@ -1192,7 +1194,7 @@ __device__ int adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lon
                 const uint32_t v = (uint32_t)__ffs(m) - 1u, l = lane_entry(lw, v);
                 const RoundSlot &o = slots[v];
                 const uint32_t sq = o.p[0][l - 1u];
-                if (kEqual) {
+                if (equal) {
                     cs1 += sq * ((unsigned long long)tfix - tfast);
                 } else {
                     cs1 += ((unsigned long long)sq << kTqShift) + o.p[1][l - 1u];
@@ -1203,8 +1205,8 @@ __device__ int adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lon
                 ch += o.p[5][l - 1u];
                 cn += min(kRoundRays, R - (g0 + v * kRoundRays));
             }
-            verdict = kEqual ? sem_quick_equal(cn, ch, sem_equal(tq, delta)) : sem_quick(cn, ch, cq1, cq2, delta);
-            if (kEqual) {
+            verdict = equal ? sem_quick_equal(cn, ch, sem_equal(tq, delta)) : sem_quick(cn, ch, cq1, cq2, delta);
+            if (equal) {
                 cq1 = (unsigned long long)ch * tq;
                 cq2 = cq1 * tq;
             }
@@ -1233,7 +1235,7 @@ __device__ int adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lon
             const uint32_t earlier = rmask & ((1u << warp) - 1u);
             if (warp <= last && !later) {  // the bin's latest round through `last`
                 st.s1[bin] = cs1;
-                if (!kEqual) {
+                if (!equal) {
                     st.q1[bin] = cq1;
                     st.q2[bin] = cq2;
                 }
@@ -1256,7 +1258,7 @@ __device__ int adaptive_row(const LaunchArgs &a, uint64_t row, unsigned long lon
     } else {
         unsigned long long *hrow = a.hist + J.hist_off + (uint64_t)k * B;
         for (uint32_t b = tid; b < B; b += nthr) {
-            const unsigned long long s1 = st.s1[b] + (kEqual ? (unsigned long long)st.h[b] * tfx : 0ull);
+            const unsigned long long s1 = st.s1[b] + (equal ? (unsigned long long)st.h[b] * tfx : 0ull);
             if (s1) hrow[b] = rescale_cell(s1, R, count);
         }
         if (tid == 0) {
@@ -1976,7 +1978,7 @@ __global__ void __launch_bounds__(32 * kMaxAdaptWarps, CPD_ADAPT_MIN_BLOCKS) ada
 
 __device__ __noinline__ int adaptive_equal_redo(const LaunchArgs &a, unsigned long long *smem)
 {
-    return adaptive_row<true, true>(a, blockIdx.x, smem, blockDim.x >> 5, threadIdx.x >> 5, threadIdx.x & 31u);
+    return adaptive_row<true, ROWS_EQUAL>(a, blockIdx.x, smem, blockDim.x >> 5, threadIdx.x >> 5, threadIdx.x & 31u);
 }
 
 // The same for the rows of designs with certified pieces, ray by ray: passes with few rows that
@@ -1988,7 +1990,7 @@ __global__ void __launch_bounds__(32 * kMaxAdaptWarps, CPD_ADAPT_MIN_BLOCKS) ada
     cudaGridDependencySynchronize();  // the setup's LamParams and LamDF
     const uint32_t kw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     if (a.adapt_pieces != 1u && !a.designs[find_job<F_ROW>(a.jobs, a.njobs, blockIdx.x)].fc.pieces) return;
-    int r = adaptive_row<false, true>(a, blockIdx.x, adapt_smem, kw, warp, lane);
+    int r = adaptive_row<false, ROWS_EQUAL>(a, blockIdx.x, adapt_smem, kw, warp, lane);
     if (r == ROW_UNSURE) r = adaptive_equal_redo(a, adapt_smem);
     if (r == ROW_OTHER && threadIdx.x == 0) queue_row(a, blockIdx.x);
 }
@@ -3851,6 +3853,25 @@ RowsPlan plan_rows(uint64_t rows, uint32_t R, uint32_t max_B, int num_sms)
     return p;
 }
 
+// Both kinds of rows in one launch, for passes of few rows that have some of each: a kernel for each
+// kind stands one behind the other in the pass's chain, and the second waits for the slowest row of the
+// first. A coated and an uncoated design of 128 rows x 4096 rays 125 -> 106 us, four of each 218 -> 176
+// (both forms inlined: 108 and 181, the kernel spills).
+__device__ __noinline__ int adaptive_mixed_redo(const LaunchArgs &a, unsigned long long *smem)
+{
+    return adaptive_row<true, ROWS_MIXED>(a, blockIdx.x, smem, blockDim.x >> 5, threadIdx.x >> 5, threadIdx.x & 31u);
+}
+__global__ void __launch_bounds__(32 * kMaxAdaptWarps, CPD_ADAPT_MIN_BLOCKS) adaptive_mixed_kernel(const LaunchArgs a)
+{
+    extern __shared__ __align__(16) unsigned long long adapt_smem[];
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();  // the setup's LamParams and LamDF
+    const uint32_t kw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    int r = adaptive_row<false, ROWS_MIXED>(a, blockIdx.x, adapt_smem, kw, warp, lane);
+    if (r == ROW_UNSURE) r = adaptive_mixed_redo(a, adapt_smem);
+    if (r == ROW_OTHER && threadIdx.x == 0) queue_row(a, blockIdx.x);
+}
+
 // Whether the rows of designs with pieces go through adaptive_block_kernel (true) or
 // adaptive_equal_kernel, in adaptive passes of fewer than 8 rows per SM. The first bins by pieces, but
 // tests every bin of every round; the second traces ray by ray, 16 (4) rounds at a time, and tests
@@ -3925,7 +3946,10 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
                          a.adapt_pieces == 1u ? smem : std::max(smem, adapt1_smem_bytes(maxB)), stream, pdl, a);
                 launches++;
             } else {
-                if (a.adapt_pieces && !adapt_by_blocks(maxB, a.total_rows, a.max_rounds, num_sms)) {
+                if (a.adapt_pieces == 3u) {
+                    launch_k(adaptive_mixed_kernel, (unsigned)a.total_rows, 32 * kw, adapt_smem_bytes(kw, maxB), stream, pdl, a);
+                    launches++;
+                } else if (a.adapt_pieces && !adapt_by_blocks(maxB, a.total_rows, a.max_rounds, num_sms)) {
                     launch_k(adaptive_equal_kernel, (unsigned)a.total_rows, 32 * kw, adapt_smem_bytes(kw, maxB), stream, pdl, a);
                     launches++;
                 } else if (a.adapt_pieces) {
@@ -3938,7 +3962,7 @@ int launch_pass(const LaunchArgs &a, int num_sms, uint32_t warps_per_cta, cudaSt
                              adapt_block_smem_bytes(maxB, a.max_rounds), stream, pdl, a);
                     launches++;
                 }
-                if (a.adapt_pieces != 1u) {
+                if (a.adapt_pieces == 0u || a.adapt_pieces == 2u) {
                     launch_k(adaptive_kernel, (unsigned)a.total_rows, 32 * kw, adapt_smem_bytes(kw, maxB), stream, pdl, a);
                     launches++;
                 }
@@ -4026,6 +4050,7 @@ cudaError_t configure_kernels()
     const int bytes = (int)adapt_smem_bytes(kMaxAdaptWarps, CPD_MAX_BINS);
     cudaError_t e = cudaFuncSetAttribute(adaptive_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(adaptive_equal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(adaptive_mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(adaptive1_pieces_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)std::max(adapt1_smem_bytes(CPD_MAX_BINS), adapt1p_smem_bytes(CPD_MAX_BINS)));

@@ -684,7 +684,7 @@ int pass_issue(cpd_context *ctx, PassSlot &S, const std::vector<PassDesign> &ds,
             with += p.dev && p.dev->fc.pieces;
             maybe += p.params && p.params->ar_coated;
         }
-        a.adapt_pieces = with == n ? 1u : with || maybe ? 2u : 0u;
+        a.adapt_pieces = with == n ? 1u : maybe == n ? 2u : with || maybe ? 3u : 0u;
     }
     a.max_B = max_B;
     a.lp = S.lp.as<LamParams>();

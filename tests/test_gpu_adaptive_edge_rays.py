@@ -8,6 +8,7 @@ import pytest
 import compound_prism_designer as cpd
 import oracle as O
 from compound_prism_designer import synth
+from test_gpu_pieces import FIELDS
 from test_gpu_tp_handed_back import _two_sided
 
 pytestmark = pytest.mark.gpu
@@ -98,3 +99,15 @@ def test_rows_of_two_transmittances(B, R):
         assert np.abs(p[:200] - po).max() <= 1e-6
         g, _ = spec.gpu_fitness_points(lam[:200], rays, want_p=True, mode=MODE)
         assert g.rays == int(count.sum()) and g.hits == st["hits"]
+
+
+@pytest.mark.parametrize("W", [5, 60, 400])
+def test_both_kinds_of_designs_in_one_pass(W):
+    rng = np.random.default_rng(W)
+    specs = [_two_sided(rng, 16)[0], synth.random_design(rng, 3, 40, ar_coated=False)[0], synth.random_design(rng, 2, 200)[0]]
+    for R in (33, 2000, 9000):
+        mixed = cpd.fitness_batch(specs, seeds=0.3, max_n=W, max_eval=R, mode=MODE)
+        for spec, f in zip(specs, mixed):
+            g = spec.gpu_fitness_full([0.3], max_n=W, max_eval=R, adaptive=True)
+            for k in FIELDS + ("status",):
+                assert getattr(f, k) == getattr(g, k), (R, k)
