@@ -7,7 +7,7 @@
 //   setup    one thread per (design, wavelength): the flat-face chain in float-float
 //            (cpd_df.h) -> LamParams for the fast path and LamDF for the re-trace
 // and then, for designs whose coated exit face admits certified pieces (cpd_piece.h) under the
-// fixed-N hybrid trace,
+// fixed-N hybrid trace (but for short tables on many rows and a few such designs beside others),
 //   rows     rows_kernel: a wavelength's trace, re-trace and entropy by one team of warps, its
 //            cells in shared memory; ahead of it, in passes of many designs, rows_kernel<HEAVY>
 //            for rows that are mostly re-traced;
@@ -29,8 +29,9 @@
 // A single-design pass with a fixed ray count (the plain call) runs setup_pair_kernel (two
 // warps per 32 rows), and trace_spans_kernel (equal shares of the ray slots per warp) in place
 // of trace; its design's constants are kernel parameters. Adaptive sampling replaces trace and
-// retrace with adaptive1_pieces_kernel / adaptive_block_kernel (designs with pieces),
-// adaptive1_kernel / adaptive_kernel (the others) and adaptive_exact_kernel.
+// retrace with adaptive1_pieces_kernel (many rows), adaptive_block_kernel or adaptive_equal_kernel
+// (designs with pieces), adaptive1_kernel or adaptive_kernel (the others), adaptive_mixed_kernel (few
+// rows of both) and adaptive_exact_kernel.
 #include <cuda_runtime.h>
 
 #include <algorithm>
